@@ -178,7 +178,7 @@ NANGILA_EXPORT int32_t nangila_compress_gpu(NangilaHandle h, const float* gradie
   const GpuLib& lib = gpu_lib();
   if (!lib.ok || count == 0) return NANGILA_COMPRESSION_ERROR;
   const int64_t payload = lib.payload_bytes(int64_t(count));
-  if (payload > lib.crc_max()) return NANGILA_COMPRESSION_ERROR;  // checksum table is a fixed-size device array
+  if (payload > lib.crc_max()) return NANGILA_COMPRESSION_ERROR;  // the checksum entry's limit
   NangilaHook* hook = as_hook(h);
   // kappa < 0: the kernels derive the least-squares gain from the history themselves
   if (lib.encode(gradient, NANGILA_DTYPE_FLOAT32, g_current, g_previous, nullptr, hook->momentum(), -1.0f, int64_t(count),

@@ -98,12 +98,10 @@ at::Tensor state_hash(const std::vector<at::Tensor>& tensors, int64_t seed) {
 at::Tensor crc32_device(const at::Tensor& t) {
   TORCH_CHECK(t.is_cuda() && t.is_contiguous(), "nangila: crc32 wants a contiguous CUDA tensor");
   const int64_t nbytes = t.numel() * t.element_size();
-  auto scratch = at::empty({nangila_crc32_scratch_words(nbytes)}, t.options().dtype(at::kInt));
-  auto out = at::zeros({1}, t.options().dtype(at::kInt));
+  auto out = at::empty({1}, t.options().dtype(at::kInt));  // written by the kernel whatever the size
+  auto* word = reinterpret_cast<uint32_t*>(out.data_ptr<int32_t>());
   c10::cuda::CUDAGuard guard(t.device());
-  check_launch(nangila_crc32(t.data_ptr(), nbytes, reinterpret_cast<uint32_t*>(scratch.data_ptr<int32_t>()),
-                             reinterpret_cast<uint32_t*>(out.data_ptr<int32_t>()), at::cuda::getCurrentCUDAStream()),
-               "crc32");
+  check_launch(nangila_crc32(t.data_ptr(), nbytes, word, word, at::cuda::getCurrentCUDAStream()), "crc32");
   return out;
 }
 // ---- device-side packet codec (host wire format) -------------------------------------------------------------

@@ -205,6 +205,7 @@ int nangila_sculptor_pair_finalize(const NangilaPairDesc* pairs, int32_t npairs,
 
 /* ---- state hash, parallel CRC32, absmax / percentile ------------------------------------------------------ */
 int nangila_state_hash(const void* data, int64_t nbytes, uint64_t seed, uint64_t* out, cudaStream_t stream);
+/* `scratch` of nangila_crc32 is no longer written (the result word is all the kernel needs); it must still not be NULL. */
 int64_t nangila_crc32_scratch_words(int64_t nbytes);
 int nangila_crc32(const void* data, int64_t nbytes, uint32_t* scratch, uint32_t* out, cudaStream_t stream);
 uint32_t nangila_absmax_scratch_words(void);
