@@ -48,6 +48,19 @@ __device__ __forceinline__ void load8_f32(const float* p, int64_t base, int64_t 
   load8_any<float>(p, base, n, v);
 }
 
+// Eight values from `base` on; as with the loads, two 16-byte stores where the address allows it (a warp's two stores
+// together fill whole lines; eight 4-byte stores per lane were 32-byte strided and took the decoder to 2.6 TB/s. Measured
+// on B200 at 38.6 M elements: decoder 183 -> 83 us, 5.8 TB/s; encoder, bf16 gradient, 134 -> 120 us, 6.0 TB/s).
+__device__ __forceinline__ void store8_f32(float* p, int64_t base, int64_t n, const float (&v)[8]) {
+  if (base + 8 <= n && ((reinterpret_cast<uintptr_t>(p + base) & 15u) == 0)) {
+    Vec8<float>::store(p + base, v);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (base + i < n) p[base + i] = v[i];
+  }
+}
+
 // sums[0] += <g + ef, g_hat>, sums[1] += <g_hat, g_hat>
 template <typename T>
 __global__ void __launch_bounds__(kThreads) packet_gain_kernel(const T* __restrict__ grad, const float* __restrict__ curr,
@@ -144,11 +157,7 @@ __global__ void __launch_bounds__(kThreads) packet_encode_kernel(const T* __rest
       } else {
         for (int k = 0; k < 4 && byte0 + k < nbytes; ++k) packed[byte0 + k] = uint8_t(word >> (8 * k));
       }
-      if (ef != nullptr) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (base + i < n) ef[base + i] = x[i];
-      }
+      if (ef != nullptr) store8_f32(ef, base, n, x);
     }
   }
 }
@@ -172,13 +181,13 @@ __global__ void __launch_bounds__(kThreads) packet_decode_kernel(const float* __
     float c[8], p[8];
     load8_f32(kappa != 0.0f ? curr : nullptr, base, n, c);
     load8_f32(kappa != 0.0f ? prev : nullptr, base, n, p);
+    float o[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      if (base + i < n) {
-        const int q = int(word << (28 - 4 * i)) >> 28;
-        out[base + i] = __fmaf_rn(kappa, __fmaf_rn(mu, c[i] - p[i], c[i]), float(q) * s);
-      }
+      const int q = int(word << (28 - 4 * i)) >> 28;
+      o[i] = __fmaf_rn(kappa, __fmaf_rn(mu, c[i] - p[i], c[i]), float(q) * s);
     }
+    store8_f32(out, base, n, o);
   }
 }
 
