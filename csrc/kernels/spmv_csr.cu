@@ -27,9 +27,11 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <algorithm>
 #include <new>
 #include <vector>
 
+#include "bicgstab.cuh"
 #include "nangila_spice_kernels.h"
 #include "ptx_sm100.cuh"
 
@@ -227,61 +229,6 @@ __global__ void residual_init_kernel(double* r, double* r0, const double* b, con
     if (i < n) { double t = b[i] - ax[i]; r[i] = t; r0[i] = t; }
 }
 
-
-// ---- graph-captured iteration: scalars live on the device --------------------------------------------
-// sc[0] rho, [1] alpha, [2] omega, [3] beta, [4] r.r, [5] state (0 running, 1 stopped, 2 stop after this
-// iteration), [6] iterations done. A breakdown (a vanishing denominator) stops the iteration on the
-// device: the remaining kernels of the graph become no-ops.
-__global__ void dot_final_step_kernel(const double* __restrict__ partial, int blocks, double* __restrict__ sc, int step) {
-    __shared__ double d[2];
-    if (threadIdx.x < 2) {
-        double t = 0.0;
-        for (int b = 0; b < blocks; ++b) t += partial[2 * b + threadIdx.x];
-        d[threadIdx.x] = t;
-    }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    const bool running = sc[5] == 0.0;
-    if (step == 1) {
-        if (!running) return;
-        if (fabs(d[0]) < 1e-300) { sc[5] = 1.0; return; }
-        sc[3] = (d[0] / sc[0]) * (sc[1] / sc[2]);
-        sc[0] = d[0];
-    } else if (step == 2) {
-        if (!running) return;
-        if (fabs(d[0]) < 1e-300) { sc[5] = 1.0; return; }
-        sc[1] = sc[0] / d[0];
-    } else if (step == 3) {
-        if (!running) return;
-        sc[2] = d[1] > 0.0 ? d[0] / d[1] : 0.0;
-        if (sc[2] == 0.0) sc[5] = 2.0;
-    } else {
-        if (sc[5] == 1.0) return;
-        sc[4] = d[0];
-        sc[6] += 1.0;
-        if (sc[5] == 2.0) sc[5] = 1.0;
-    }
-}
-__global__ void update_p_dev_kernel(double* p, double* ph, const double* r, const double* v, const double* inv_diag, const double* sc, int n) {
-    if (sc[5] != 0.0) return;
-    const double beta = sc[3], omega = sc[2];
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) { double t = r[i] + beta * (p[i] - omega * v[i]); p[i] = t; ph[i] = t * inv_diag[i]; }
-}
-__global__ void update_s_dev_kernel(double* s, double* sh, const double* r, const double* v, const double* inv_diag, const double* sc, int n) {
-    if (sc[5] != 0.0) return;
-    const double alpha = sc[1];
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) { double t = r[i] - alpha * v[i]; s[i] = t; sh[i] = t * inv_diag[i]; }
-}
-__global__ void update_xr_dev_kernel(double* x, double* r, const double* ph, const double* sh, const double* s, const double* t, const double* sc,
-                                     int n) {
-    if (sc[5] == 1.0) return;
-    const double alpha = sc[1], omega = sc[2];
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) { x[i] += alpha * ph[i] + omega * sh[i]; r[i] = s[i] - omega * t[i]; }
-}
-
 }  // namespace
 
 struct NangilaSpmv {
@@ -291,12 +238,16 @@ struct NangilaSpmv {
     int* d_status = nullptr;  // set by a kernel whose bulk copy timed out
     bool plain_loads = false;  // NANGILA_SPMV_PLAIN=1: use the plain-load kernel
     int cap = kCap;            // non-zeros per row block: 2048 (256 threads) or 1024 (128 threads, NANGILA_SPMV_TILE=1024)
-    double* d_work = nullptr;   // 9 solver vectors + inverse diagonal, allocated on first solve
-    double* d_partial = nullptr;  // reduction scratch: 2 * kRedBlocks + 2
+    double* d_work = nullptr;   // solver vectors (kWorkVectors), allocated on first solve
+    double* d_partial = nullptr;  // partial sums, then results and counter of the solver kernel
     std::vector<double> h_inv_diag;
-    double* d_sc = nullptr;           // device scalars of the graph-captured solver iteration
+    bool inv_diag_on_device = false;  // d_work holds h_inv_diag
     cudaStream_t solve_stream = nullptr;
-    cudaGraphExec_t iter_graph = nullptr;
+    // the solver kernel's split of the rows: see bicgstab.cuh
+    int ctas = 0, max_rows = 0, max_entries = 0;
+    bool resident = false;
+    double* d_scaled = nullptr;  // the solver's scaled values where they do not fit into shared memory
+    int* d_plan = nullptr;  // first_row [ctas + 1], first_long [ctas + 1], long_rows
     std::vector<int> h_row_ptr, h_diag_slot;  // kept on the host to refresh the preconditioner when values change
 };
 
@@ -305,6 +256,7 @@ struct NangilaSpmv {
 // zero or tiny diagonal).
 static void refresh_preconditioner(NangilaSpmv* c, const double* val) {
     const int n = c->n;
+    c->inv_diag_on_device = false;
     c->h_inv_diag.assign(size_t(n), 1.0);
     for (int r = 0; r < n; ++r) {
         double mx = 0.0;
@@ -317,12 +269,13 @@ static void refresh_preconditioner(NangilaSpmv* c, const double* val) {
 
 static void free_arrays(NangilaSpmv* c) {
     cudaFree(c->d_row_ptr); cudaFree(c->d_col); cudaFree(c->d_blocks); cudaFree(c->d_val); cudaFree(c->d_x); cudaFree(c->d_y);
-    cudaFree(c->d_work); cudaFree(c->d_partial); cudaFree(c->d_status); cudaFree(c->d_sc);
-    if (c->iter_graph) cudaGraphExecDestroy(c->iter_graph);
+    cudaFree(c->d_work); cudaFree(c->d_partial); cudaFree(c->d_status); cudaFree(c->d_plan);
+    cudaFree(c->d_scaled);
     if (c->solve_stream) cudaStreamDestroy(c->solve_stream);
-    c->iter_graph = nullptr;
     c->solve_stream = nullptr;
-    c->d_sc = nullptr;
+    c->d_plan = nullptr;
+    c->d_scaled = nullptr;
+    c->inv_diag_on_device = false;
     c->d_status = nullptr;
     c->d_row_ptr = c->d_col = c->d_blocks = nullptr;
     c->d_val = c->d_x = c->d_y = c->d_work = c->d_partial = nullptr;
@@ -458,9 +411,92 @@ extern "C" int nangila_spmv_dims(const NangilaSpmv* c, int* n, int* nnz, int* n_
     return 0;
 }
 
-// Solves A x = b (x starts at 0) with vectors resident on the device. Default: the iteration is a CUDA graph
-// with its scalars on the device (below). NANGILA_SPMV_GRAPH=0: per iteration two SpMVs, three fused vector
-// kernels and four 16-byte reads of reduction results by the host.
+// ---- BiCGSTAB ---------------------------------------------------------------------------------------
+constexpr int kWorkVectors = 11;  // inverse diagonal, right-hand side, then nine that either form of the solver uses as it needs
+
+// Splits the rows over the CTAs of the solver kernel: contiguous ranges of about equal cost (an entry counts one, a row
+// three more for its vector work).
+static cudaError_t plan_solver(NangilaSpmv* c) {
+    using namespace nangila::krylov;
+    int dev = 0, sms = 0, smem_max = 0;
+    cudaError_t e;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+    const int n = c->n;
+    const int ctas = c->nnz <= kOneCta ? 1 : std::min({sms, kMaxCtas, c->nnz / kEntriesPerCta});
+    std::vector<int> first_row(size_t(ctas) + 1, n), first_long(size_t(ctas) + 1, 0), long_rows;
+    const double total = double(c->nnz) + 3.0 * n;
+    int row = 0, max_rows = 0, max_entries = 0;
+    first_row[0] = 0;
+    for (int b = 0; b < ctas; ++b) {
+        const int begin = row;
+        first_long[size_t(b)] = int(long_rows.size());
+        const double until = total * (b + 1) / ctas;
+        while (row < n && (b == ctas - 1 || double(c->h_row_ptr[size_t(row)]) + 3.0 * row < until)) {
+            if (c->h_row_ptr[size_t(row) + 1] - c->h_row_ptr[size_t(row)] > kLongRow) long_rows.push_back(row);
+            ++row;
+        }
+        first_row[size_t(b) + 1] = row;
+        max_rows = std::max(max_rows, row - begin);
+        max_entries = std::max(max_entries, c->h_row_ptr[size_t(row)] - c->h_row_ptr[size_t(begin)]);
+    }
+    first_long[size_t(ctas)] = int(long_rows.size());
+    std::vector<int> plan(first_row);
+    plan.insert(plan.end(), first_long.begin(), first_long.end());
+    plan.insert(plan.end(), long_rows.begin(), long_rows.end());
+    if ((e = cudaMalloc(&c->d_plan, sizeof(int) * plan.size())) != cudaSuccess) return e;
+    if ((e = cudaMemcpy(c->d_plan, plan.data(), sizeof(int) * plan.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return e;
+    c->ctas = ctas;
+    c->max_rows = max_rows;
+    c->max_entries = max_entries;
+    const size_t room = size_t(smem_max) - 4096;  // the kernel's static shared memory, and what the runtime keeps
+    c->resident = solver_smem(true, max_rows, max_entries) <= room;
+    if (!c->resident) return cudaSuccess;
+    return cudaFuncSetAttribute(bicgstab_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(room));
+}
+
+// The solver kernel: one launch for the whole solve (bicgstab.cuh).
+static int solve_on_device(NangilaSpmv* c, double* h_x, double tol, int max_iter, int* iterations, double* rel_residual) {
+    using namespace nangila::krylov;
+    const size_t N = size_t(c->n), S = (N + 1) & ~size_t(1);
+    cudaStream_t st = c->solve_stream;
+    double* w = c->d_work + 2 * S;
+    const size_t sums = 2 * kSlot * size_t(c->ctas);
+    SolverArgs a;
+    a.row_ptr = c->d_row_ptr; a.col = c->d_col; a.val = c->d_val;
+    a.first_row = c->d_plan; a.first_long = c->d_plan + c->ctas + 1; a.long_rows = c->d_plan + 2 * (c->ctas + 1);
+    a.inv_diag = c->d_work; a.b = c->d_work + S;
+    a.status = c->d_status;
+    a.parts = reinterpret_cast<Parts*>(w); a.rv = reinterpret_cast<double2*>(w + 4 * S);
+    a.x = w + 6 * S; a.r0 = w + 7 * S; a.p = w + 8 * S;
+    a.scaled = c->d_scaled;
+    a.partial = c->d_partial;
+    a.out = c->d_partial + sums;
+    a.arrived = reinterpret_cast<uint32_t*>(a.out + 4);
+    a.max_iter = max_iter; a.max_entries = c->max_entries;
+    a.tol = tol;
+    a.timeout_ns = 2000000000ull;
+    cudaError_t e;
+    if ((e = cudaMemsetAsync(a.out, 0, 5 * sizeof(double), st)) != cudaSuccess) return int(e);
+    void* args[] = {&a};
+    const void* fn = c->resident ? reinterpret_cast<const void*>(&bicgstab_kernel<true>) : reinterpret_cast<const void*>(&bicgstab_kernel<false>);
+    e = cudaLaunchCooperativeKernel(fn, dim3(unsigned(c->ctas)), dim3(unsigned(solver_threads(c->resident))), args, solver_smem(c->resident, c->max_rows, c->max_entries), st);
+    if (e != cudaSuccess) return int(e);
+    double out[4];
+    if ((e = cudaMemcpyAsync(out, a.out, sizeof out, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return int(e);
+    if ((e = cudaMemcpyAsync(h_x, a.x, sizeof(double) * N, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return int(e);
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return int(e);
+    const double rel = sqrt(out[0]) / out[1];
+    if (iterations) *iterations = int(out[2]);
+    if (rel_residual) *rel_residual = rel;
+    if (out[3] != 0.0) return int(cudaErrorTimeout);
+    return rel < tol ? 0 : -1;
+}
+
+// Solves A x = b (x starts at 0) with vectors resident on the device: one kernel for the whole solve, which tests the
+// residual every fourth iteration. NANGILA_SPMV_GRAPH=0: per iteration two SpMVs, three fused vector kernels and four 16-byte reads
+// of reduction results by the host, the residual tested after every one.
 extern "C" int nangila_spmv_bicgstab(NangilaSpmv* c, const double* h_b, double* h_x, double tol, int max_iter, int* iterations,
                                      double* rel_residual) {
     if (!c || !c->d_val || !h_b || !h_x) return int(cudaErrorInvalidValue);
@@ -469,13 +505,25 @@ extern "C" int nangila_spmv_bicgstab(NangilaSpmv* c, const double* h_b, double* 
     const size_t S = (N + 1) & ~size_t(1);  // vector stride: keeps every work vector 16-byte aligned
     cudaError_t e;
     if (!c->d_work) {
-        e = cudaMalloc(&c->d_work, sizeof(double) * S * 11);
-        if (e != cudaSuccess) return int(e);
-        e = cudaMalloc(&c->d_partial, sizeof(double) * (2 * kRedBlocks + 2));
-        if (e != cudaSuccess) return int(e);
+        if (!c->d_plan && (e = plan_solver(c)) != cudaSuccess) return int(e);
+        if (!c->solve_stream && (e = cudaStreamCreateWithFlags(&c->solve_stream, cudaStreamNonBlocking)) != cudaSuccess) return int(e);
+        // sums of either form, results and the counter
+        const size_t doubles = std::max(size_t(2) * kRedBlocks + 2, 2 * nangila::krylov::kSlot * size_t(c->ctas) + 5);
+        if (!c->d_partial && (e = cudaMalloc(&c->d_partial, sizeof(double) * doubles)) != cudaSuccess) return int(e);
+        if (!c->resident && !c->d_scaled && (e = cudaMalloc(&c->d_scaled, sizeof(double) * size_t(c->nnz))) != cudaSuccess) return int(e);
+        if ((e = cudaMalloc(&c->d_work, sizeof(double) * S * kWorkVectors)) != cudaSuccess) return int(e);
     }
-    double *x = c->d_work, *r = x + S, *r0 = r + S, *p = r0 + S, *v = p + S, *s = v + S, *t = s + S, *ph = t + S, *sh = ph + S, *b = sh + S,
-           *inv = b + S;
+    double *inv = c->d_work, *b = inv + S;
+    const char* genv = getenv("NANGILA_SPMV_GRAPH");
+    if (!(genv && genv[0] == '0')) {
+        cudaStream_t st = c->solve_stream;
+        if (!c->inv_diag_on_device && (e = cudaMemcpyAsync(inv, c->h_inv_diag.data(), sizeof(double) * N, cudaMemcpyHostToDevice, st)) != cudaSuccess)
+            return int(e);
+        c->inv_diag_on_device = true;
+        if ((e = cudaMemcpyAsync(b, h_b, sizeof(double) * N, cudaMemcpyHostToDevice, st)) != cudaSuccess) return int(e);
+        return solve_on_device(c, h_x, tol, max_iter, iterations, rel_residual);
+    }
+    double *x = b + S, *r = x + S, *r0 = r + S, *p = r0 + S, *v = p + S, *s = v + S, *t = s + S, *ph = t + S, *sh = ph + S;
     double* out = c->d_partial + 2 * kRedBlocks;
     const int grid = (n + kThreads - 1) / kThreads;
     auto dots = [&](const double* a1, const double* b1, const double* a2, const double* b2, double res[2]) -> cudaError_t {
@@ -494,60 +542,6 @@ extern "C" int nangila_spmv_bicgstab(NangilaSpmv* c, const double* h_b, double* 
     double rel = sqrt(d[1]) / bnorm, rho = 1.0, alpha = 1.0, omega = 1.0;
     int it = 0;
     bool ok = rel < tol;
-    const char* genv = getenv("NANGILA_SPMV_GRAPH");
-    if (!ok && !(genv && genv[0] == '0')) {
-        // One iteration (2 SpMVs, 3 vector kernels, 4 reductions with their scalar updates) is captured
-        // once per loaded matrix as a CUDA graph and replayed; the host reads 24 bytes every 4th
-        // iteration to test convergence, so the loop is not bound by launch or copy latency.
-        if (!c->d_sc) {
-            if ((e = cudaMalloc(&c->d_sc, sizeof(double) * 8)) != cudaSuccess) return int(e);
-            if ((e = cudaStreamCreateWithFlags(&c->solve_stream, cudaStreamNonBlocking)) != cudaSuccess) return int(e);
-        }
-        cudaStream_t st = c->solve_stream;
-        double* sc = c->d_sc;
-        if (!c->iter_graph) {
-            cudaGraph_t graph = nullptr;
-            if ((e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return int(e);
-            dot2_partial_kernel<<<kRedBlocks, kThreads, 0, st>>>(r0, r, nullptr, nullptr, n, c->d_partial);
-            dot_final_step_kernel<<<1, 32, 0, st>>>(c->d_partial, kRedBlocks, sc, 1);
-            update_p_dev_kernel<<<grid, kThreads, 0, st>>>(p, ph, r, v, inv, sc, n);
-            nangila_spmv_device(c, ph, v, st);
-            dot2_partial_kernel<<<kRedBlocks, kThreads, 0, st>>>(r0, v, nullptr, nullptr, n, c->d_partial);
-            dot_final_step_kernel<<<1, 32, 0, st>>>(c->d_partial, kRedBlocks, sc, 2);
-            update_s_dev_kernel<<<grid, kThreads, 0, st>>>(s, sh, r, v, inv, sc, n);
-            nangila_spmv_device(c, sh, t, st);
-            dot2_partial_kernel<<<kRedBlocks, kThreads, 0, st>>>(t, s, t, t, n, c->d_partial);
-            dot_final_step_kernel<<<1, 32, 0, st>>>(c->d_partial, kRedBlocks, sc, 3);
-            update_xr_dev_kernel<<<grid, kThreads, 0, st>>>(x, r, ph, sh, s, t, sc, n);
-            dot2_partial_kernel<<<kRedBlocks, kThreads, 0, st>>>(r, r, nullptr, nullptr, n, c->d_partial);
-            dot_final_step_kernel<<<1, 32, 0, st>>>(c->d_partial, kRedBlocks, sc, 4);
-            e = cudaStreamEndCapture(st, &graph);
-            if (e != cudaSuccess || !graph) return int(e != cudaSuccess ? e : cudaErrorUnknown);
-            e = cudaGraphInstantiate(&c->iter_graph, graph, 0);
-            cudaGraphDestroy(graph);
-            if (e != cudaSuccess) { c->iter_graph = nullptr; return int(e); }
-        }
-        const double init[8] = {1.0, 1.0, 1.0, 0.0, d[1], 0.0, 0.0, 0.0};
-        if ((e = cudaMemcpy(sc, init, sizeof init, cudaMemcpyHostToDevice)) != cudaSuccess) return int(e);
-        const int check_every = 4;
-        double tail[3] = {d[1], 0.0, 0.0};  // r.r, state, iterations
-        while (it < max_iter) {
-            for (int k = 0; k < check_every; ++k)
-                if ((e = cudaGraphLaunch(c->iter_graph, st)) != cudaSuccess) return int(e);
-            if ((e = cudaMemcpyAsync(tail, sc + 4, sizeof tail, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return int(e);
-            if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return int(e);
-            it = int(tail[2]);
-            rel = sqrt(tail[0]) / bnorm;
-            if (rel < tol) { ok = true; break; }
-            if (tail[1] != 0.0) break;
-        }
-        if ((e = cudaMemcpy(h_x, x, sizeof(double) * N, cudaMemcpyDeviceToHost)) != cudaSuccess) return int(e);
-        if (iterations) *iterations = it;
-        if (rel_residual) *rel_residual = rel;
-        if ((e = cudaGetLastError()) != cudaSuccess) return int(e);
-        if (int stt = nangila_spmv_status(c)) return stt;
-        return ok ? 0 : -1;
-    }
     while (!ok && it < max_iter) {
         if ((e = dots(r0, r, nullptr, nullptr, d)) != cudaSuccess) return int(e);
         double rho_new = d[0];
