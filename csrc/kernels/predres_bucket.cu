@@ -226,15 +226,13 @@ constexpr int kMaxDepth = 6;
 // bytes are in flight than registers could hold. Each warp owns its ring and its barriers; `kuse`
 // counts the stage uses of this warp since the start of the kernel (stage = kuse % D, parity from
 // kuse / D). Returns false if a copy did not complete in time (the caller reports the failure).
-// SINGLE (a world of one rank): nothing is exchanged; the dequantized value is written straight back to
-// the bucket and the history, so the whole step is this one pass.
-template <typename T, typename S, bool LEAN, bool SINGLE>
+template <typename T, typename S, bool LEAN>
 __device__ __forceinline__ bool phase1_bulk(T* __restrict__ grad, S* __restrict__ prev,
                                             const S* __restrict__ curr, S* __restrict__ ef, uint8_t* dst,
                                             int64_t tbase, int iters, int C, int tid, float mu, float kappa,
                                             bool use_history, uint32_t key1, bool stochastic, Stats& st,
                                             uint8_t* ring, uint64_t* bars, uint32_t& kuse, uint64_t timeout_ns,
-                                            int ndst, uint8_t* const* regions, uint64_t dst_off, bool keep_history) {
+                                            int ndst, uint8_t* const* regions, uint64_t dst_off) {
   using R = Ring<T, S, LEAN>;
   constexpr int D = R::D;
   const int lane = tid & 31, warp = tid >> 5;
@@ -294,11 +292,7 @@ __device__ __forceinline__ bool phase1_bulk(T* __restrict__ grad, S* __restrict_
         uint32_t packed, sb, qs[4];
         quantize8_bf16(x, packed, sb, qs);
         if (has_ef) *reinterpret_cast<uint4*>(ef + base) = make_uint4(x[0], x[1], x[2], x[3]);
-        if constexpr (SINGLE) {
-          const uint4 o = make_uint4(qs[0], qs[1], qs[2], qs[3]);
-          *reinterpret_cast<uint4*>(grad + base) = o;
-          if (keep_history) *reinterpret_cast<uint4*>(prev + base) = o;
-        } else if (ndst == 1) {
+        if (ndst == 1) {
           *packed_ptr(dst, C, it, tid) = packed;
           if ((tid & (kLanes8 - 1)) == 0) *scale_ptr(dst, C, it, tid) = uint16_t(sb);
         } else {
@@ -350,11 +344,6 @@ __device__ __forceinline__ bool phase1_bulk(T* __restrict__ grad, S* __restrict_
         st.e2 = __fmaf_rn(e[i], e[i], st.e2);
       }
     }
-    float out[kE];
-    if constexpr (SINGLE) {
-#pragma unroll
-      for (int i = 0; i < kE; ++i) out[i] = e[i];
-    }
     uint32_t packed, sb;
     quantize8(e, key1, uint32_t(base >> 1), stochastic, packed, sb);
     if (has_ef) {
@@ -364,16 +353,7 @@ __device__ __forceinline__ bool phase1_bulk(T* __restrict__ grad, S* __restrict_
         for (int i = 0; i < kE; ++i) st.f2 = __fmaf_rn(e[i], e[i], st.f2);
       }
     }
-    if constexpr (SINGLE) {
-#pragma unroll
-      for (int i = 0; i < kE; ++i) out[i] -= e[i];  // q * scale
-      if constexpr (!LEAN) {
-#pragma unroll
-        for (int i = 0; i < kE; ++i) out[i] = __fmaf_rn(kappa, __fmaf_rn(mu, cu[i] - pv[i], cu[i]), out[i]);
-      }
-      Vec8<T>::store(grad + base, out);
-      if (keep_history) Vec8<S>::store(prev + base, out);  // becomes g(t) after the caller swaps prev and curr
-    } else if (ndst == 1) {
+    if (ndst == 1) {
       *packed_ptr(dst, C, it, tid) = packed;
       if ((tid & (kLanes8 - 1)) == 0) *scale_ptr(dst, C, it, tid) = uint16_t(sb);
     } else {
@@ -390,6 +370,26 @@ __device__ __forceinline__ bool phase1_bulk(T* __restrict__ grad, S* __restrict_
 }
 
 constexpr int kWarps = kThreads / 32;
+
+// Adds a CTA's running sums to the rank's statistics: five atomics per CTA.
+__device__ __forceinline__ void add_stats(const Stats& st, float (*red)[kWarps], float* out) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  float v[5] = {st.e2, st.g2, st.xp, st.pp, st.f2};
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);
+    if (lane == 0) red[k][tid >> 5] = v[k];
+  }
+  __syncthreads();
+  if (tid < 5) {
+    float a = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i) a += red[tid][i];
+    atomicAdd(out + tid, a);
+  }
+}
+
 constexpr int kSlots = 4;  // completion counters in flight per CTA
 
 // The eight warps of a CTA work on the same task but never meet at a block barrier: each warp waits
@@ -401,7 +401,7 @@ constexpr int kSlots = 4;  // completion counters in flight per CTA
 // MODE 0: exact all-reduce; 1: compressed all-reduce; 2: compressed reduce-scatter (phases 1 and 2
 // only: the owner writes the mean of its shard to out_shard, nothing is broadcast, no history);
 // 3: compressed all-reduce, lean phase 1 (this rank's gain is zero and no statistics are wanted);
-// 4 / 5: world of one rank, full / lean: phase 1 alone quantizes, reconstructs and writes the result;
+// (a world of one rank has a kernel of its own: predres_single_kernel;)
 // 6 / 7: gather mode, full / lean (small worlds): phase 1 pushes the packed chunk to every rank, and
 // every rank sums the W contributions of every chunk itself: one quantization, two phases.
 template <typename T, typename S, int MODE>
@@ -409,8 +409,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
   constexpr bool COMPRESSED = MODE != 0;
   constexpr bool RS = MODE == 2;
-  constexpr bool LEAN = MODE == 2 || MODE == 3 || MODE == 5 || MODE == 7;
-  constexpr bool SINGLE = MODE == 4 || MODE == 5;
+  constexpr bool LEAN = MODE == 2 || MODE == 3 || MODE == 7;
   constexpr bool GATHER = MODE == 6 || MODE == 7;
   const int vr = blockIdx.y;
   const int me = p.rank0 + vr;
@@ -430,7 +429,7 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
   uint32_t* status = p.status[vr];
   uint8_t* myreg = p.region[me];
   const int T1 = owned_max * W;
-  const int ntasks = GATHER ? 2 * NC : SINGLE ? T1 : T1 + my_owned + (RS ? 0 : NC);
+  const int ntasks = GATHER ? 2 * NC : T1 + my_owned + (RS ? 0 : NC);
   // Reduce-scatter has no phase 3 to prove that the owner is done reading, so its slots alternate
   // between two sets by launch parity (a rank cannot get two launches ahead of a peer: its phase 2 of
   // the launch in between needs that peer's flags).
@@ -486,7 +485,7 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
   // phase, so a contiguous set of phases is a contiguous task range.
   const int pm = (p.phase_mask & 7) == 0 ? 7 : (p.phase_mask & 7);
   const int end1 = GATHER ? NC : T1;
-  const int end2 = GATHER ? 2 * NC : SINGLE ? T1 : T1 + my_owned;
+  const int end2 = GATHER ? 2 * NC : T1 + my_owned;
   const int task_begin = (pm & 1) ? 0 : (pm & 2) ? end1 : end2;
   const int task_end = (pm & 4) ? ntasks : (pm & 2) ? end2 : end1;
 
@@ -540,18 +539,18 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
         if (full) {
           using R = Ring<T, S, LEAN>;
           const int warp = tid >> 5;
-          if (!phase1_bulk<T, S, LEAN, SINGLE>(grad, prev, curr, ef, dst, t.base, iters, C, tid, mu, kappa, use_history, key1,
+          if (!phase1_bulk<T, S, LEAN>(grad, prev, curr, ef, dst, t.base, iters, C, tid, mu, kappa, use_history, key1,
                                        stochastic, acc_stats, s_ring + warp * R::BYTES_PER_WARP, &s_bars[warp][0],
-                                       ring_uses, p.timeout_ns, ndst, p.region, dst_off, keep_history)) {
+                                       ring_uses, p.timeout_ns, ndst, p.region, dst_off)) {
             if (lane == 0)
               report_failure(status, kTimeoutBulk, uint32_t(me), 0xffffffffu, epoch, 0u, 1u, uint32_t(c));
             break;
           }
         } else
-          phase1_compressed<T, S, LEAN, true, SINGLE>(grad, prev, curr, ef, dst, t.base, lim, iters, C, tid, mu, kappa,
+          phase1_compressed<T, S, LEAN, true, false>(grad, prev, curr, ef, dst, t.base, lim, iters, C, tid, mu, kappa,
                                               use_history, key1, stochastic, acc_stats, ndst, p.region, dst_off,
                                               keep_history);
-        if (!SINGLE && !GATHER && tid == 0) *reinterpret_cast<float*>(dst + compressed_trailer_off(C)) = kappa;
+        if (!GATHER && tid == 0) *reinterpret_cast<float*>(dst + compressed_trailer_off(C)) = kappa;
         if (GATHER && tid < W) *reinterpret_cast<float*>(p.region[tid] + dst_off + compressed_trailer_off(C)) = kappa;
       } else {
 #pragma unroll 2
@@ -872,7 +871,7 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
           __threadfence_system();
           for (int r = 0; r < W; ++r)
             st_release_sys(reinterpret_cast<uint32_t*>(p.region[r] + p.flag1_off) + (uint64_t(j) * W + me), epoch);
-        } else if (t.phase == 1 && !SINGLE) {
+        } else if (t.phase == 1) {
           __threadfence_system();
           st_release_sys(reinterpret_cast<uint32_t*>(p.region[t.o] + p.flag1_off) + (uint64_t(j) * W + me), epoch);
         } else if (t.phase == 2 && !RS && !GATHER) {
@@ -886,28 +885,100 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
     }
   }
 
-  // per-rank telemetry: five atomics per CTA
-  if (p.stats[vr] != nullptr && COMPRESSED && !LEAN && (pm & 1)) {
-    float v[5] = {acc_stats.e2, acc_stats.g2, acc_stats.xp, acc_stats.pp, acc_stats.f2};
+  if (p.stats[vr] != nullptr && COMPRESSED && !LEAN && (pm & 1)) add_stats(acc_stats, red, p.stats[vr]);
+}
+
+// A world of one rank: the compressed all-reduce is one elementwise pass, so neither chunks nor flags nor a task protocol are
+// needed. A CTA handles a few tiles of 2048 elements and ends; the grid covers the bucket.
+// Bound by HBM: lean, bf16, 8 bytes an element (gradient and error memory, in and out). What it takes to get there on
+// this part is CTAs that the hardware hands out as SMs come free: a plain 2-in 2-out copy of 52.4 M bf16 elements runs at 6.4 TB/s
+// that way and at 5.5 to 6.0 with a resident grid that strides (SMs differ in speed, and a fixed share waits for the slowest).
+// The exchange kernel did this before, one chunk per resident CTA: 104 us; a resident grid with rings of bulk copies that
+// never drain, 82 us; this, 68 us. History and statistics, fp32, 28 bytes an element, 6.55 M elements: 42 -> 35 us.
+// Codes and sums are computed as in the exchange kernel, chunk by chunk: a chunk that lies wholly inside the bucket takes the
+// packed-bf16 path where there is one, the last partial one FP32.
+constexpr int kLeanTiles = 2;  // per CTA: both tiles' loads are in flight before either is used (1: 83 us, 4: 70)
+template <typename T, typename S, bool LEAN>
+__global__ void __launch_bounds__(kThreads) predres_single_kernel(const __grid_constant__ NangilaPredResParams p, int tiles) {
+  [[maybe_unused]] __shared__ float red[5][kWarps];
+  const int tid = threadIdx.x;
+  // A rank that has failed does nothing more. The word is looked at when the first data are there, so it costs no latency.
+  const uint32_t failed = *reinterpret_cast<volatile uint32_t*>(&p.status[0][kStatusCode]);
+  T* __restrict__ grad = static_cast<T*>(p.grad[0]);
+  S* __restrict__ prev = static_cast<S*>(p.prev[0]);
+  const S* __restrict__ curr = static_cast<const S*>(p.curr[0]);
+  S* __restrict__ ef = static_cast<S*>(p.ef[0]);
+  const int64_t n = p.n, cta_elems = int64_t(tiles) * kElemsPerIter;
+  const float kappa = p.pred_gain[0];
+  const uint32_t key = make_key(p.seed, p.step, p.bucket_id, 0u, 1u);
+  const bool stochastic = p.stochastic != 0;
+  const bool use_history = kappa != 0.0f || p.measure != 0;
+  const bool keep_history = p.skip_history == 0 || use_history;
+  Stats stats;
+  auto fp32_tiles = [&](int64_t first, int count) {
+    if (first + int64_t(count) * kElemsPerIter <= n)
+      phase1_compressed<T, S, LEAN, false, true>(grad, prev, curr, ef, nullptr, first, n, count, 0, tid, p.mu, kappa, use_history, key,
+                                                 stochastic, stats, 1, nullptr, 0, keep_history);
+    else
+      phase1_compressed<T, S, LEAN, true, true>(grad, prev, curr, ef, nullptr, first, n, count, 0, tid, p.mu, kappa, use_history, key,
+                                                stochastic, stats, 1, nullptr, 0, keep_history);
+  };
+  auto load_sum = [&](int64_t base, uint32_t (&x)[4]) {  // eight values of gradient + error memory, packed
+    const uint4 g = *reinterpret_cast<const uint4*>(grad + base);
+    const uint4 e = ef != nullptr ? *reinterpret_cast<const uint4*>(ef + base) : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, ew[4] = {e.x, e.y, e.z, e.w};
 #pragma unroll
-    for (int k = 0; k < 5; ++k) {
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);
-      if (lane == 0) red[k][tid >> 5] = v[k];
+    for (int j = 0; j < 4; ++j) x[j] = ef != nullptr ? as_u32(__hadd2(as_bf162(gw[j]), as_bf162(ew[j]))) : gw[j];
+  };
+  auto bf16_tile = [&](int64_t first, uint32_t (&x)[4]) {
+    const int64_t base = first + tid * kE;
+    if (__any_sync(0xffffffffu, maybe_nonfinite8(x))) {
+      fp32_tiles(first, 1);  // a NaN / Inf in the warp's slice (or magnitudes >= 2): sanitised there
+      return;
     }
-    __syncthreads();
-    if (tid < 5) {
-      float a = 0.0f;
+    uint32_t packed, sb, qs[4];
+    quantize8_bf16(x, packed, sb, qs);
+    if (ef != nullptr) *reinterpret_cast<uint4*>(ef + base) = make_uint4(x[0], x[1], x[2], x[3]);
+    const uint4 o = make_uint4(qs[0], qs[1], qs[2], qs[3]);
+    *reinterpret_cast<uint4*>(grad + base) = o;
+    if (keep_history) *reinterpret_cast<uint4*>(prev + base) = o;
+  };
+  // (one round, unless the caller has capped the CTAs)
+  for (int64_t tile0 = int64_t(blockIdx.x) * cta_elems; tile0 < n; tile0 += int64_t(gridDim.x) * cta_elems) {
+    if constexpr (kFastBf16<T, S, LEAN>) {
+      const int64_t whole = n / p.chunk_elems * p.chunk_elems;  // end of the last whole chunk (chunks are whole tiles)
+      if (tile0 + cta_elems <= whole) {
+        uint32_t x[kLeanTiles][4];  // all loads first: nothing waits for a store
 #pragma unroll
-      for (int i = 0; i < kWarps; ++i) a += red[tid][i];
-      atomicAdd(&p.stats[vr][tid], a);
+        for (int it = 0; it < kLeanTiles; ++it) load_sum(tile0 + it * kElemsPerIter + tid * kE, x[it]);
+        if (failed != 0u) return;
+#pragma unroll
+        for (int it = 0; it < kLeanTiles; ++it) bf16_tile(tile0 + it * kElemsPerIter, x[it]);
+      } else {
+        if (failed != 0u) return;
+        for (int64_t first = tile0; first < n && first < tile0 + cta_elems; first += kElemsPerIter) {
+          if (first + kElemsPerIter <= whole) {
+            uint32_t x[4];
+            load_sum(first + tid * kE, x);
+            bf16_tile(first, x);
+          } else {
+            fp32_tiles(first, 1);
+          }
+        }
+      }
+    } else {
+      if (failed != 0u) return;
+      fp32_tiles(tile0, tiles);
     }
+  }
+  if constexpr (!LEAN) {
+    if (p.stats[0] != nullptr) add_stats(stats, red, p.stats[0]);
   }
 }
 
 template <typename T, typename S, int MODE>
 cudaError_t launch_mode(const NangilaPredResParams& p, cudaStream_t stream) {
-  constexpr bool LEAN = MODE == 2 || MODE == 3 || MODE == 5 || MODE == 7;
+  constexpr bool LEAN = MODE == 2 || MODE == 3 || MODE == 7;
   constexpr int smem = MODE == 0 ? 0 : kWarps * Ring<T, S, LEAN>::BYTES_PER_WARP;
   static_assert(Ring<T, S, LEAN>::D <= kMaxDepth, "ring depth");
   const void* fn = reinterpret_cast<const void*>(&predres_bucket_kernel<T, S, MODE>);
@@ -923,11 +994,25 @@ cudaError_t launch_mode(const NangilaPredResParams& p, cudaStream_t stream) {
   return cudaLaunchKernel(fn, grid, block, args, size_t(smem), stream);
 }
 
+template <typename T, typename S, bool LEAN>
+cudaError_t launch_single(const NangilaPredResParams& p, cudaStream_t stream) {
+  if ((p.phase_mask & 7) != 0 && (p.phase_mask & 1) == 0) return cudaSuccess;  // there is only a first phase
+  // With statistics a CTA ends in a block-wide sum and atomics on five words that all CTAs share, so it takes up to eight tiles, but
+  // never so many that fewer than about three waves of CTAs are left.
+  const int64_t total = (p.n + kElemsPerIter - 1) / kElemsPerIter;
+  const int tiles = LEAN ? kLeanTiles : int(std::min<int64_t>(8, std::max<int64_t>(1, total / 1600)));
+  int64_t ctas = (total + tiles - 1) / tiles;
+  if (p.grid_x > 0 && p.grid_x < p.nchunks) ctas = std::min<int64_t>(ctas, p.grid_x);  // fewer CTAs than chunks: a cap
+  if (ctas > 0x7fffffffll) return cudaErrorInvalidValue;
+  predres_single_kernel<T, S, LEAN><<<unsigned(ctas), kThreads, 0, stream>>>(p, tiles);
+  return cudaGetLastError();
+}
+
 template <typename T, typename S>
 cudaError_t launch_ts(const NangilaPredResParams& p, cudaStream_t stream) {
   bool lean = p.mode == 0 && p.measure == 0;
   for (int v = 0; v < p.nvr; ++v) lean = lean && p.pred_gain[v] == 0.0f;
-  if (p.mode == 0 && p.world == 1) return lean ? launch_mode<T, S, 5>(p, stream) : launch_mode<T, S, 4>(p, stream);
+  if (p.mode == 0 && p.world == 1) return lean ? launch_single<T, S, true>(p, stream) : launch_single<T, S, false>(p, stream);
   if (p.mode == 0 && p.gather != 0) return lean ? launch_mode<T, S, 7>(p, stream) : launch_mode<T, S, 6>(p, stream);
   if (p.mode == 0) return lean ? launch_mode<T, S, 3>(p, stream) : launch_mode<T, S, 1>(p, stream);
   if (p.mode == 1) return launch_mode<T, S, 0>(p, stream);
