@@ -161,18 +161,14 @@ at::Tensor to_device_descs(const std::vector<Desc>& v, const at::Device& dev) {
 at::Tensor sculptor_layer_sumsq(const std::vector<at::Tensor>& layers) {
   TORCH_CHECK(!layers.empty(), "nangila: no layers");
   std::vector<NangilaLayerDesc> d(layers.size());
-  int64_t mx = 1;
   for (size_t i = 0; i < layers.size(); ++i) {
     TORCH_CHECK(layers[i].is_cuda() && layers[i].is_contiguous(), "nangila: layers must be contiguous CUDA tensors");
     d[i] = NangilaLayerDesc{layers[i].data_ptr(), layers[i].numel(), dtype_code(layers[i]), 0};
-    mx = std::max<int64_t>(mx, layers[i].numel());
   }
   c10::cuda::CUDAGuard guard(layers[0].device());
-  at::Tensor descs = to_device_descs(d, layers[0].device());
   auto out = at::zeros({int64_t(layers.size())}, layers[0].options().dtype(at::kDouble));
-  check_launch(nangila_sculptor_layer_sumsq(reinterpret_cast<const NangilaLayerDesc*>(descs.data_ptr()),
-                                            int32_t(layers.size()), mx, out.data_ptr<double>(),
-                                            at::cuda::getCurrentCUDAStream()), "sculptor_layer_sumsq");
+  check_launch(nangila_sculptor_layer_sumsq_host(d.data(), int32_t(layers.size()), out.data_ptr<double>(),
+                                                 at::cuda::getCurrentCUDAStream()), "sculptor_layer_sumsq");
   return out;
 }
 std::vector<NangilaPairDesc> pair_descs(const std::vector<at::Tensor>& xi, const std::vector<at::Tensor>& xj,
@@ -198,9 +194,7 @@ void sculptor_pair_update(const std::vector<at::Tensor>& xi, const std::vector<a
   int64_t mx;
   auto d = pair_descs(xi, xj, state, count_after, &mx);
   c10::cuda::CUDAGuard guard(xi[0].device());
-  at::Tensor descs = to_device_descs(d, xi[0].device());
-  check_launch(nangila_sculptor_pair_update(reinterpret_cast<const NangilaPairDesc*>(descs.data_ptr()), int32_t(d.size()),
-                                            mx, at::cuda::getCurrentCUDAStream()), "sculptor_pair_update");
+  check_launch(nangila_sculptor_pair_update_host(d.data(), int32_t(d.size()), at::cuda::getCurrentCUDAStream()), "sculptor_pair_update");
 }
 at::Tensor sculptor_pair_finalize(const std::vector<at::Tensor>& state, const std::vector<int64_t>& count) {
   std::vector<at::Tensor> dummy;

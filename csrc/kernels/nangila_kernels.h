@@ -182,7 +182,7 @@ uint32_t nangila_dgc_scratch_words(void);
 int nangila_dgc_launch(const NangilaDgcParams* p, cudaStream_t stream);
 
 /* ---- Sculptor calibration statistics (sculptor_stats.cu) -----------------------------------------------
- * Descriptor arrays live in DEVICE memory. */
+ * Descriptor arrays live in DEVICE memory, or in HOST memory for the functions ending in _host, which copy them into the launch. */
 typedef struct NangilaLayerDesc {
   const void* data;
   int64_t numel;
@@ -200,6 +200,8 @@ typedef struct NangilaPairDesc {
 int nangila_sculptor_layer_sumsq(const NangilaLayerDesc* layers, int32_t nlayers, int64_t max_numel, double* out,
                                  cudaStream_t stream);
 int nangila_sculptor_pair_update(const NangilaPairDesc* pairs, int32_t npairs, int64_t max_numel, cudaStream_t stream);
+int nangila_sculptor_layer_sumsq_host(const NangilaLayerDesc* layers, int32_t nlayers, double* out, cudaStream_t stream);
+int nangila_sculptor_pair_update_host(const NangilaPairDesc* pairs, int32_t npairs, cudaStream_t stream);
 int nangila_sculptor_pair_finalize(const NangilaPairDesc* pairs, int32_t npairs, int64_t max_numel, double* out,
                                    cudaStream_t stream);
 
