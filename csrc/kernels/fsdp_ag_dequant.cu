@@ -17,6 +17,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "launch_util.cuh"
 #include "nangila_kernels.h"
 #include "quant.cuh"
@@ -35,6 +37,12 @@ constexpr int kPerIter = kThreads * kE;  // 2048
 __host__ __device__ inline uint64_t ag_slot_bytes(int chunk, int bits) {
   return uint64_t(chunk) * bits / 8 + uint64_t(chunk) / kQuantBlock * 2;
 }
+
+// eight values as they lie in memory
+template <typename T>
+struct __align__(16) Raw {
+  T v[kE];
+};
 
 template <typename T, int BITS>
 __global__ void __launch_bounds__(kThreads, 4) fsdp_ag_kernel(const __grid_constant__ NangilaAgParams p) {
@@ -62,10 +70,9 @@ __global__ void __launch_bounds__(kThreads, 4) fsdp_ag_kernel(const __grid_const
     if (task < cps) {
       // ---- quantize chunk `task` of my shard and store it into every rank's slot [me][task] ----
       const int j = task;
-      for (int it = 0; it < iters; ++it) {
-        const int64_t local = int64_t(j) * C + int64_t(it) * kPerIter + tid * kE;
+      auto quantize = [&](int it, const Raw<T>& raw) {
         float x[kE];
-        load8_guarded<T>(in, local, shard, x);
+        Vec8<T>::load(reinterpret_cast<const T*>(&raw), x);
         float amax = 0.0f;
 #pragma unroll
         for (int i = 0; i < kE; ++i) {
@@ -98,6 +105,20 @@ __global__ void __launch_bounds__(kThreads, 4) fsdp_ag_kernel(const __grid_const
           if ((tid & 7) == 0)
             reinterpret_cast<uint16_t*>(dst + uint64_t(C) * BITS / 8)[it * (kPerIter / kQuantBlock) + tid / 8] = uint16_t(sb);
         }
+      };
+      // The loads of kBatch iterations are issued before the first is used (the stores into the slots may alias the shard as far as
+      // the compiler knows). The shard is a multiple of 8: a lane has eight values or none.
+      constexpr int kBatch = sizeof(T) == 2 ? 4 : 2;
+      for (int it0 = 0; it0 < iters; it0 += kBatch) {
+        Raw<T> raw[kBatch];
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) {
+          const int64_t local = int64_t(j) * C + int64_t(it0 + b) * kPerIter + tid * kE;
+          raw[b] = it0 + b < iters && local < shard ? *reinterpret_cast<const Raw<T>*>(in + local) : Raw<T>{};
+        }
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b)
+          if (it0 + b < iters) quantize(it0 + b, raw[b]);
       }
       __syncthreads();
       if (tid < W) {
@@ -170,6 +191,19 @@ extern "C" uint64_t nangila_ag_region_bytes(int64_t shard_elems, int32_t world, 
   if (flag_off) *flag_off = off;
   off = align(off + uint64_t(world) * cps * 4);
   return off;
+}
+
+// Chunk size for a shard. A rank has one quantize task per chunk and W dequantize tasks, walked by the CTAs the device holds at
+// once (`resident` per rank): the largest chunk that still gives every CTA a quantize task, in whole iterations, since each
+// task ends in a block barrier and a system-wide flag (four ranks, 3.1 M bf16 elements each: chunks of 4096 elements 120 us,
+// 8192 78, 24576 59, 32768 64). Not below 4096 elements, where a task is nearly all barrier and flag (131 072 elements on four ranks:
+// 19.7 us, 21.4 with 2048), except for shards of less than four such chunks.
+extern "C" int32_t nangila_ag_chunk_elems(int64_t shard_elems, int32_t resident) {
+  const int64_t g = resident > 0 ? resident : 1, most = 131072;
+  const int64_t waves = std::max<int64_t>(1, (shard_elems + g * most - 1) / (g * most));
+  const int64_t per = (shard_elems + g * waves - 1) / (g * waves);
+  const int64_t least = (shard_elems < 4 * 4096 ? 1 : 2) * nangila::kPerIter;
+  return int32_t(std::min<int64_t>(most, std::max<int64_t>(least, (per + nangila::kPerIter - 1) / nangila::kPerIter * nangila::kPerIter)));
 }
 
 extern "C" int nangila_ag_launch(const NangilaAgParams* p, cudaStream_t stream) {

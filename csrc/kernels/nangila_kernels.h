@@ -104,6 +104,7 @@ typedef struct NangilaAgParams {
 } NangilaAgParams;
 uint64_t nangila_ag_region_bytes(int64_t shard_elems, int32_t world, int32_t chunk_elems, int32_t bits,
                                  uint64_t* recv_off, uint64_t* flag_off);
+int32_t nangila_ag_chunk_elems(int64_t shard_elems, int32_t resident_ctas);
 int nangila_ag_launch(const NangilaAgParams* p, cudaStream_t stream);
 
 /* ---- PowerSGD on tcgen05 tensor cores (powersgd_tcgen05.cu) ------------------------------------------------ */

@@ -39,20 +39,6 @@ except Exception:  # pragma: no cover - older torch
     ReduceScatter = object  # type: ignore
 
 
-def _chunk_for(shard: int, per_shard: int = 1024, cap: int = 131072) -> int:
-    """Chunk size for a shard: the power of two at or above shard / per_shard in [4096, cap] (every chunk
-    costs a flag round trip), halved while the shard would give fewer than 4 chunks, never below 2048."""
-    env = os.environ.get("NANGILA_CHUNK")
-    if env:
-        return int(env)
-    c = 4096
-    while c < cap and c * per_shard < shard:
-        c *= 2
-    while c > 2048 and shard < 4 * c:
-        c //= 2
-    return c
-
-
 class _Base:
     def __init__(self, arena=None, group: Optional[dist.ProcessGroup] = None, device: Optional[torch.device] = None,
                  timeout_s: Optional[float] = None):
@@ -297,7 +283,9 @@ class NangilaAllGather(_Base, AllGather):
         key = (shard, inputs[0].dtype)
         st = self._regions.get(key)
         if st is None:
-            chunk = _chunk_for(shard)
+            env = os.environ.get("NANGILA_CHUNK")
+            resident = max(1, int(self._glue.predres_resident_ctas()) // self.nvr)
+            chunk = int(env) if env else int(self._glue.ag_chunk_elems(shard, resident))
             total, r, f = self._glue.ag_region_layout(shard, self.world, chunk, self.bits)
             st = dict(region=arena.allocate(int(total)), r=r, f=f, chunk=chunk, epoch=0)
             self._regions[key] = st
