@@ -21,7 +21,7 @@ enum StatusWord : int {
   kStatusSeen = 4,    // last flag value it saw
   kStatusPhase = 5,   // kernel phase (1, 2, 3)
   kStatusChunk = 6,   // chunk / task index
-  kStatusBarrier = 7, // counter of the in-kernel grid barrier (kernels launched without a cooperative launch)
+  // word 7 is not used
   kStatusWords = 8,
 };
 enum StatusCode : uint32_t {

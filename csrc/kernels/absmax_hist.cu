@@ -42,7 +42,7 @@ absmax_hist_kernel(const T* __restrict__ x, int64_t n, uint32_t k, float qmax, u
                    uint32_t* hist256) {
   cg::grid_group grid = cg::this_grid();
   __shared__ uint32_t sh[kBins0];
-  __shared__ uint32_t sel[2];
+  __shared__ uint32_t sel[10];
   const int64_t t0 = int64_t(blockIdx.x) * kThreads + threadIdx.x, stride = int64_t(gridDim.x) * kThreads;
   for (int i = int(t0); i < kWords; i += int(stride)) scratch[i] = 0u;
   grid.sync();
@@ -68,7 +68,7 @@ absmax_hist_kernel(const T* __restrict__ x, int64_t n, uint32_t k, float qmax, u
     if (sh[i]) atomicAdd(&scratch[kH0 + i], sh[i]);
   grid.sync();
   uint32_t want = k, b0, b1, b2, dummy = 0;
-  select_bin(scratch + kH0, kBins0, want, b0, sel);
+  select_bin<kBins0>(scratch + kH0, want, b0, sel);
   for (int i = threadIdx.x; i < kBins1; i += kThreads) sh[i] = 0u;
   __syncthreads();
   for (int64_t i = t0; i < n; i += stride) {
@@ -79,7 +79,7 @@ absmax_hist_kernel(const T* __restrict__ x, int64_t n, uint32_t k, float qmax, u
   for (int i = threadIdx.x; i < kBins1; i += kThreads)
     if (sh[i]) atomicAdd(&scratch[kH1 + i], sh[i]);
   grid.sync();
-  select_bin(scratch + kH1, kBins1, want, b1, sel);
+  select_bin<kBins1>(scratch + kH1, want, b1, sel);
   const uint32_t prefix = (b0 << 11) | b1;
   const float vmax = __uint_as_float(scratch[kMax]);
   const float inv = vmax > 0.0f ? 255.999f / vmax : 0.0f;
@@ -94,7 +94,7 @@ absmax_hist_kernel(const T* __restrict__ x, int64_t n, uint32_t k, float qmax, u
   for (int i = threadIdx.x; i < kBins2 + 256; i += kThreads)
     if (sh[i]) atomicAdd(&scratch[kH2 + i], sh[i]);  // kLin == kH2 + kBins2
   grid.sync();
-  select_bin(scratch + kH2, kBins2, want, b2, sel);
+  select_bin<kBins2>(scratch + kH2, want, b2, sel);
   if (blockIdx.x == 0) {
     if (threadIdx.x == 0) {
       const float kth = __uint_as_float((prefix << 9) | b2);

@@ -11,17 +11,24 @@
 // accumulation.
 //
 // Phases (grid-wide barriers between them: hardware barriers of a cooperative launch in the single-GPU
-// loopback world, counter barriers with a time limit otherwise, see comm/signal.cuh):
-//   0  clear the scratch histograms / cursor
-//   1  u = m u + g ; v = v + u ; histogram of bits [30:20] of |v|
-//   2  histogram of bits [19:9] among elements whose top bits equal the selected bin
-//   3  histogram of bits [8:0]  among elements matching both        -> threshold bit pattern tau
-//   4  compaction: every element with |v| >= tau is appended to the local send list (bounded by the
-//      list capacity), u and v are zeroed there; the dense bucket is zeroed
-//   5  the list is copied into every rank's receive slot for this rank, then a flag is released
-//   6  wait (bounded) for every rank's list, add value / W into the bucket, list by list in rank order
-// The selection is exact: tau is the k-th largest |v|. Elements equal to tau are all selected, so
+// loopback world, counter barriers with a time limit otherwise, see comm/signal.cuh; the launcher clears the scratch words):
+//   1  u = m u + g ; v = v + u ; the dense bucket is zeroed. Entries a little below the previous threshold and up, the candidates, are
+//      listed, with a histogram of their distance from that bound in steps of 4096 units in the last place
+//   2  histogram of the last 12 bits among the candidates of the selected step                   -> threshold bit pattern tau
+//   3  compaction: every candidate with |v| >= tau is appended to the send list (bounded by the list capacity), u and v are
+//      zeroed there. A group of one rank writes the bucket here and is done
+//   4  the list is copied into every rank's receive slot for this rank, then a flag is released
+//   5  wait (bounded) for every rank's list, add value / W into the bucket, list by list in rank order
+// Without a previous threshold, or if the list does not hold the k largest for sure (fewer than k candidates,
+// no room for all of them, a threshold above twice the bound), the threshold comes from a three-pass radix select over
+// the dense state (bits [30:20], [19:9], [8:0]; the first histogram is built in phase 1 if there is no previous threshold).
+// The selection is exact either way: tau is the k-th largest |v|. Elements equal to tau are all selected, so
 // with ties the list can be longer than k (it is cut at the capacity; what is cut stays in v).
+//
+// What bounds it: phase 1 is HBM (20 bytes an element with a bf16 bucket); what follows is latency, about 2.5 us a barrier and 1.5
+// a selection. Measured on B200, one rank, bf16, launch included: 13.1 M elements 155 -> 100 us while the threshold grows, 195 -> 84 once it
+// has settled; 1.05 M 80 -> 53. Before, phase 1 also voted every element into a histogram, the selections walked their bins with
+// one warp (45 us), there were eight barriers, and the settled list (36 k entries) often had no room.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -43,12 +50,22 @@ using namespace rsel;
 
 constexpr int kThreads = 256;
 
-// scratch layout (uint32 words)
+// scratch layout (uint32 words), the first kClearWords cleared before the launch; the candidate list (index, bits pairs) follows
 constexpr int kHist0 = 0, kHist1 = kHist0 + kBins0, kHist2 = kHist1 + kBins1;
 constexpr int kCursor = kHist2 + kBins2;  // number of selected entries
 constexpr int kCandCount = kCursor + 1;   // candidates collected in phase 1, summed over the CTAs
-constexpr int kCandOverflow = kCursor + 4;  // non-zero if a CTA ran out of room for its candidates
-constexpr int kScratchWords = kCursor + 8;  // the candidate list (index, bits pairs) follows
+constexpr int kPath = kCursor + 2;        // telemetry: 1 if the selection ran on the list, then the candidates seen
+constexpr int kBarrierWord = kCursor + 5;   // counter of the grid barriers of a plain launch
+constexpr int kDone = kCursor + 6;          // CTAs that are through (a group of one rank)
+constexpr int kSpill = kCursor + 7;         // candidates that found their CTA's segment full
+constexpr int kCoarse = kCursor + 8;        // candidates by distance from the bound, kStep apart
+constexpr int kStepBits = 12, kCoarseBins = 2048, kFineBins = 1 << kStepBits;
+constexpr int kFine = kCoarse + kCoarseBins;  // the selected step's candidates by distance
+constexpr int kClearWords = kFine + kFineBins;
+// kept from launch to launch (whatever is there at first does no harm): a threshold, and the bound for the launch after it
+constexpr int kKept = kClearWords;
+constexpr int kScratchWords = kClearWords + 8;
+constexpr uint32_t kBand = 4;  // candidates wanted, in multiples of k
 
 template <typename T>
 __device__ __forceinline__ float ldf(const T* p, int64_t i) { return dev::Vec16<T>::to_float(p[i]); }
@@ -90,7 +107,7 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
   // real process group a counter barrier over the CTAs of this launch, so the kernel needs no cooperative
   // launch, can start while backward still holds part of the GPU, and runs with a capped number of CTAs.
   const bool coop = p.nvr > 1;
-  GridBarrier soft(p.status[vr] + kStatusBarrier, gridDim.x);
+  GridBarrier soft(p.scratch[vr] + kBarrierWord, gridDim.x);
   auto gsync = [&]() -> bool {
     if (coop) {
       grid.sync();
@@ -111,7 +128,7 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
   const uint64_t slot_bytes = 16 + uint64_t(cap) * 8;
   // Two sets of receive slots, used alternately by epoch parity: a rank that runs one launch ahead
   // writes the other set while a slower peer may still be scattering from this one; it cannot get
-  // two launches ahead because its wait in phase 6 needs the peer's flag of the launch in between.
+  // two launches ahead because its wait in phase 5 needs the peer's flag of the launch in between.
   const uint64_t recv_base = p.recv_off + uint64_t(p.epoch & 1u) * uint64_t(W) * slot_bytes;
   // local send list lives in this rank's own receive slot for itself
   uint8_t* myslot = myreg + recv_base + uint64_t(me) * slot_bytes;
@@ -119,7 +136,7 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
   float* my_val = reinterpret_cast<float*>(myslot + 16 + uint64_t(cap) * 4);
 
   __shared__ uint32_t sh_hist[kBins0];
-  __shared__ uint32_t sh_sel[2];
+  __shared__ uint32_t sh_sel[10];
   __shared__ uint32_t sh_cand_cnt;  // candidates this CTA has appended to its segment of the list
   const int64_t tid0 = int64_t(blockIdx.x) * kThreads + threadIdx.x;
   const int64_t stride = int64_t(gridDim.x) * kThreads;
@@ -129,50 +146,76 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
   const int64_t groups = (n + 3) / 4;                // including the ragged last one
   const int64_t groups_rounded = (groups + 31) / 32 * 32;
 
-  // Candidates. Between two calls on the same bucket the threshold moves little, so phase 1 also
-  // collects every entry with |v| >= 0.96 * (previous threshold) into a short list (unsent entries
-  // pile up just below the threshold, so the band has to be narrow). If that list holds
-  // at least k entries and did not overflow, the k largest entries of the bucket are all in it and the
-  // three selection passes and the compaction run over the list (a few thousand entries) instead of
-  // the dense state; otherwise (first call, threshold moved a lot) the dense passes run as before.
+  // Candidates. Between two calls on the same bucket the threshold moves little, so the k largest entries are nearly always among
+  // those above a bound a little below the previous threshold, a few thousand to look through instead of the dense state. The bound
+  // is 0.96 of the threshold, or the value that 4 k entries were above last time if that is higher: unsent entries pile up just
+  // below the threshold, and once the threshold has settled 36 k lie within 4 % of it.
   const uint32_t tau_prev = p.out_count[vr][1];
   const uint32_t cand_cap = p.cand_capacity;
-  const uint32_t cand_thr = (cand_cap > 0 && tau_prev > 0 && tau_prev < 0x7f800000u)
-                                ? __float_as_uint(__uint_as_float(tau_prev) * 0.96f)
-                                : 0xffffffffu;  // nothing qualifies
-  const uint32_t seg_cap = cand_cap / gridDim.x;  // entries per CTA
+  const bool use_list = cand_cap > 0 && tau_prev > 0 && tau_prev < 0x7f800000u;
+  uint32_t cand_thr = 0xffffffffu;  // nothing qualifies
+  if (use_list) {
+    cand_thr = __float_as_uint(__uint_as_float(tau_prev) * 0.96f);
+    if (scratch[kKept] == tau_prev && scratch[kKept + 1] <= tau_prev) cand_thr = max(cand_thr, scratch[kKept + 1]);
+  }
+  // Half of the list is cut into a segment per CTA, which fills it without asking anybody; the candidates are not spread evenly (layers
+  // have gradients of different size), so what finds its segment full goes to the other half, place by place.
+  const uint32_t seg_cap = cand_cap / 2 / gridDim.x;
+  const uint32_t spill_cap = cand_cap - seg_cap * gridDim.x;
   uint32_t* cand_idx = scratch + kScratchWords + uint64_t(blockIdx.x) * seg_cap;
   uint32_t* cand_bits = cand_idx + cand_cap;
+  uint32_t* spill_idx = scratch + kScratchWords + uint64_t(gridDim.x) * seg_cap;
+  uint32_t* spill_bits = spill_idx + cand_cap;
 
-  // ---- phase 0 ----
-  for (int i = int(tid0); i < kScratchWords; i += int(stride)) scratch[i] = 0u;
   if (threadIdx.x == 0) sh_cand_cnt = 0u;
-  if (!gsync()) return;
 
-  // ---- phase 1: momentum correction + histogram of bits [30:20] ----
+  // ---- phase 1: momentum correction, candidates (or the first histogram) ----
   for (int i = threadIdx.x; i < kBins0; i += kThreads) sh_hist[i] = 0u;
   __syncthreads();
-  for (int64_t q = tid0; q < groups_rounded; q += stride) {
-    float vn[4];
+  auto collect = [&](int64_t i, float v_new) {  // few entries qualify: only the lanes that have one meet in here
+    const uint32_t b = __float_as_uint(v_new) & 0x7fffffffu;
+    if (b >= cand_thr) {
+      const uint32_t here = __activemask(), lane = threadIdx.x & 31;
+      const int leader = __ffs(here) - 1;
+      uint32_t pos = 0;
+      if (int(lane) == leader) pos = atomicAdd(&sh_cand_cnt, uint32_t(__popc(here)));
+      pos = __shfl_sync(here, pos, leader) + uint32_t(__popc(here & ((1u << lane) - 1u)));
+      if (pos < seg_cap) {
+        cand_idx[pos] = uint32_t(i);
+        cand_bits[pos] = b;
+      } else {
+        pos = atomicAdd(&scratch[kSpill], 1u);
+        if (pos < spill_cap) {
+          spill_idx[pos] = uint32_t(i);
+          spill_bits[pos] = b;
+        }
+      }
+      atomicAdd(&sh_hist[min((b - cand_thr) >> kStepBits, uint32_t(kCoarseBins - 1))], 1u);
+    }
+  };
+  const int64_t n8 = n / 8, groups8 = (n + 7) / 8, groups8_rounded = (groups8 + 31) / 32 * 32;
+  for (int64_t q = tid0; q < groups8_rounded; q += stride) {
+    float vn[8];
     int valid = 0;
-    if (q < n4) {
-      float g[4];
-      ld4<T>(grad, q * 4, g);
-      float4 uu = *reinterpret_cast<const float4*>(u + q * 4);
-      float4 vv = *reinterpret_cast<const float4*>(v + q * 4);
-      uu.x = __fmaf_rn(p.momentum, uu.x, dev::sanitize(g[0]));
-      uu.y = __fmaf_rn(p.momentum, uu.y, dev::sanitize(g[1]));
-      uu.z = __fmaf_rn(p.momentum, uu.z, dev::sanitize(g[2]));
-      uu.w = __fmaf_rn(p.momentum, uu.w, dev::sanitize(g[3]));
-      vv.x += uu.x; vv.y += uu.y; vv.z += uu.z; vv.w += uu.w;
-      *reinterpret_cast<float4*>(u + q * 4) = uu;
-      *reinterpret_cast<float4*>(v + q * 4) = vv;
-      st4_zero<T>(grad, q * 4);  // the dense result starts from zero; phase 6 scatters into it
-      vn[0] = vv.x; vn[1] = vv.y; vn[2] = vv.z; vn[3] = vv.w;
-      valid = 4;
-    } else if (q < groups) {
-      for (int k = 0; k < 4; ++k) {
-        const int64_t i = q * 4 + k;
+    if (q < n8) {
+      float g[8], uu[8];
+      ld4<T>(grad, q * 8, reinterpret_cast<float (&)[4]>(g[0]));
+      ld4<T>(grad, q * 8 + 4, reinterpret_cast<float (&)[4]>(g[4]));
+      dev::Vec8<float>::load(u + q * 8, uu);
+      dev::Vec8<float>::load(v + q * 8, vn);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        uu[k] = __fmaf_rn(p.momentum, uu[k], dev::sanitize(g[k]));
+        vn[k] += uu[k];
+      }
+      dev::Vec8<float>::store(u + q * 8, uu);
+      dev::Vec8<float>::store(v + q * 8, vn);
+      st4_zero<T>(grad, q * 8);  // the dense result starts from zero
+      st4_zero<T>(grad, q * 8 + 4);
+      valid = 8;
+    } else if (q < groups8) {
+      for (int k = 0; k < 8; ++k) {
+        const int64_t i = q * 8 + k;
         vn[k] = 0.0f;
         if (i < n) {
           const float un = __fmaf_rn(p.momentum, u[i], dev::sanitize(ldf(grad, i)));
@@ -184,89 +227,96 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
         }
       }
     }
+    if (use_list) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint32_t b = __float_as_uint(vn[k]) & 0x7fffffffu;
-      hist_add(sh_hist, b >> 20, k < valid);
-      const bool cand = k < valid && b >= cand_thr;
-      const uint32_t mask = __ballot_sync(0xffffffffu, cand);
-      if (mask) {
-        const int lane = threadIdx.x & 31;
-        uint32_t base = 0;
-        if (lane == __ffs(mask) - 1) base = atomicAdd(&sh_cand_cnt, uint32_t(__popc(mask)));
-        base = __shfl_sync(0xffffffffu, base, __ffs(mask) - 1);
-        if (cand) {
-          const uint32_t pos = base + uint32_t(__popc(mask & ((1u << lane) - 1u)));
-          if (pos < seg_cap) {
-            cand_idx[pos] = uint32_t(q * 4 + k);
-            cand_bits[pos] = b;
-          }
-        }
-      }
+      for (int k = 0; k < 8; ++k)
+        if (k < valid) collect(q * 8 + k, vn[k]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) hist_add(sh_hist, (__float_as_uint(vn[k]) & 0x7fffffffu) >> 20, k < valid);
     }
   }
   __syncthreads();
+  static_assert(kCoarseBins == kBins0, "one histogram in shared memory for either");
+  const int first_hist = use_list ? kCoarse : kHist0;
   for (int i = threadIdx.x; i < kBins0; i += kThreads)
-    if (sh_hist[i]) atomicAdd(&scratch[kHist0 + i], sh_hist[i]);
+    if (sh_hist[i]) atomicAdd(&scratch[first_hist + i], sh_hist[i]);
   const uint32_t my_cand = min(sh_cand_cnt, seg_cap);  // entries of this CTA's segment
-  if (threadIdx.x == 0) {
-    atomicAdd(&scratch[kCandCount], my_cand);
-    if (sh_cand_cnt > seg_cap) atomicOr(&scratch[kCandOverflow], 1u);
-  }
+  if (threadIdx.x == 0) atomicAdd(&scratch[kCandCount], my_cand);
   if (!gsync()) return;
   uint32_t want = p.k, bin0, bin1, bin2;
-  select_bin(scratch + kHist0, kBins0, want, bin0, sh_sel);
-
-  const uint32_t ncand = scratch[kCandCount];
-  const bool from_list = seg_cap > 0 && ncand >= p.k && scratch[kCandOverflow] == 0u;  // same on every CTA
+  const uint32_t nspill = __ldcg(scratch + kSpill), ncand = __ldcg(scratch + kCandCount) + nspill;
+  bool from_list = use_list && ncand >= p.k && nspill <= spill_cap;  // same on every CTA
+  uint32_t coarse = 0;
+  if (from_list) {
+    select_bin<kCoarseBins>(scratch + kCoarse, want, coarse, sh_sel);
+    from_list = coarse < uint32_t(kCoarseBins - 1);  // the last one holds everything from there on
+  }
+  // Appends the entries that the lanes of a warp have selected to the send list, and takes them out of the state.
+  const float inv_w = 1.0f / float(W);
+  auto append = [&](bool sel, int64_t i) {
+    const uint32_t mask = __ballot_sync(0xffffffffu, sel);
+    if (mask == 0u) return;
+    const int lane = threadIdx.x & 31;
+    uint32_t base = 0;
+    if (lane == __ffs(mask) - 1) base = atomicAdd(&scratch[kCursor], uint32_t(__popc(mask)));
+    base = __shfl_sync(0xffffffffu, base, __ffs(mask) - 1);
+    if (sel) {
+      const uint32_t pos = base + uint32_t(__popc(mask & ((1u << lane) - 1u)));
+      if (pos < cap) {
+        const float x = v[i];
+        my_idx[pos] = uint32_t(i);
+        my_val[pos] = x;
+        v[i] = 0.0f;
+        u[i] = 0.0f;
+        if (W == 1) grad[i] = dev::Vec16<T>::from_float(__fmaf_rn(x, inv_w, 0.0f));  // nobody else's entries to add
+      }
+    }
+  };
+  // The ranks of a cooperative launch share its barriers but not their choice of path: there, every path passes kSelectSyncs.
+  constexpr int kSelectSyncs = 3;
+  int select_syncs = 0;
+  auto ssync = [&]() -> bool {
+    ++select_syncs;
+    return gsync();
+  };
+  auto even_out = [&] {
+    if (coop)
+      for (; select_syncs < kSelectSyncs; ++select_syncs) grid.sync();
+  };
   uint32_t tau;
   if (from_list) {
-    // ---- phases 2-4 over the candidate list ----
-    for (int i = threadIdx.x; i < kBins1; i += kThreads) sh_hist[i] = 0u;
-    __syncthreads();
-    const uint32_t nc_rounded = (my_cand + 31u) / 32u * 32u;  // this CTA scans its own segment
-    for (uint32_t j = threadIdx.x; j < nc_rounded; j += kThreads) {
-      const uint32_t b = j < my_cand ? cand_bits[j] : 0xffffffffu;
-      hist_add(sh_hist, (b >> 9) & 0x7ffu, b != 0xffffffffu && (b >> 20) == bin0);
+    // ---- phases 2 and 3 over the candidate list: this CTA scans its own segment ----
+    auto count_fine = [&](uint32_t bits) {
+      const uint32_t d = bits - cand_thr;
+      if ((d >> kStepBits) == coarse) atomicAdd(&scratch[kFine + (d & (kFineBins - 1))], 1u);
+    };
+    for (uint32_t j = threadIdx.x; j < my_cand; j += kThreads) count_fine(cand_bits[j]);
+    for (uint32_t j = uint32_t(tid0); j < nspill; j += uint32_t(stride)) count_fine(__ldcg(spill_bits + j));
+    uint32_t next_bound = 0;
+    if (blockIdx.x == 0) {
+      uint32_t rank = min(kBand * p.k, ncand), bin;
+      select_bin<kCoarseBins>(scratch + kCoarse, rank, bin, sh_sel);
+      next_bound = cand_thr + (bin << kStepBits);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kBins1; i += kThreads)
-      if (sh_hist[i]) atomicAdd(&scratch[kHist1 + i], sh_hist[i]);
-    if (!gsync()) return;
-    select_bin(scratch + kHist1, kBins1, want, bin1, sh_sel);
-    for (int i = threadIdx.x; i < kBins2; i += kThreads) sh_hist[i] = 0u;
-    __syncthreads();
-    const uint32_t prefix = (bin0 << 11) | bin1;
-    for (uint32_t j = threadIdx.x; j < nc_rounded; j += kThreads) {
-      const uint32_t b = j < my_cand ? cand_bits[j] : 0xffffffffu;
-      hist_add(sh_hist, b & 0x1ffu, b != 0xffffffffu && (b >> 9) == prefix);
+    if (!ssync()) return;
+    uint32_t fine;
+    select_bin<kFineBins>(scratch + kFine, want, fine, sh_sel);
+    tau = cand_thr + (coarse << kStepBits) + fine;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // every CTA has read the old pair before the first barrier
+      scratch[kKept] = tau;
+      scratch[kKept + 1] = next_bound;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kBins2; i += kThreads)
-      if (sh_hist[i]) atomicAdd(&scratch[kHist2 + i], sh_hist[i]);
-    if (!gsync()) return;
-    select_bin(scratch + kHist2, kBins2, want, bin2, sh_sel);
-    tau = (prefix << 9) | bin2;
+    even_out();
+    const uint32_t nc_rounded = (my_cand + 31u) / 32u * 32u;
     for (uint32_t j = threadIdx.x; j < nc_rounded; j += kThreads) {
-      const uint32_t b = j < my_cand ? cand_bits[j] : 0xffffffffu;
-      const bool sel = b != 0xffffffffu && b >= tau && (p.k > 0) && b != 0u;
-      const uint32_t mask = __ballot_sync(0xffffffffu, sel);
-      if (mask) {
-        const int lane = threadIdx.x & 31;
-        uint32_t base = 0;
-        if (lane == __ffs(mask) - 1) base = atomicAdd(&scratch[kCursor], uint32_t(__popc(mask)));
-        base = __shfl_sync(0xffffffffu, base, __ffs(mask) - 1);
-        if (sel) {
-          const uint32_t pos = base + uint32_t(__popc(mask & ((1u << lane) - 1u)));
-          if (pos < cap) {
-            const uint32_t i = cand_idx[j];
-            my_idx[pos] = i;
-            my_val[pos] = v[i];
-            v[i] = 0.0f;
-            u[i] = 0.0f;
-          }
-        }
-      }
+      const bool sel = j < my_cand && cand_bits[j] >= tau && p.k > 0;
+      append(sel, sel ? int64_t(cand_idx[j]) : 0);
+    }
+    const uint32_t ns_rounded = (nspill + 31u) / 32u * 32u;
+    for (uint32_t j = uint32_t(tid0); j < ns_rounded; j += uint32_t(stride)) {
+      const bool sel = j < nspill && __ldcg(spill_bits + j) >= tau && p.k > 0;
+      append(sel, sel ? int64_t(__ldcg(spill_idx + j)) : 0);
     }
   } else {
     // bit patterns of |v| for one group (0 beyond the end: never selected, never counted)
@@ -280,7 +330,25 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
       }
     };
 
-    // ---- phase 2: bits [19:9] ----
+    if (use_list) {
+      // ---- bits [30:20], which phase 1 has left out ----
+      for (int i = threadIdx.x; i < kBins0; i += kThreads) sh_hist[i] = 0u;
+      __syncthreads();
+      for (int64_t q = tid0; q < groups_rounded; q += stride) {
+        uint32_t b[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+        if (q < groups) load_bits(q, b);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) hist_add(sh_hist, b[k] >> 20, b[k] != 0xffffffffu);
+      }
+      __syncthreads();
+      for (int i = threadIdx.x; i < kBins0; i += kThreads)
+        if (sh_hist[i]) atomicAdd(&scratch[kHist0 + i], sh_hist[i]);
+      if (!ssync()) return;
+    }
+    want = p.k;
+    select_bin<kBins0>(scratch + kHist0, want, bin0, sh_sel);
+
+    // ---- bits [19:9] ----
     for (int i = threadIdx.x; i < kBins1; i += kThreads) sh_hist[i] = 0u;
     __syncthreads();
     for (int64_t q = tid0; q < groups_rounded; q += stride) {
@@ -292,10 +360,10 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
     __syncthreads();
     for (int i = threadIdx.x; i < kBins1; i += kThreads)
       if (sh_hist[i]) atomicAdd(&scratch[kHist1 + i], sh_hist[i]);
-    if (!gsync()) return;
-    select_bin(scratch + kHist1, kBins1, want, bin1, sh_sel);
+    if (!ssync()) return;
+    select_bin<kBins1>(scratch + kHist1, want, bin1, sh_sel);
 
-    // ---- phase 3: bits [8:0] ----
+    // ---- bits [8:0] ----
     for (int i = threadIdx.x; i < kBins2; i += kThreads) sh_hist[i] = 0u;
     __syncthreads();
     const uint32_t prefix = (bin0 << 11) | bin1;
@@ -308,49 +376,45 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
     __syncthreads();
     for (int i = threadIdx.x; i < kBins2; i += kThreads)
       if (sh_hist[i]) atomicAdd(&scratch[kHist2 + i], sh_hist[i]);
-    if (!gsync()) return;
-    select_bin(scratch + kHist2, kBins2, want, bin2, sh_sel);
+    if (!ssync()) return;
+    select_bin<kBins2>(scratch + kHist2, want, bin2, sh_sel);
     tau = (prefix << 9) | bin2;  // bit pattern of the k-th largest |v|
 
-    // ---- phase 4: compaction + masking ----
+    even_out();
+
+    // ---- phase 3: compaction ----
     for (int64_t q = tid0; q < groups_rounded; q += stride) {
       uint32_t b[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
       if (q < groups) load_bits(q, b);
-      const int lane = threadIdx.x & 31;
-  #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const bool sel = b[k] != 0xffffffffu && b[k] >= tau && (p.k > 0) && b[k] != 0u;
-        // warp-aggregated append
-        const uint32_t mask = __ballot_sync(0xffffffffu, sel);
-        if (mask) {
-          uint32_t base = 0;
-          if (lane == __ffs(mask) - 1) base = atomicAdd(&scratch[kCursor], uint32_t(__popc(mask)));
-          base = __shfl_sync(0xffffffffu, base, __ffs(mask) - 1);
-          if (sel) {
-            const uint32_t pos = base + uint32_t(__popc(mask & ((1u << lane) - 1u)));
-            if (pos < cap) {
-              const int64_t i = q * 4 + k;
-              my_idx[pos] = uint32_t(i);
-              my_val[pos] = v[i];
-              v[i] = 0.0f;
-              u[i] = 0.0f;
-            }
-          }
-        }
-      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) append(b[k] != 0xffffffffu && b[k] >= tau && (p.k > 0) && b[k] != 0u, q * 4 + k);
     }
   }
-  if (!gsync()) return;
-  const uint32_t count = min(scratch[kCursor], cap);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  auto publish = [&](uint32_t count) {
     *reinterpret_cast<uint32_t*>(myslot) = count;
     p.out_count[vr][0] = count;
     p.out_count[vr][1] = tau;
-    scratch[kCursor + 2] = from_list ? 1u : 0u;  // which selection path ran (telemetry)
-    scratch[kCursor + 3] = ncand;
+    scratch[kPath] = from_list ? 1u : 0u;
+    scratch[kPath + 1] = ncand;
+  };
+  if (W == 1) {
+    // the bucket is complete; the CTA that ends last knows how many entries there were
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (atomicAdd(&scratch[kDone], 1u) == gridDim.x - 1) {
+        __threadfence();
+        publish(min(__ldcg(scratch + kCursor), cap));
+        st_release_sys(reinterpret_cast<uint32_t*>(myreg + p.flag_off) + me, p.epoch);
+      }
+    }
+    return;
   }
+  if (!gsync()) return;
+  const uint32_t count = min(scratch[kCursor], cap);
+  if (blockIdx.x == 0 && threadIdx.x == 0) publish(count);
 
-  // ---- phase 5: copy the list into every other rank's slot for this rank, release flags ----
+  // ---- phase 4: copy the list into every other rank's slot for this rank, release flags ----
   for (int d = 1; d < W; ++d) {
     const int r = (me + d) % W;
     uint8_t* dst = p.region[r] + recv_base + uint64_t(me) * slot_bytes;
@@ -369,12 +433,11 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
     st_release_sys(reinterpret_cast<uint32_t*>(p.region[threadIdx.x] + p.flag_off) + me, p.epoch);
   }
 
-  // ---- phase 6: wait for every rank's list and accumulate it ----
+  // ---- phase 5: wait for every rank's list and accumulate it ----
   // The lists are added in rank order with a grid barrier after each, so every rank performs the same
   // floating-point additions in the same order and all replicas end up with identical bits. Indices
   // inside one list are unique, so no atomics are needed. A CTA whose wait fails keeps taking part in
   // the barriers (skipping the work) so that nobody is left waiting for it.
-  const float inv_w = 1.0f / float(W);
   bool alive = true;
   for (int r = 0; r < W; ++r) {
     bool ok = true;
@@ -430,9 +493,12 @@ extern "C" int nangila_dgc_launch(const NangilaDgcParams* p, cudaStream_t stream
   if (ce != cudaSuccess) return int(ce);
   dim3 grid(unsigned(grid_x), unsigned(p->nvr)), block(kThreads);
   void* args[] = {const_cast<NangilaDgcParams*>(p)};
+  // histograms, cursors and the counter of the in-kernel grid barrier start from zero
+  for (int v = 0; v < p->nvr; ++v) {
+    const cudaError_t me = cudaMemsetAsync(p->scratch[v], 0, sizeof(uint32_t) * kClearWords, stream);
+    if (me != cudaSuccess) return int(me);
+  }
   if (p->nvr > 1) return int(cudaLaunchCooperativeKernel(fn, grid, block, args, 0, stream));
-  // real process group: plain launch; the counter of the in-kernel grid barrier starts from zero
-  const cudaError_t me = cudaMemsetAsync(p->status[0] + comm::kStatusBarrier, 0, sizeof(uint32_t), stream);
-  if (me != cudaSuccess) return int(me);
+  // real process group: plain launch
   return int(cudaLaunchKernel(fn, grid, block, args, 0, stream));
 }

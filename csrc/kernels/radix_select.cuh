@@ -9,41 +9,55 @@ namespace rsel {
 constexpr int kBins0 = 2048, kBins1 = 2048, kBins2 = 512;
 
 // Scanning bins from the top, find the bin that holds the `want`-th largest element (1-based) and
-// reduce `want` to the rank inside that bin. The first warp of the CTA scans; the result is broadcast
-// through `sh` (2 words of shared memory). `hist` must be complete (grid barrier before the call).
-__device__ inline void select_bin(const uint32_t* hist, int nbins, uint32_t& want, uint32_t& bin, uint32_t* sh) {
-  if (threadIdx.x < 32) {
-    uint32_t remaining = want;
-    uint32_t found = 0;
-    bool done = false;
-    for (int base = nbins - 32; base >= 0 && !done; base -= 32) {
-      uint32_t c = hist[base + 31 - threadIdx.x];  // lane 0 = highest bin of this group
-      uint32_t incl = c;
+// reduce `want` to the rank inside that bin; bin 0 if there are fewer elements. All 256 threads of the CTA take part: thread t owns
+// the t-th stretch of bins from the top, a block-wide prefix sum finds the stretch, its owner the bin. (One warp walking down 32 bins
+// at a time waits for L2 at every step: 20 us for a value near 1, whose bin is in the middle; this takes about 1.5.)
+// `sh` is 10 words of shared memory. `hist` must be complete (grid barrier before the call).
+template <int NBINS>
+__device__ inline void select_bin(const uint32_t* hist, uint32_t& want, uint32_t& bin, uint32_t* sh) {
+  constexpr int kPer = NBINS / 256;
+  static_assert(NBINS % 256 == 0, "whole stretches");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int top = NBINS - 1 - tid * kPer;  // highest bin of this thread
+  uint32_t c[kPer], mine = 0;
 #pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
-        if (threadIdx.x >= off) incl += t;
-      }
-      uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-      if (total >= remaining) {
-        uint32_t hit = __ballot_sync(0xffffffffu, incl >= remaining);
-        int lane = __ffs(hit) - 1;
-        uint32_t before = __shfl_sync(0xffffffffu, incl - c, lane);
-        found = uint32_t(base + 31 - lane);
-        remaining -= before;
-        done = true;
-      } else {
-        remaining -= total;
+  for (int i = 0; i < kPer; ++i) {
+    c[i] = __ldcg(hist + top - i);
+    mine += c[i];
+  }
+  uint32_t incl = mine;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += t;
+  }
+  if (lane == 31) sh[warp] = incl;
+  if (tid == 0) sh[8] = 0u;
+  __syncthreads();
+  uint32_t before = incl - mine, all = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    if (w < warp) before += sh[w];
+    all += sh[w];
+  }
+  if (before < want && want <= before + mine) {
+    uint32_t rest = want - before;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      if (rest > 0 && rest <= c[i]) {
+        sh[8] = uint32_t(top - i);
+        sh[9] = rest;
+        rest = 0;
+      } else if (rest > 0) {
+        rest -= c[i];
       }
     }
-    if (threadIdx.x == 0) {
-      sh[0] = found;
-      sh[1] = remaining;
-    }
+  } else if (tid == 0 && want > all) {
+    sh[9] = want - all;
   }
   __syncthreads();
-  bin = sh[0];
-  want = sh[1];
+  bin = sh[8];
+  want = sh[9];
   __syncthreads();
 }
 
