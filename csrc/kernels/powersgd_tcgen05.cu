@@ -152,8 +152,13 @@ psgd_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (row < rows_out) {
         float* dst = out + int64_t(row) * kCols;
         if (use_atomics) {
+          // four columns per reduction; with a push only the factor's columns are ever read
+          const int cols = push.counters != nullptr ? push.rank : kCols;
 #pragma unroll
-          for (int c = 0; c < kCols; ++c) atomicAdd(dst + c, v[c]);
+          for (int c = 0; c < kCols; c += 4)
+            if (c < cols)
+              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + c), "f"(v[c]), "f"(v[c + 1]), "f"(v[c + 2]), "f"(v[c + 3])
+                           : "memory");
         } else {
 #pragma unroll
           for (int c = 0; c < kCols; c += 4) *reinterpret_cast<float4*>(dst + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
@@ -188,20 +193,26 @@ psgd_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         float v[kCols];
 #pragma unroll
         for (int c = 0; c < kCols; c += 4) {
-          const float4 a = __ldcg(reinterpret_cast<const float4*>(out + int64_t(row) * kCols + c));
-          v[c] = a.x; v[c + 1] = a.y; v[c + 2] = a.z; v[c + 3] = a.w;
+          if (c < r) {
+            const float4 a = __ldcg(reinterpret_cast<const float4*>(out + int64_t(row) * kCols + c));
+            v[c] = a.x; v[c + 1] = a.y; v[c + 2] = a.z; v[c + 3] = a.w;
+          }
         }
         for (int d = 0; d < W; ++d) {
           float* dst = reinterpret_cast<float*>(push.region[(push.me + d) % W] + base);
-          for (int c = 0; c < r; ++c) dst[int64_t(c) * rows_out + row] = v[c];   // adjacent rows: adjacent addresses
+#pragma unroll
+          for (int c = 0; c < kCols; ++c)
+            if (c < r) dst[int64_t(c) * rows_out + row] = v[c];   // adjacent rows: adjacent addresses
         }
       }
-      __threadfence_system();
+      if (W > 1) __threadfence_system();
+      else __threadfence();  // nobody outside this GPU reads it
       __syncthreads();
       if (threadIdx.x == 0) {
         const uint32_t tiles = gridDim.x;
         if (atomicAdd(&push.counters[tiles], 1u) == tiles - 1) {
-          __threadfence_system();  // every tile's stores were fenced before its CTA counted itself in
+          if (W > 1) __threadfence_system();  // every tile's stores were fenced before its CTA counted itself in
+          else __threadfence();
           for (int d = 0; d < W; ++d)
             st_release_sys(reinterpret_cast<uint32_t*>(push.region[d] + push.flag_off) + push.me, epoch);
         }
@@ -217,7 +228,19 @@ __global__ void __launch_bounds__(256) psgd_prep_kernel(const T* __restrict__ gr
                                                        float* __restrict__ z0, int64_t n0, float* __restrict__ z1,
                                                        int64_t n1) {
   const int64_t t0 = int64_t(blockIdx.x) * 256 + threadIdx.x, stride = int64_t(gridDim.x) * 256;
-  for (int64_t i = t0; i < numel; i += stride)
+  // Eight elements a thread where the addresses allow it (bound by HBM; one element a thread was bound by latency: 2.4 M elements
+  // 4.7 -> 3.6 us).
+  const bool vec = ((reinterpret_cast<uintptr_t>(grad) | reinterpret_cast<uintptr_t>(ef) | reinterpret_cast<uintptr_t>(mef)) & 15u) == 0;
+  const int64_t n8 = vec ? numel / 8 : 0;
+  for (int64_t q = t0; q < n8; q += stride) {
+    float g[8], e[8];
+    dev::Vec8<T>::load(grad + q * 8, g);
+    dev::Vec8<__nv_bfloat16>::load(ef + q * 8, e);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) e[k] += dev::sanitize(g[k]);
+    dev::Vec8<__nv_bfloat16>::store(mef + q * 8, e);
+  }
+  for (int64_t i = n8 * 8 + t0; i < numel; i += stride)
     mef[i] = __float2bfloat16_rn(dev::sanitize(dev::Vec16<T>::to_float(grad[i])) + __bfloat162float(ef[i]));
   // the two projections accumulate into these with atomics (split K): clear them here, not in launches of their own
   for (int64_t i = t0; i < n0; i += stride) z0[i] = 0.0f;
@@ -288,15 +311,79 @@ __global__ void __launch_bounds__(256) psgd_reconstruct_kernel(T* __restrict__ g
 // Orthonormalisation is Gram-Schmidt through the Gram matrix (Q = W R^-1 with R^T R = W^T W, the
 // Cholesky factor), applied twice ("CholeskyQR2"): each round is one pass that accumulates the r x r Gram
 // matrix, a cluster-wide sum over distributed shared memory in a fixed order (every CTA gets the same
-// bits), a 16 x 16 factorisation done redundantly by every CTA, and one pass that applies R^-1. A column
+// bits), a factorisation done redundantly by one warp of every CTA, and one pass that applies R^-1. A column
 // whose pivot vanishes (rank-deficient factor) becomes zero, as a column of norm 0 stays in classical
 // Gram-Schmidt. The second round removes the orthogonality loss of the first.
+//
+// Bound by latency: the factor is a few hundred rows of r values per CTA, which stay in shared memory from the mean to the
+// results (a factor too tall for that is worked on in memory, SMEM = false), so that between the flags and the results there are
+// two cluster barriers and two factorisations per launch and no trip to L2. Measured on B200, rank 4, 2048 rows: 23.5 -> 9.9 us;
+// rank 8 (four factors of 512 to 4608 rows at once): 72 -> 18 us each. Before, every pass went through memory, and one thread
+// factorised with its matrices in local memory.
 constexpr int kXCtas = 8;
 constexpr int kXThreads = 512;
-constexpr int kPairs = kCols * (kCols + 1) / 2;
+constexpr int kXWarps = kXThreads / 32;
 
-// RMAX: compile-time bound on the rank (4 keeps the 10 pair sums and the row in registers).
+// Factorises the Gram matrix in `gram` (lower triangle, packed) and leaves R^-1 (upper triangular) in `rinv`. One warp: lane i holds row
+// i of the matrix, columns are eliminated one after the other; then lane c solves for column c of the inverse.
 template <int RMAX>
+__device__ __forceinline__ void factorise(const float* gram, int r, float (*L)[kCols], float (*rinv)[kCols]) {
+  const int lane = threadIdx.x & 31;
+  const int row = lane < RMAX ? lane : 0;
+  float g[RMAX], diag = 0.0f;
+#pragma unroll
+  for (int j = 0; j < RMAX; ++j) {
+    g[j] = j <= row && row < r ? gram[row * (row + 1) / 2 + j] : 0.0f;
+    if (j == row) diag = g[j];
+  }
+  uint32_t dead = 0;
+#pragma unroll
+  for (int c = 0; c < RMAX; ++c) {
+    if (c < r) {
+      const float pivot = __shfl_sync(0xffffffffu, g[c], c), d0 = __shfl_sync(0xffffffffu, diag, c);
+      const bool gone = !(pivot > 1e-20f) || !(pivot > 1e-7f * d0);  // pivot vanished: dependent (or zero) column
+      const float root = gone ? 1.0f : sqrtf(pivot);
+      if (gone) dead |= 1u << c;
+      const float l = row == c ? root : gone || row < c ? 0.0f : g[c] / root;
+      g[c] = l;
+#pragma unroll
+      for (int j = c + 1; j < RMAX; ++j) {
+        const float lj = __shfl_sync(0xffffffffu, l, j);
+        if (j <= row) g[j] = __fmaf_rn(-l, lj, g[j]);
+      }
+    }
+  }
+  if (lane < RMAX) {
+#pragma unroll
+    for (int j = 0; j < RMAX; ++j) L[lane][j] = j <= lane ? g[j] : 0.0f;
+  }
+  __syncwarp();
+  // X = R^-1 where R = L^T (upper triangular): X[j][c] for j <= c; a dead column is zero, and nothing depends on a dead row
+  if (lane < RMAX) {
+    const int c = lane;
+    float x[RMAX];
+#pragma unroll
+    for (int j = RMAX - 1; j >= 0; --j) {
+      float v = 0.0f;
+      if (c < r && j <= c && !((dead >> c) & 1u) && !((dead >> j) & 1u)) {
+        if (j == c) {
+          v = 1.0f / L[c][c];
+        } else {
+          float sum = 0.0f;
+#pragma unroll
+          for (int k = RMAX - 1; k > j; --k)
+            if (k <= c) sum = __fmaf_rn(L[k][j], x[k], sum);  // R[j][k] = L[k][j]
+          v = -sum / L[j][j];
+        }
+      }
+      x[j] = v;
+      rinv[j][c] = v;
+    }
+  }
+}
+
+// RMAX: compile-time bound on the rank (4, 8 or 16). SMEM: this CTA's rows fit into shared memory.
+template <int RMAX, bool SMEM>
 __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_constant__ NangilaPsgdExchangeParams p) {
   constexpr int kAcc = RMAX * (RMAX + 1) / 2;
   cg::cluster_group cluster = cg::this_cluster();
@@ -304,20 +391,22 @@ __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_c
   const int vr = blockIdx.x / kXCtas;
   const int me = p.rank0 + vr;
   const int W = p.world, rows = p.rows, r = p.rank;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint64_t slot_bytes = (uint64_t(rows) * r * 4 + 255) & ~uint64_t(255);
   const uint32_t epoch = p.epoch_dev != nullptr ? *p.epoch_dev : p.epoch;
   const uint64_t base = p.recv_off + uint64_t(epoch & 1u) * W * slot_bytes;  // two slot sets, by launch parity
   uint32_t* status = p.status[vr];
   const float* local = p.local[vr];
   float* mean = p.mean_out[vr];
+  __nv_bfloat16* t_out = static_cast<__nv_bfloat16*>(p.t_out[vr]);
   // this CTA's rows
   const int per = (rows + kXCtas - 1) / kXCtas;
-  const int r0 = min(rows, g * per), r1 = min(rows, r0 + per);
-  __shared__ float s_warp[kXThreads / 32][kPairs];  // per-warp partial sums (summed in warp order: no float atomics)
-  __shared__ float s_part[kPairs];          // this CTA's partial Gram matrix (lower triangle, packed)
-  __shared__ float s_gram[kPairs];          // cluster-wide sum
-  __shared__ float s_rinv[kCols][kCols];    // R^-1 (upper triangular); a zero column for a vanished pivot
+  const int r0 = min(rows, g * per), r1 = min(rows, r0 + per), mine = r1 - r0;
+  extern __shared__ float s_rows[];         // [r][per]: the factor's rows, column-major
+  __shared__ float s_warp[kXWarps][kAcc];   // per-warp partial sums (summed in warp order: no float atomics)
+  __shared__ float s_part[2][kAcc];         // this CTA's partial Gram matrix (lower triangle, packed), one per round
+  __shared__ float s_gram[kAcc];            // cluster-wide sum
+  __shared__ float s_l[kCols][kCols], s_rinv[kCols][kCols];  // the factor, R^-1 (upper triangular)
   __shared__ int s_ok;
 
   // 1. store my rows of my factor (r columns, column-major) into every rank's slot [me] (unless the GEMM's
@@ -329,11 +418,11 @@ __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_c
         for (int i = r0 + tid; i < r1; i += kXThreads) dst[int64_t(c) * rows + i] = local[int64_t(i) * kCols + c];
     }
     __threadfence_system();
-  }
-  cluster.sync();
-  if (p.pushed == 0 && g == 0 && tid < W) {
-    __threadfence_system();
-    st_release_sys(reinterpret_cast<uint32_t*>(p.region[tid] + p.flag_off) + me, epoch);
+    cluster.sync();
+    if (g == 0 && tid < W) {
+      __threadfence_system();
+      st_release_sys(reinterpret_cast<uint32_t*>(p.region[tid] + p.flag_off) + me, epoch);
+    }
   }
   // 2. wait for every rank's factor (every CTA polls for itself; on failure all of them still take part in
   //    the cluster barriers below, doing no work)
@@ -347,118 +436,108 @@ __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_c
   __syncthreads();
   const bool ok = s_ok != 0;
   // 3. mean in rank order (identical on every rank); columns >= r are zero
-  float* work = p.orth_mean ? mean : p.scratch[vr];
+  float* work = SMEM ? s_rows : (p.orth_mean ? mean : p.scratch[vr]) + r0;
+  const int pitch = SMEM ? per : rows;  // element (row r0 + i, c) at work[c * pitch + i]
   if (ok) {
     const float inv_w = 1.0f / float(W);
-    for (int c = 0; c < kCols; ++c)
-      for (int i = r0 + tid; i < r1; i += kXThreads) {
+    for (int c = 0; c < r; ++c)
+      for (int i = tid; i < mine; i += kXThreads) {
         float acc = 0.0f;
-        if (c < r)
-          for (int src = 0; src < W; ++src)
-            acc += reinterpret_cast<const float*>(p.region[me] + base + uint64_t(src) * slot_bytes)[int64_t(c) * rows + i];
+        for (int src = 0; src < W; ++src)
+          acc += reinterpret_cast<const float*>(p.region[me] + base + uint64_t(src) * slot_bytes)[int64_t(c) * rows + r0 + i];
         acc *= inv_w;
-        mean[int64_t(c) * rows + i] = acc;
-        if (!p.orth_mean && c < r) work[int64_t(c) * rows + i] = acc;
+        if (!p.orth_mean) mean[int64_t(c) * rows + r0 + i] = acc;
+        work[int64_t(c) * pitch + i] = acc;
+      }
+    for (int c = r; c < kCols; ++c)
+      for (int i = r0 + tid; i < r1; i += kXThreads) {
+        mean[int64_t(c) * rows + i] = 0.0f;
+        t_out[int64_t(c) * rows + i] = __float2bfloat16_rn(0.0f);
       }
   }
-  __syncthreads();
   // 4. two rounds of Cholesky-QR on `work`
   for (int round = 0; round < 2; ++round) {
-    for (int i = tid; i < (kXThreads / 32) * kPairs; i += kXThreads) (&s_warp[0][0])[i] = 0.0f;
-    __syncthreads();
-    if (ok) {
-      // every thread owns whole rows: all pair products of a row come from registers
+    if constexpr (RMAX <= 8) {
+      // every thread works on whole rows of its own: all pair products of a row come from registers
       float acc[kAcc];
 #pragma unroll
       for (int q = 0; q < kAcc; ++q) acc[q] = 0.0f;
-      for (int i = r0 + tid; i < r1; i += kXThreads) {
-        float w[RMAX];
+      if (ok) {
+        for (int i = tid; i < mine; i += kXThreads) {
+          float w[RMAX];
 #pragma unroll
-        for (int c = 0; c < RMAX; ++c) w[c] = c < r ? work[int64_t(c) * rows + i] : 0.0f;
-        int q = 0;
+          for (int c = 0; c < RMAX; ++c) w[c] = c < r ? work[int64_t(c) * pitch + i] : 0.0f;
+          int q = 0;
 #pragma unroll
-        for (int c = 0; c < RMAX; ++c)
+          for (int c = 0; c < RMAX; ++c)
 #pragma unroll
-          for (int j = 0; j <= c; ++j, ++q) acc[q] = __fmaf_rn(w[c], w[j], acc[q]);
+            for (int j = 0; j <= c; ++j, ++q) acc[q] = __fmaf_rn(w[c], w[j], acc[q]);
+        }
       }
 #pragma unroll
       for (int q = 0; q < kAcc; ++q) {
         float v = acc[q];
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if ((tid & 31) == 0) s_warp[tid >> 5][q] = v;
+        if (lane == 0) s_warp[warp][q] = v;
+      }
+    } else {
+      // 136 sums are too many for a thread's registers: a warp's lanes share them out, and each lane walks the warp's rows
+      __syncthreads();  // rows of other threads: the pass before this one has written them
+      for (int q = lane; q < kAcc; q += 32) {
+        int c = 0;
+        while ((c + 1) * (c + 2) / 2 <= q) ++c;
+        const int j = q - c * (c + 1) / 2;
+        float v = 0.0f;
+        if (ok && c < r)
+          for (int i = warp; i < mine; i += kXWarps) v = __fmaf_rn(work[int64_t(c) * pitch + i], work[int64_t(j) * pitch + i], v);
+        s_warp[warp][q] = v;
       }
     }
     __syncthreads();
-    for (int q = tid; q < kPairs; q += kXThreads) {
+    for (int q = tid; q < kAcc; q += kXThreads) {
       float v = 0.0f;
-      for (int w = 0; w < kXThreads / 32; ++w) v += s_warp[w][q];  // fixed order: the same bits on every rank
-      s_part[q] = v;
+#pragma unroll
+      for (int w = 0; w < kXWarps; ++w) v += s_warp[w][q];  // fixed order: the same bits on every rank
+      s_part[round][q] = v;
     }
     cluster.sync();  // every CTA's partial matrix is complete
-    for (int q = tid; q < kPairs; q += kXThreads) {
-      float v = 0.0f;
-      for (int b = 0; b < kXCtas; ++b) v += *cluster.map_shared_rank(&s_part[q], b);  // fixed order
+    for (int q = tid; q < kAcc; q += kXThreads) {
+      float part[kXCtas], v = 0.0f;
+#pragma unroll
+      for (int b = 0; b < kXCtas; ++b) part[b] = *cluster.map_shared_rank(&s_part[round][q], b);
+#pragma unroll
+      for (int b = 0; b < kXCtas; ++b) v += part[b];  // fixed order
       s_gram[q] = v;
     }
     __syncthreads();
-    if (tid == 0) {
-      // Cholesky of the r x r Gram matrix: L L^T; then R^-1 = (L^T)^-1 by back substitution
-      float L[kCols][kCols];
-      bool dead[kCols];
-      for (int c = 0; c < r; ++c) {
-        for (int j = 0; j <= c; ++j) {
-          float sum = s_gram[c * (c + 1) / 2 + j];
-          for (int k = 0; k < j; ++k) sum -= L[c][k] * L[j][k];
-          if (j < c) {
-            L[c][j] = dead[j] ? 0.0f : sum / L[j][j];
-          } else {
-            const float diag = s_gram[c * (c + 1) / 2 + c];
-            dead[c] = !(sum > 1e-20f) || !(sum > 1e-7f * diag);  // pivot vanished: dependent (or zero) column
-            L[c][c] = dead[c] ? 1.0f : sqrtf(sum);
-          }
-        }
-      }
-      // X = R^-1 where R = L^T (upper triangular): X[j][c] for j <= c
-      for (int c = 0; c < kCols; ++c)
-        for (int j = 0; j < kCols; ++j) s_rinv[j][c] = 0.0f;
-      for (int c = 0; c < r; ++c) {
-        if (dead[c]) continue;  // column of zeros
-        s_rinv[c][c] = 1.0f / L[c][c];
-        for (int j = c - 1; j >= 0; --j) {
-          if (dead[j]) continue;
-          float sum = 0.0f;
-          for (int k = j + 1; k <= c; ++k) sum += L[k][j] * s_rinv[k][c];  // R[j][k] = L[k][j]
-          s_rinv[j][c] = -sum / L[j][j];
-        }
-      }
-    }
+    if (warp == 0) factorise<RMAX>(s_gram, r, s_l, s_rinv);
     __syncthreads();
     if (ok) {
-      for (int i = r0 + tid; i < r1; i += kXThreads) {
+      for (int i = tid; i < mine; i += kXThreads) {
         float w[RMAX];
 #pragma unroll
-        for (int c = 0; c < RMAX; ++c) w[c] = c < r ? work[int64_t(c) * rows + i] : 0.0f;
+        for (int c = 0; c < RMAX; ++c) w[c] = c < r ? work[int64_t(c) * pitch + i] : 0.0f;
 #pragma unroll
         for (int c = 0; c < RMAX; ++c) {
           if (c < r) {
             float o = 0.0f;
 #pragma unroll
             for (int j = 0; j <= c; ++j) o = __fmaf_rn(w[j], s_rinv[j][c], o);
-            work[int64_t(c) * rows + i] = o;
+            if (round == 0) {
+              work[int64_t(c) * pitch + i] = o;
+            } else {
+              // 5. the results: the orthonormal factor where it is the mean's, and its bf16 copy for the next GEMM's B operand
+              const int64_t at = int64_t(c) * rows + r0 + i;
+              if (p.orth_mean) mean[at] = o;
+              t_out[at] = __float2bfloat16_rn(o);
+            }
           }
         }
       }
     }
-    cluster.sync();  // nobody reads a neighbour's s_part after this; safe to clear it in the next round
   }
-  // 5. bf16 copy for the next GEMM's B operand (same layout)
-  if (ok) {
-    __nv_bfloat16* t_out = static_cast<__nv_bfloat16*>(p.t_out[vr]);
-    for (int c = 0; c < kCols; ++c)
-      for (int i = r0 + tid; i < r1; i += kXThreads)
-        t_out[int64_t(c) * rows + i] = __float2bfloat16_rn(c < r ? work[int64_t(c) * rows + i] : 0.0f);
-  }
+  cluster.sync();  // a neighbour may still be reading this CTA's part of the last sum
 }
 
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -564,7 +643,7 @@ extern "C" int nangila_psgd_prep(const void* grad, int32_t dtype, const void* ef
                                  cudaStream_t stream) {
   using namespace nangila;
   if (!grad || !ef || !mef || numel <= 0) return int(cudaErrorInvalidValue);
-  const int blocks = int(std::min<int64_t>((numel + 255) / 256, 148 * 8));
+  const int blocks = int(std::min<int64_t>((numel + 2047) / 2048, 148 * 32));
   auto* e = static_cast<const __nv_bfloat16*>(ef);
   auto* o = static_cast<__nv_bfloat16*>(mef);
   switch (dtype) {
@@ -614,10 +693,13 @@ extern "C" int nangila_psgd_exchange(const NangilaPsgdExchangeParams* p, cudaStr
   if (!p || p->rows <= 0 || p->rank <= 0 || p->rank > 16 || p->world < 1 || p->world > NANGILA_MAX_RANKS || p->nvr < 1 ||
       p->nvr > NANGILA_MAX_VRANKS || (p->nvr > 1 && p->nvr != p->world) || (p->epoch == 0 && p->epoch_dev == nullptr))
     return int(cudaErrorInvalidValue);
+  // the CTA's rows stay in shared memory up to this much: with the static part below the default limit of 48 KB
+  const size_t rows_bytes = size_t((p->rows + kXCtas - 1) / kXCtas) * size_t(p->rank) * sizeof(float);
+  const bool smem = rows_bytes <= 32768;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3{unsigned(p->nvr * kXCtas), 1u, 1u};
   cfg.blockDim = dim3{unsigned(kXThreads), 1u, 1u};
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem ? rows_bytes : 0;
   cfg.stream = stream;
   cudaLaunchAttribute attrs[2];
   attrs[0].id = cudaLaunchAttributeClusterDimension;
@@ -631,7 +713,13 @@ extern "C" int nangila_psgd_exchange(const NangilaPsgdExchangeParams* p, cudaStr
   cfg.attrs = attrs;
   cfg.numAttrs = p->nvr > 1 ? 2 : 1;
   const NangilaPsgdExchangeParams params = *p;
-  cudaError_t e = p->rank <= 4 ? cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<4>, params)
-                               : cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<kCols>, params);
+  cudaError_t e;
+  if (p->rank <= 4)
+    e = smem ? cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<4, true>, params) : cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<4, false>, params);
+  else if (p->rank <= 8)
+    e = smem ? cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<8, true>, params) : cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<8, false>, params);
+  else
+    e = smem ? cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<kCols, true>, params)
+             : cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<kCols, false>, params);
   return int(e);
 }
