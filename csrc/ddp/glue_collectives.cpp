@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <string>
 #include <vector>
 
 #include "nangila_kernels.h"
@@ -123,6 +124,54 @@ void packet_encode(const at::Tensor& grad, const c10::optional<at::Tensor>& curr
   check_launch(nangila_packet_encode(grad.data_ptr(), dtype_code(grad), f32(curr, "curr"), f32(prev, "prev"), f32(ef, "ef"),
                                      float(mu), float(gain), n, payload.data_ptr<uint8_t>(), at::cuda::getCurrentCUDAStream()),
                "packet_encode");
+}
+// The whole packet of `grad`: header (32 bytes), checksum and payload, queued without touching the host again.
+at::Tensor packet_compress(const at::Tensor& grad, const c10::optional<at::Tensor>& curr, const c10::optional<at::Tensor>& prev,
+                           const c10::optional<at::Tensor>& ef, double mu, double gain, const std::string& header) {
+  TORCH_CHECK(grad.is_cuda() && grad.is_contiguous(), "nangila: packet_compress wants a contiguous CUDA gradient");
+  TORCH_CHECK(header.size() == 32, "nangila: a packet header has 32 bytes");
+  const int64_t n = grad.numel();
+  auto f32 = [&](const c10::optional<at::Tensor>& t, const char* what) -> float* {
+    if (!t.has_value()) return nullptr;
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() == n, "nangila: ", what,
+                " must be a contiguous FP32 CUDA tensor of the gradient's size");
+    return t->data_ptr<float>();
+  };
+  c10::cuda::CUDAGuard guard(grad.device());
+  auto packet = at::empty({32 + nangila_packet_payload_bytes(n)}, grad.options().dtype(at::kByte));
+  auto sums = at::empty({2}, grad.options().dtype(at::kFloat));
+  check_launch(nangila_packet_compress(grad.data_ptr(), dtype_code(grad), f32(curr, "curr"), f32(prev, "prev"), f32(ef, "ef"), float(mu),
+                                       float(gain), n, reinterpret_cast<const uint8_t*>(header.data()), packet.data_ptr<uint8_t>(),
+                                       sums.data_ptr<float>(), at::cuda::getCurrentCUDAStream()), "packet_compress");
+  return packet;
+}
+// What the host has to know of a packet before it decodes it: the first (up to) 44 bytes and, if asked for, the CRC32 of everything
+// behind the header. One synchronisation for both.
+py::tuple packet_inspect(const at::Tensor& packet, bool checksum) {
+  TORCH_CHECK(packet.is_cuda() && packet.scalar_type() == at::kByte && packet.is_contiguous() && packet.numel() > 32,
+              "nangila: packet_inspect wants a contiguous uint8 CUDA packet");
+  const int64_t fixed = std::min<int64_t>(packet.numel(), 44);
+  c10::cuda::CUDAGuard guard(packet.device());
+  auto stream = at::cuda::getCurrentCUDAStream();
+  auto host = at::empty({48}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
+  uint8_t* h = host.data_ptr<uint8_t>();
+  at::Tensor word;
+  if (checksum) {
+    word = at::empty({1}, packet.options().dtype(at::kInt));
+    auto* w = reinterpret_cast<uint32_t*>(word.data_ptr<int32_t>());
+    check_launch(nangila_crc32(packet.data_ptr<uint8_t>() + 32, packet.numel() - 32, w, w, stream), "crc32");
+    check_launch(int(cudaMemcpyAsync(h + 44, w, 4, cudaMemcpyDeviceToHost, stream)), "packet_inspect");
+  }
+  check_launch(int(cudaMemcpyAsync(h, packet.data_ptr<uint8_t>(), size_t(fixed), cudaMemcpyDeviceToHost, stream)), "packet_inspect");
+  cudaError_t e;
+  {
+    py::gil_scoped_release release;
+    e = cudaStreamSynchronize(stream);
+  }
+  check_launch(int(e), "packet_inspect");
+  uint32_t crc = 0;
+  if (checksum) std::memcpy(&crc, h + 44, 4);
+  return py::make_tuple(py::bytes(reinterpret_cast<const char*>(h), size_t(fixed)), crc);
 }
 void packet_decode(const at::Tensor& payload, int64_t ndim, const c10::optional<at::Tensor>& curr,
                    const c10::optional<at::Tensor>& prev, double mu, double gain, at::Tensor out) {
@@ -436,6 +485,9 @@ void register_more(py::module_& m) {
   m.def("packet_payload_bytes", &packet_payload_bytes);
   m.def("packet_encode", &packet_encode, py::arg("grad"), py::arg("curr"), py::arg("prev"), py::arg("ef"), py::arg("mu"),
         py::arg("gain"), py::arg("payload"));
+  m.def("packet_compress", &packet_compress, py::arg("grad"), py::arg("curr"), py::arg("prev"), py::arg("ef"), py::arg("mu"),
+        py::arg("gain"), py::arg("header"));
+  m.def("packet_inspect", &packet_inspect, py::arg("packet"), py::arg("checksum"));
   m.def("packet_decode", &packet_decode, py::arg("payload"), py::arg("ndim"), py::arg("curr"), py::arg("prev"), py::arg("mu"),
         py::arg("gain"), py::arg("out"));
   m.def("dgc_region_layout", &dgc_region_layout);

@@ -232,6 +232,10 @@ int nangila_dequant_reconstruct_gamma(const uint8_t* packed, const float* g_curr
 int64_t nangila_packet_payload_bytes(int64_t n);
 int nangila_packet_encode(const void* grad, int32_t dtype, const float* curr, const float* prev, float* ef, float mu,
                           float gain, int64_t n, uint8_t* payload, cudaStream_t stream);
+/* A whole packet: `header` (32 bytes, HOST memory) with the payload's CRC32 put into bytes 12..16, then the payload. `packet` (device, 4-byte
+ * aligned) holds 32 + nangila_packet_payload_bytes(n) bytes, `sums` (device) two floats of scratch. */
+int nangila_packet_compress(const void* grad, int32_t dtype, const float* curr, const float* prev, float* ef, float mu, float gain, int64_t n,
+                            const uint8_t* header, uint8_t* packet, float* sums, cudaStream_t stream);
 /* decode: out = q scale + kappa (curr + mu (curr - prev)); gain < 0 takes kappa from the payload. `ndim` is the
  * payload's dimension count (its third word), which fixes where the gain, scales and nibbles start. */
 int nangila_packet_decode(const uint8_t* payload, int64_t payload_bytes, int32_t ndim, const float* curr, const float* prev,

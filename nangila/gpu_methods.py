@@ -16,8 +16,8 @@ made by ``compress`` decodes with ``decompress_gpu``:
 The history (two FP32 tensors per layer) and the error memory live on the device, attached to the hook
 object; the host-side state machine supplies step numbers, warm-up and momentum. Nothing synchronises
 unless ``sync_mode`` says so: 0 (ASYNC) never, 1 (ALWAYS) after every call, 2 (PERIODIC) every 100th call.
-``decompress_gpu`` reads the 44 fixed bytes of the packet on the host (a small synchronising copy) to
-validate it before anything is launched, and verifies the checksum unless ``sync_mode`` is 0.
+``decompress_gpu`` reads the 44 fixed bytes of the packet on the host (one synchronisation, which brings the checksum of
+the payload with it unless ``sync_mode`` is 0) and validates them before anything is decoded.
 """
 from __future__ import annotations
 
@@ -107,14 +107,9 @@ def compress_gpu(self: NangilaHook, layer_id: int, gradient: torch.Tensor, sync_
             glue = _glue()
             ls = _layer(self, layer_id, n, dev)
             have_history = ls.updates >= 2
-            nbytes = int(glue.packet_payload_bytes(n))
-            packet = torch.empty(_HEADER + nbytes, dtype=torch.uint8, device=dev)
-            head = _header_bytes(_FLAG_DRIVER, step, layer_id)
-            packet[:_HEADER] = torch.frombuffer(bytearray(head), dtype=torch.uint8).to(dev, non_blocking=True)
-            glue.packet_encode(g, ls.curr if have_history else None, ls.prev if have_history else None, ls.ef,
-                               float(self.momentum()), -1.0, packet[_HEADER:])
-            out = _finish_packet(packet)
-            self.record_external(layer_id, n * g.element_size(), _HEADER + nbytes, 0.0)
+            out = glue.packet_compress(g, ls.curr if have_history else None, ls.prev if have_history else None, ls.ef,
+                                       float(self.momentum()), -1.0, _header_bytes(_FLAG_DRIVER, step, layer_id))
+            self.record_external(layer_id, n * g.element_size(), out.numel(), 0.0)
     _maybe_sync(self, sync_mode)
     return out
 
@@ -126,7 +121,8 @@ def decompress_gpu(self: NangilaHook, layer_id: int, compressed: torch.Tensor, o
     if packet.numel() < _HEADER + 8:
         raise RuntimeError(f"decompress_gpu: packet of {packet.numel()} bytes is too small")
     dev = packet.device
-    fixed = bytes(packet[:min(packet.numel(), _HEADER + 12)].cpu().numpy())
+    with torch.cuda.device(dev):
+        fixed, got = _glue().packet_inspect(packet, sync_mode != 0)
     magic, version, flags, _step, layer, crc, _hash, _s, _e = struct.unpack("<HBBIIIQII", fixed[:_HEADER])
     if magic != _MAGIC or version != _VERSION:
         raise RuntimeError("decompress_gpu: not a nangila packet (bad magic or version)")
@@ -134,10 +130,8 @@ def decompress_gpu(self: NangilaHook, layer_id: int, compressed: torch.Tensor, o
         raise RuntimeError(f"decompress_gpu: packet is for layer {layer}, expected {layer_id}")
     with torch.cuda.device(dev):
         glue = _glue()
-        if sync_mode != 0:
-            got = int(glue.crc32(packet[_HEADER:]).item()) & 0xFFFFFFFF
-            if got != crc:
-                raise RuntimeError(f"decompress_gpu: checksum mismatch on layer {layer_id} ({got:#x} != {crc:#x})")
+        if sync_mode != 0 and got != crc:
+            raise RuntimeError(f"decompress_gpu: checksum mismatch on layer {layer_id} ({got:#x} != {crc:#x})")
         out = torch.empty(int(output_size), dtype=torch.float32, device=dev)
         if not flags & _FLAG_DRIVER:
             # raw tensor payload: u32 numel, u32 ndim, u32 dims[ndim], f32 data
