@@ -173,6 +173,39 @@ __global__ void __launch_bounds__(T) spmv_row_blocks_bulk_kernel(const int* __re
     }
 }
 
+// Short rows: one thread per row, no staging, no barrier. Four entries of the row are in flight at once; a warp's loads of one
+// entry are strided by the row length, but the lines they touch are the ones its next entries need, so L1 serves them.
+// Bound by HBM where the matrix does not fit L2, by the chain row_ptr -> col -> x otherwise; the staged kernel adds to that chain
+// the block table, a barrier initialisation, a copy of the slice and two block barriers, and gives a CTA so much of the matrix that a
+// ladder of 10^6 rows is 1.2 waves of CTAs. Products are rounded and added in the staged kernel's order for two and four lanes a row, so
+// that ladders and meshes keep their bits. Measured on B200, vectors on the device: ladder of 10^6 rows 24 -> 14 us, of 4 10^6 59 -> 41 us
+// (5.5 TB/s); mesh of 10^6 nodes 35 -> 19, of 4 10^6 100 -> 56 us.
+constexpr int kShortRow = 16;   // longest row of a matrix that takes this path
+constexpr int kShortMean = 6;   // and its mean row length: beyond, a lane's serial share outweighs what the staging costs
+__global__ void __launch_bounds__(kThreads) spmv_short_rows_kernel(const int* __restrict__ row_ptr, const int* __restrict__ col,
+                                                                   const double* __restrict__ val, const double* __restrict__ x,
+                                                                   double* __restrict__ y, int n) {
+    const int r = int(blockIdx.x * unsigned(kThreads) + threadIdx.x);
+    if (unsigned(r) >= unsigned(n)) return;
+    const int s = __ldg(row_ptr + r), e = __ldg(row_ptr + r + 1);
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int j = s; j < e; j += 4) {
+        int c[4];
+        double v[4], g[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            c[u] = j + u < e ? __ldg(col + j + u) : -1;
+            v[u] = j + u < e ? __ldg(val + j + u) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) g[u] = c[u] >= 0 ? __ldg(x + c[u]) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (c[u] >= 0) acc[u] = __dadd_rn(acc[u], __dmul_rn(v[u], g[u]));
+    }
+    y[r] = (acc[0] + acc[2]) + (acc[1] + acc[3]);
+}
+
 // ---- vector kernels of the Krylov solver -------------------------------------------------------
 
 constexpr int kRedBlocks = 296;  // two CTAs per SM
@@ -237,6 +270,7 @@ struct NangilaSpmv {
     double *d_val = nullptr, *d_x = nullptr, *d_y = nullptr;
     int* d_status = nullptr;  // set by a kernel whose bulk copy timed out
     bool plain_loads = false;  // NANGILA_SPMV_PLAIN=1: use the plain-load kernel
+    bool short_rows = false;   // every row suits one thread: spmv_short_rows_kernel
     int cap = kCap;            // non-zeros per row block: 2048 (256 threads) or 1024 (128 threads, NANGILA_SPMV_TILE=1024)
     double* d_work = nullptr;   // solver vectors (kWorkVectors), allocated on first solve
     double* d_partial = nullptr;  // partial sums, then results and counter of the solver kernel
@@ -328,6 +362,11 @@ extern "C" int nangila_spmv_load(NangilaSpmv* c, int n, int nnz, const int* row_
     build_row_blocks(row_ptr, n, c->cap, blocks.data(), nb + 1);
     c->n_blocks = nb;
     c->h_row_ptr.assign(row_ptr, row_ptr + n + 1);
+    {
+        int longest = 0;
+        for (int r = 0; r < n; ++r) longest = std::max(longest, row_ptr[r + 1] - row_ptr[r]);
+        c->short_rows = longest <= kShortRow && nnz <= int64_t(kShortMean) * n;
+    }
     c->h_diag_slot.assign(size_t(n), -1);
     for (int r = 0; r < n; ++r)
         for (int k = row_ptr[r]; k < row_ptr[r + 1]; ++k)
@@ -375,6 +414,11 @@ extern "C" int nangila_spmv_device(NangilaSpmv* c, const double* d_x, double* d_
     if (!c || !c->d_val || !d_x || !d_y) return int(cudaErrorInvalidValue);
     if (c->plain_loads) return nangila_spmv_launch(c->d_row_ptr, c->d_col, c->d_val, d_x, d_y, c->d_blocks, c->n_blocks, stream);
     if (c->n_blocks <= 0) return 0;
+    if (c->short_rows) {
+        spmv_short_rows_kernel<<<unsigned((int64_t(c->n) + kThreads - 1) / kThreads), kThreads, 0, stream>>>(c->d_row_ptr, c->d_col, c->d_val, d_x,
+                                                                                                        d_y, c->n);
+        return int(cudaGetLastError());
+    }
     if (c->cap == 1024)
         spmv_row_blocks_bulk_kernel<128, 1024><<<c->n_blocks, 128, 0, stream>>>(c->d_row_ptr, c->d_col, c->d_val, d_x, d_y, c->d_blocks,
                                                                                c->d_status, 2000000000ull);
