@@ -315,6 +315,10 @@ static void free_arrays(NangilaSpmv* c) {
     c->d_val = c->d_x = c->d_y = c->d_work = c->d_partial = nullptr;
 }
 
+// The matrix is uploaded on the legacy stream, where a copy from pageable memory may return before it has reached the device and a
+// memset before it has run; solve_stream, and products on streams of the caller's, do not wait for that stream by themselves.
+static cudaError_t uploads_landed() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 static int build_row_blocks(const int* row_ptr, int n, int cap, int* out, int max_out);
 
 extern "C" int nangila_spmv_build_row_blocks(const int* row_ptr, int n, int* out, int max_out) {
@@ -394,13 +398,15 @@ extern "C" int nangila_spmv_load(NangilaSpmv* c, int n, int nnz, const int* row_
     NG_TRY(cudaMemcpy(c->d_col, col, sizeof(int) * size_t(nnz), cudaMemcpyHostToDevice));
     NG_TRY(cudaMemcpy(c->d_val, val, sizeof(double) * size_t(nnz), cudaMemcpyHostToDevice));
     NG_TRY(cudaMemcpy(c->d_blocks, blocks.data(), sizeof(int) * (size_t(nb) + 1), cudaMemcpyHostToDevice));
+    NG_TRY(uploads_landed());
     return 0;
 }
 
 extern "C" int nangila_spmv_update_values(NangilaSpmv* c, const double* val) {
     if (!c || !c->d_val || !val) return int(cudaErrorInvalidValue);
     refresh_preconditioner(c, val);
-    return int(cudaMemcpy(c->d_val, val, sizeof(double) * size_t(c->nnz), cudaMemcpyHostToDevice));
+    const cudaError_t e = cudaMemcpy(c->d_val, val, sizeof(double) * size_t(c->nnz), cudaMemcpyHostToDevice);
+    return int(e != cudaSuccess ? e : uploads_landed());
 }
 
 extern "C" int nangila_spmv_launch(const int* d_row_ptr, const int* d_col, const double* d_val, const double* d_x, double* d_y,
@@ -491,6 +497,7 @@ static cudaError_t plan_solver(NangilaSpmv* c) {
     plan.insert(plan.end(), long_rows.begin(), long_rows.end());
     if ((e = cudaMalloc(&c->d_plan, sizeof(int) * plan.size())) != cudaSuccess) return e;
     if ((e = cudaMemcpy(c->d_plan, plan.data(), sizeof(int) * plan.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return e;
+    if ((e = uploads_landed()) != cudaSuccess) return e;
     c->ctas = ctas;
     c->max_rows = max_rows;
     c->max_entries = max_entries;
