@@ -21,7 +21,8 @@
 //   5  wait (bounded) for every rank's list, add value / W into the bucket, list by list in rank order
 // Without a previous threshold, or if the list does not hold the k largest for sure (fewer than k candidates,
 // no room for all of them, a threshold above twice the bound), the threshold comes from a three-pass radix select over
-// the dense state (bits [30:20], [19:9], [8:0]; the first histogram is built in phase 1 if there is no previous threshold).
+// the dense state (bits [30:20], [19:9], [8:0]; the first histogram is built in phase 1 if there is no previous threshold, and by a CTA
+// whose list is full from there on).
 // The selection is exact either way: tau is the k-th largest |v|. Elements equal to tau are all selected, so
 // with ties the list can be longer than k (it is cut at the capacity; what is cut stays in v).
 //
@@ -135,9 +136,10 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
   uint32_t* my_idx = reinterpret_cast<uint32_t*>(myslot + 16);
   float* my_val = reinterpret_cast<float*>(myslot + 16 + uint64_t(cap) * 4);
 
-  __shared__ uint32_t sh_hist[kBins0];
+  __shared__ uint32_t sh_hist[kBins0], sh_top[kBins0];
   __shared__ uint32_t sh_sel[10];
-  __shared__ uint32_t sh_cand_cnt;  // candidates this CTA has appended to its segment of the list
+  __shared__ uint32_t sh_cand_cnt;   // candidates this CTA has found
+  __shared__ uint32_t sh_list_full;  // not 0: one of them had no room
   const int64_t tid0 = int64_t(blockIdx.x) * kThreads + threadIdx.x;
   const int64_t stride = int64_t(gridDim.x) * kThreads;
   // The dense passes walk the bucket in groups of 4 elements; every warp keeps all 32 lanes in the loop
@@ -167,33 +169,72 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
   uint32_t* spill_idx = scratch + kScratchWords + uint64_t(gridDim.x) * seg_cap;
   uint32_t* spill_bits = spill_idx + cand_cap;
 
-  if (threadIdx.x == 0) sh_cand_cnt = 0u;
+  if (threadIdx.x == 0) sh_cand_cnt = sh_list_full = 0u;
 
   // ---- phase 1: momentum correction, candidates (or the first histogram) ----
-  for (int i = threadIdx.x; i < kBins0; i += kThreads) sh_hist[i] = 0u;
+  static_assert(kCoarseBins == kBins0, "cleared together");
+  for (int i = threadIdx.x; i < kBins0; i += kThreads) sh_hist[i] = sh_top[i] = 0u;
   __syncthreads();
-  auto collect = [&](int64_t i, float v_new) {  // few entries qualify: only the lanes that have one meet in here
-    const uint32_t b = __float_as_uint(v_new) & 0x7fffffffu;
-    if (b >= cand_thr) {
-      const uint32_t here = __activemask(), lane = threadIdx.x & 31;
-      const int leader = __ffs(here) - 1;
-      uint32_t pos = 0;
-      if (int(lane) == leader) pos = atomicAdd(&sh_cand_cnt, uint32_t(__popc(here)));
-      pos = __shfl_sync(here, pos, leader) + uint32_t(__popc(here & ((1u << lane) - 1u)));
-      if (pos < seg_cap) {
-        cand_idx[pos] = uint32_t(i);
-        cand_bits[pos] = b;
-      } else {
-        pos = atomicAdd(&scratch[kSpill], 1u);
-        if (pos < spill_cap) {
-          spill_idx[pos] = uint32_t(i);
-          spill_bits[pos] = b;
-        }
-      }
-      atomicAdd(&sh_hist[min((b - cand_thr) >> kStepBits, uint32_t(kCoarseBins - 1))], 1u);
+  // The candidates among a lane's eight entries, from `first` on; all lanes of a warp come here. Space is reserved once for the
+  // warp's 256 entries. Where far more entries qualify than the list holds (the first steps of a bucket, gradients that have jumped) the
+  // selection goes over the dense state whatever is collected, so a CTA that has found the list full stops: without that, 13.1 M entries
+  // that all qualify made as many reservations in one word (455 us a step; 180 to 200 this way, 33 M: 1100 to 1200 and 410 to 490). From
+  // there on its warps count bits [30:20] instead, as they do without a previous threshold, so that less is left to be read again.
+  // Returns false if the entries were not collected because the list is full.
+  volatile uint32_t* list_full = &sh_list_full;
+  auto collect = [&](int64_t first, const float (&v_new)[8], int valid) -> bool {
+    uint32_t mine = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (k < valid && (__float_as_uint(v_new[k]) & 0x7fffffffu) >= cand_thr) mine |= 1u << k;
+    if (!__any_sync(0xffffffffu, mine != 0u)) return true;
+    if (__any_sync(0xffffffffu, *list_full != 0u)) return false;
+    const int lane = threadIdx.x & 31;
+    uint32_t incl = uint32_t(__popc(mine));
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += t;
     }
+    uint32_t base = 0, spill = 0;  // the warp's entries get base, base + 1, ...; those from seg_cap on go to spill, spill + 1, ...
+    if (lane == 31) {
+      base = atomicAdd(&sh_cand_cnt, incl);
+      const uint32_t over = base + incl > seg_cap ? base + incl - max(base, seg_cap) : 0u;
+      if (over > 0u) {
+        spill = atomicAdd(&scratch[kSpill], over);
+        if (spill + over > spill_cap) *list_full = 1u;
+      }
+    }
+    base = __shfl_sync(0xffffffffu, base, 31);
+    spill = __shfl_sync(0xffffffffu, spill, 31);
+    uint32_t pos = base + incl - uint32_t(__popc(mine));
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (mine & (1u << k)) {
+        const uint32_t b = __float_as_uint(v_new[k]) & 0x7fffffffu;
+        if (pos < seg_cap) {
+          cand_idx[pos] = uint32_t(first + k);
+          cand_bits[pos] = b;
+        } else {
+          const uint32_t at = spill + (pos - max(base, seg_cap));
+          if (at < spill_cap) {
+            spill_idx[at] = uint32_t(first + k);
+            spill_bits[at] = b;
+          }
+        }
+        atomicAdd(&sh_hist[min((b - cand_thr) >> kStepBits, uint32_t(kCoarseBins - 1))], 1u);
+        ++pos;
+      }
+    }
+    return true;
+  };
+  auto vote_top = [&](const float (&x)[8], int valid) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) hist_add(sh_top, (__float_as_uint(x[k]) & 0x7fffffffu) >> 20, k < valid);
   };
   const int64_t n8 = n / 8, groups8 = (n + 7) / 8, groups8_rounded = (groups8 + 31) / 32 * 32;
+  bool collecting = use_list;
+  int64_t vote_from = use_list ? groups8_rounded : 0;  // this lane's groups from here on are in the first histogram (the same iteration for a warp)
   for (int64_t q = tid0; q < groups8_rounded; q += stride) {
     float vn[8];
     int valid = 0;
@@ -227,20 +268,23 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
         }
       }
     }
-    if (use_list) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (k < valid) collect(q * 8 + k, vn[k]);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) hist_add(sh_hist, (__float_as_uint(vn[k]) & 0x7fffffffu) >> 20, k < valid);
+    if (collecting && !collect(q * 8, vn, valid)) {
+      collecting = false;
+      vote_from = q;
     }
+    if (!collecting) vote_top(vn, valid);
   }
   __syncthreads();
-  static_assert(kCoarseBins == kBins0, "one histogram in shared memory for either");
-  const int first_hist = use_list ? kCoarse : kHist0;
-  for (int i = threadIdx.x; i < kBins0; i += kThreads)
-    if (sh_hist[i]) atomicAdd(&scratch[first_hist + i], sh_hist[i]);
+  auto add_top = [&] {
+    for (int i = threadIdx.x; i < kBins0; i += kThreads)
+      if (sh_top[i]) atomicAdd(&scratch[kHist0 + i], sh_top[i]);
+  };
+  if (use_list) {
+    for (int i = threadIdx.x; i < kCoarseBins; i += kThreads)
+      if (sh_hist[i]) atomicAdd(&scratch[kCoarse + i], sh_hist[i]);
+  } else {
+    add_top();
+  }
   const uint32_t my_cand = min(sh_cand_cnt, seg_cap);  // entries of this CTA's segment
   if (threadIdx.x == 0) atomicAdd(&scratch[kCandCount], my_cand);
   if (!gsync()) return;
@@ -331,18 +375,23 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
     };
 
     if (use_list) {
-      // ---- bits [30:20], which phase 1 has left out ----
-      for (int i = threadIdx.x; i < kBins0; i += kThreads) sh_hist[i] = 0u;
-      __syncthreads();
-      for (int64_t q = tid0; q < groups_rounded; q += stride) {
-        uint32_t b[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
-        if (q < groups) load_bits(q, b);
+      // ---- bits [30:20] of what phase 1 went through while it still collected ----
+      for (int64_t q = tid0; q < vote_from; q += stride) {
+        float x[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        int valid = 0;
+        if (q < n8) {
+          dev::Vec8<float>::load(v + q * 8, x);
+          valid = 8;
+        } else if (q < groups8) {
+          valid = int(n - q * 8);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) hist_add(sh_hist, b[k] >> 20, b[k] != 0xffffffffu);
+          for (int k = 0; k < 8; ++k)
+            if (k < valid) x[k] = v[q * 8 + k];
+        }
+        vote_top(x, valid);
       }
       __syncthreads();
-      for (int i = threadIdx.x; i < kBins0; i += kThreads)
-        if (sh_hist[i]) atomicAdd(&scratch[kHist0 + i], sh_hist[i]);
+      add_top();
       if (!ssync()) return;
     }
     want = p.k;

@@ -76,3 +76,18 @@ def test_ties_at_the_threshold_are_all_sent_or_cut_at_the_capacity():
         eng.check_status()
         assert int(eng.buckets[0].out_count[0][0]) == 420
         assert int((g == 2.0).sum()) == 420 and not eng.buckets[0].v[0].any()
+
+
+def test_a_full_candidate_list_stops_the_collection():
+    """Gradients that jump put nearly every entry above the previous threshold. The list has no room for them, so what is reserved must
+    stay near its size (every warp may add its 256 entries once or twice after it is full) instead of counting them all."""
+    n = 16_777_216
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    eng = _engine(1, sparsity=0.999)
+    us, vs = [torch.zeros(n, device="cuda")], [torch.zeros(n, device="cuda")]
+    paths = [_check(eng, [torch.randn(n, device="cuda", generator=gen) * scale], us, vs, 0.9) for scale in (1e-3, 1.0)]
+    assert paths == [0, 0]
+    st = eng.buckets[0]
+    reserved = int(st.scratch[0][2048 + 2048 + 512 + 7])
+    capacity = (st.scratch[0].numel() - 2048) // 2  # an upper bound: the fixed words come off
+    assert 0 < reserved <= capacity + eng._grid(n) * 8 * 256 * 2 < n // 3 * 2
