@@ -510,6 +510,7 @@ void register_more(py::module_& m) {
   m.def("rs_region_layout", &rs_region_layout);
   m.def("rs_launch", &rs_launch);
   m.def("ag_region_layout", &ag_region_layout);
+  m.attr("LAYOUT_CTAS") = py::int_(NANGILA_LAYOUT_CTAS);
   m.def("ag_chunk_elems", [](int64_t shard, int64_t resident) { return nangila_ag_chunk_elems(shard, int32_t(resident)); });
   m.def("ag_launch", &ag_launch);
   m.def("state_hash", &state_hash, py::arg("tensors"), py::arg("seed") = 0);

@@ -193,10 +193,10 @@ extern "C" uint64_t nangila_ag_region_bytes(int64_t shard_elems, int32_t world, 
   return off;
 }
 
-// Chunk size for a shard. A rank has one quantize task per chunk and W dequantize tasks, walked by the CTAs the device holds at
-// once (`resident` per rank): the largest chunk that still gives every CTA a quantize task, in whole iterations, since each
+// Chunk size for a shard. A rank has one quantize task per chunk and W dequantize tasks, walked by the CTAs a whole device holds at
+// once (`resident` per rank, from NANGILA_LAYOUT_CTAS: 64 registers and 256 threads make four an SM): the largest chunk that still gives every CTA a quantize task, in whole iterations, since each
 // task ends in a block barrier and a system-wide flag (four ranks, 3.1 M bf16 elements each: chunks of 4096 elements 120 us,
-// 8192 78, 24576 59, 32768 64). Not below 4096 elements, where a task is nearly all barrier and flag (131 072 elements on four ranks:
+// 8192 78, 24576 59, 32768 64; the rule gives 22528 there, one rank alone 6144). Not below 4096 elements, where a task is nearly all barrier and flag (131 072 elements on four ranks:
 // 19.7 us, 21.4 with 2048), except for shards of less than four such chunks.
 extern "C" int32_t nangila_ag_chunk_elems(int64_t shard_elems, int32_t resident) {
   const int64_t g = resident > 0 ? resident : 1, most = 131072;

@@ -104,6 +104,10 @@ typedef struct NangilaAgParams {
 } NangilaAgParams;
 uint64_t nangila_ag_region_bytes(int64_t shard_elems, int32_t world, int32_t chunk_elems, int32_t bits,
                                  uint64_t* recv_off, uint64_t* flag_off);
+/* CTAs of a collective's kernel that the layout of an exchange region is cut for: four on each of a B200's 148 SMs. A constant and not
+ * what this process's device holds: peers write slots and flags into one another's regions, so every rank has to arrive at the
+ * same layout, whatever part of a GPU it was given. */
+#define NANGILA_LAYOUT_CTAS 592
 int32_t nangila_ag_chunk_elems(int64_t shard_elems, int32_t resident_ctas);
 int nangila_ag_launch(const NangilaAgParams* p, cudaStream_t stream);
 

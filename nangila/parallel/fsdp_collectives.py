@@ -284,8 +284,8 @@ class NangilaAllGather(_Base, AllGather):
         st = self._regions.get(key)
         if st is None:
             env = os.environ.get("NANGILA_CHUNK")
-            resident = max(1, int(self._glue.predres_resident_ctas()) // self.nvr)
-            chunk = int(env) if env else int(self._glue.ag_chunk_elems(shard, resident))
+            # a function of the size alone (see NANGILA_LAYOUT_CTAS), not of the CTAs that this rank's device holds
+            chunk = int(env) if env else int(self._glue.ag_chunk_elems(shard, max(1, self._glue.LAYOUT_CTAS // self.nvr)))
             total, r, f = self._glue.ag_region_layout(shard, self.world, chunk, self.bits)
             st = dict(region=arena.allocate(int(total)), r=r, f=f, chunk=chunk, epoch=0)
             self._regions[key] = st
