@@ -524,14 +524,8 @@ class DdpHook {
     Bucket b;
     b.n = t.numel();
     b.grad_dtype = code;
-    // sized against the CTAs the device holds at once, so that each phase is whole, equally loaded waves
-    int32_t c;
-    if (chunk_override_ > 0) {
-      c = chunk_override_;
-    } else {
-      if (resident_ <= 0) resident_ = nangila_predres_resident_ctas();
-      c = nangila_predres_chunk_elems(b.n, resident_);
-    }
+    // sized against the CTAs a whole device holds at once, so that each phase is whole, equally loaded waves
+    const int32_t c = chunk_override_ > 0 ? chunk_override_ : nangila_predres_chunk_elems(b.n, NANGILA_LAYOUT_CTAS);
     b.chunk = c;
     b.nchunks = int32_t((b.n + c - 1) / c);
     const uint64_t total = nangila_predres_region_bytes(b.n, world_, c, code, &b.r1, &b.r2, &b.f1, &b.f2);
@@ -604,7 +598,6 @@ class DdpHook {
   int32_t ctas_wait_ = 0;
   bool defer_ = true;
   bool dry_run_ = false;
-  int resident_ = 0;  // CTAs of the bucket kernel the device holds at once (queried once)
   std::deque<Pending> pending_;
   int32_t gather_max_world_;
   bool timing_ = false;

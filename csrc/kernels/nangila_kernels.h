@@ -80,9 +80,10 @@ uint64_t nangila_predres_region_bytes(int64_t n, int32_t world, int32_t chunk_el
 uint64_t nangila_rs_region_bytes(int64_t n, int32_t world, int32_t chunk_elems, uint64_t* recv1_off,
                                  uint64_t* flag1_off, int32_t* nchunks);
 int nangila_predres_launch(const NangilaPredResParams* p, cudaStream_t stream);
-/* CTAs of the compressed variants that the current device holds at once (occupancy x SM count): what a host
- * sizes chunks against so that every phase is a whole number of equally loaded waves. <= 0 on error. */
-int nangila_predres_resident_ctas(void);
+/* CTAs of a collective's kernel that the layout of an exchange region is cut for: four on each of a B200's 148 SMs. A constant and not
+ * what this process's device holds: peers write slots and flags into one another's regions, so every rank has to arrive at the
+ * same layout, whatever part of a GPU it was given. */
+#define NANGILA_LAYOUT_CTAS 592
 /* Chunk size (elements, a multiple of 4096) for a bucket of n elements: the smallest that covers the bucket
  * with at most `waves x resident` chunks, waves = the least that keeps a chunk at or below 131072 elements. */
 int32_t nangila_predres_chunk_elems(int64_t n, int32_t resident_ctas);
@@ -104,10 +105,6 @@ typedef struct NangilaAgParams {
 } NangilaAgParams;
 uint64_t nangila_ag_region_bytes(int64_t shard_elems, int32_t world, int32_t chunk_elems, int32_t bits,
                                  uint64_t* recv_off, uint64_t* flag_off);
-/* CTAs of a collective's kernel that the layout of an exchange region is cut for: four on each of a B200's 148 SMs. A constant and not
- * what this process's device holds: peers write slots and flags into one another's regions, so every rank has to arrive at the
- * same layout, whatever part of a GPU it was given. */
-#define NANGILA_LAYOUT_CTAS 592
 int32_t nangila_ag_chunk_elems(int64_t shard_elems, int32_t resident_ctas);
 int nangila_ag_launch(const NangilaAgParams* p, cudaStream_t stream);
 

@@ -44,8 +44,8 @@ def _glue():
 
 
 def default_chunk_elems(n: int, world: int, resident: int = 0) -> int:
-    """Chunk size (elements). Each phase of the kernel walks the chunks in waves of ``resident`` CTAs (what the
-    device holds at once, divided by the emulated ranks): the size is the smallest multiple of 4096 that covers
+    """Chunk size (elements). Each phase of the kernel walks the chunks in waves of ``resident`` CTAs (what a
+    whole device holds at once, divided by the emulated ranks): the size is the smallest multiple of 4096 that covers
     the bucket in whole waves with no chunk above 131072 elements, so the last wave is as full as the others.
     ``NANGILA_CHUNK`` overrides."""
     env = os.environ.get("NANGILA_CHUNK")
@@ -135,7 +135,6 @@ class PredResEngine:
         if use_side_stream:
             self.stream = torch.cuda.Stream(device=self.device, priority=-1)
         self._glue = _glue()
-        self._resident: Optional[int] = None  # CTAs per (emulated) rank the device holds at once
 
     # ------------------------------------------------------------------------------------------
     def _grid(self, st: BucketState) -> int:
@@ -170,9 +169,8 @@ class PredResEngine:
             return st
         if g0.dtype not in _DTYPE_CODE:
             raise TypeError(f"nangila: unsupported gradient dtype {g0.dtype}")
-        if self._resident is None:
-            self._resident = max(1, int(self._glue.predres_resident_ctas()) // self.nvr)
-        chunk = default_chunk_elems(n, self.world, self._resident)
+        # the same on every rank (see NANGILA_LAYOUT_CTAS): peers write into this region
+        chunk = default_chunk_elems(n, self.world, max(1, self._glue.LAYOUT_CTAS // self.nvr))
         total, r1, r2, f1, f2 = self._glue.predres_region_layout(n, self.world, chunk, _DTYPE_CODE[g0.dtype])
         region = self.arena.allocate(int(total))
         sdt = self._state_dtype_for(g0.dtype)

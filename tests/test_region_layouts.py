@@ -28,20 +28,34 @@ class _Glue:
     def ag_launch(self, inputs, outputs, status, ptrs, r, f, rank, chunk, *rest):
         self.chunks.append((r, f, chunk))
 
+    def rs_launch(self, inputs, outputs, ef, status, ptrs, r, f, nchunks, rank, chunk, *rest):
+        self.chunks.append((r, f, nchunks, chunk))
+
 
 SIZES = [2048, 131_072, 3_145_728, 50_000_000]
 
 
-def _chunks(resident):
-    from nangila.parallel.fsdp_collectives import NangilaAllGather
+def _chunks(what, resident):
+    from nangila.parallel import fsdp_collectives as F
+    from nangila.parallel.predres_engine import PredResEngine
 
-    ag = NangilaAllGather(arena=_Arena())
-    ag._glue = _Glue(resident)
+    glue = _Glue(resident)
+    if what == "bucket":
+        eng = PredResEngine(_Arena(), torch.device("meta"), use_side_stream=False)
+        eng._glue = glue
+        return [(st.layout, st.chunk) for i, n in enumerate(SIZES) for st in [eng.bucket_state(i, [torch.empty(n, dtype=torch.bfloat16, device="meta")])]]
+    obj = (F.NangilaAllGather if what == "all_gather" else F.NangilaReduceScatter)(arena=_Arena())
+    obj._glue = glue
     for n in SIZES:
-        ag.gather([torch.empty(0)], [torch.empty(n, dtype=torch.bfloat16, device="meta")])
-    return ag._glue.chunks
+        x = [torch.empty(n, dtype=torch.bfloat16, device="meta")]
+        if what == "all_gather":
+            obj.gather([torch.empty(0)], x)
+        else:
+            obj.reduce([torch.empty(0)], x, 0.25, unit=n)
+    return glue.chunks
 
 
+@pytest.mark.parametrize("what", ["all_gather", "reduce_scatter", "bucket"])
 @pytest.mark.parametrize("resident", [592, 148, 4])
-def test_all_gather_layout_is_the_same_on_every_device(resident):
-    assert _chunks(resident) == _chunks(528)
+def test_layout_is_the_same_on_every_device(what, resident):
+    assert _chunks(what, resident) == _chunks(what, 528)
