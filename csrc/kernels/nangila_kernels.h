@@ -184,7 +184,8 @@ uint32_t nangila_dgc_scratch_words(void);
 int nangila_dgc_launch(const NangilaDgcParams* p, cudaStream_t stream);
 
 /* ---- Sculptor calibration statistics (sculptor_stats.cu) -----------------------------------------------
- * Descriptor arrays live in DEVICE memory, or in HOST memory for the functions ending in _host, which copy them into the launch. */
+ * Descriptor arrays live in DEVICE memory, or in HOST memory for the functions ending in _host, which copy them into the launch.
+ * `max_numel` sizes the grid: the largest numel of the descriptors, or less at the price of more rounds per CTA. */
 typedef struct NangilaLayerDesc {
   const void* data;
   int64_t numel;

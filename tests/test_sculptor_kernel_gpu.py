@@ -1,5 +1,8 @@
 """The calibration kernels where their work is cut: tiles of 1024 elements, odd lengths (the five state vectors of a pair are
 then unaligned), gradients at odd addresses, pairs of different sizes in one step, more pairs than one launch carries."""
+import ctypes
+import os
+
 import pytest
 import torch
 
@@ -47,3 +50,35 @@ def test_more_pairs_than_one_launch_carries():
     for (i, j), st in ds._pair_state.items():
         a, b = (seen[0][i] + seen[1][i]) / 2, (seen[0][j] + seen[1][j]) / 2
         assert torch.allclose(st[:n], a, atol=1e-5) and torch.allclose(st[n:2 * n], b, atol=1e-5)
+
+
+@pytest.mark.parametrize("max_numel", [1, 1024, 5000, 70_001, 1 << 30])
+def test_descriptors_in_device_memory_whatever_the_grid_is_sized_for(max_numel):
+    """The C entries take descriptors in device memory and a size for the grid, which may be less than a pair's."""
+    lib = ctypes.CDLL(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "nangila", "libnangila_kernels.so"))
+
+    class Pair(ctypes.Structure):
+        _fields_ = [("i", ctypes.c_void_p), ("j", ctypes.c_void_p), ("state", ctypes.c_void_p), ("numel", ctypes.c_int64),
+                    ("dtype", ctypes.c_int32), ("count", ctypes.c_int32)]
+
+    class Layer(ctypes.Structure):
+        _fields_ = [("data", ctypes.c_void_p), ("numel", ctypes.c_int64), ("dtype", ctypes.c_int32), ("reserved", ctypes.c_int32)]
+
+    lib.nangila_sculptor_pair_update.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_void_p]
+    lib.nangila_sculptor_layer_sumsq.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p]
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    sizes = [70_001, 333]
+    x = [torch.randn(n, device="cuda", generator=gen) for n in sizes for _ in range(2)]
+    state = [torch.zeros(5 * n, device="cuda") for n in sizes]
+    to_device = lambda d: torch.frombuffer(bytearray(bytes(d)), dtype=torch.uint8).cuda()  # noqa: E731
+    pairs = to_device((Pair * 2)(*[Pair(x[2 * p].data_ptr(), x[2 * p + 1].data_ptr(), state[p].data_ptr(), n, 0, 1) for p, n in enumerate(sizes)]))
+    layers = to_device((Layer * 4)(*[Layer(t.data_ptr(), t.numel(), 0, 0) for t in x]))
+    out = torch.zeros(4, dtype=torch.float64, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    assert lib.nangila_sculptor_pair_update(pairs.data_ptr(), 2, max_numel, st) == 0
+    assert lib.nangila_sculptor_layer_sumsq(layers.data_ptr(), 4, max_numel, out.data_ptr(), st) == 0
+    for p, n in enumerate(sizes):
+        # the first observation: means are the values, everything else is zero
+        assert torch.equal(state[p], torch.cat([x[2 * p], x[2 * p + 1], torch.zeros(3 * n, device="cuda")]))
+    want = torch.stack([(t.double() ** 2).sum() for t in x])
+    assert ((out - want).abs() <= 1e-12 * want).all()
