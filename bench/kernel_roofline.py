@@ -114,8 +114,8 @@ def main() -> int:
             ms = time_ms(lambda i: eng.reduce(base + i % pool, [bufs[i % pool]], compressed=True, step=i), args.iters)
             eng.check_status()
             hist = 4 if gain else 0
-            if world == 1:  # one pass: read g, ef (+ history), write ef, g, history
-                hb = n * (2 + 2 + hist + 2 + 2 + 2)
+            if world == 1:  # one pass: read g, ef (+ history), write ef, g (+ history, which is left alone between probes at gain 0)
+                hb = n * (2 + 2 + hist + 2 + 2 + (2 if gain else 0))
             else:
                 hb = n * (2 + hist + 4 + q4) + n * q4 * 2 + n * (q4 + hist + 2 + 2)
             emit(name, ms, hb, 2 * n * q4 * w1, algbw_gbs=2 * n / ms / 1e6)
@@ -144,8 +144,8 @@ def main() -> int:
         ms = time_ms(dgc_call, args.iters) - t_copy
         eng.check_status()
         k = eng.buckets[0].k
-        # read g, u, v; write u, v; one selection pass over v; dense result written once
-        hb = n * (4 + 8 + 8 + 4 + 4)
+        # read g, u, v; write u, v; dense result written once
+        hb = n * (4 + 8 + 8 + 4)
         tele = eng.buckets[0].scratch[0][2048 + 2048 + 512:2048 + 2048 + 512 + 4].tolist()  # cursor, candidates seen, path
         emit("dgc_fused (sparsity 0.999, fp32)", ms, hb, 8.0 * k * (world - 1), k=k, refill_copy_ms_subtracted=t_copy,
              selected=tele[0], candidates_seen=tele[3], selection_from_candidate_list=bool(tele[2]))

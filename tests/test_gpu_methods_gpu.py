@@ -148,3 +148,24 @@ def test_c_entry_points_on_device_tensors():
                                     ctypes.byref(out_size), ctypes.addressof(header), stream, scratch.data_ptr(), 2) == 1
     lib.nangila_free(h)
     lib.nangila_free(peer)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n", [1, 64, 10_007])
+def test_bare_payload_is_the_packets_payload(n, dtype):
+    """``packet_encode`` (the payload alone) and ``packet_compress`` (header, checksum and payload in one call) write the same bytes."""
+    from nangila import _cuda as C
+
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    g = torch.randn(n, device="cuda", generator=gen).to(dtype)
+    curr, prev = (torch.randn(n, device="cuda", generator=gen) for _ in range(2))
+    efs = [torch.zeros(n, device="cuda") for _ in range(2)]
+    payload = torch.empty(C.packet_payload_bytes(n), dtype=torch.uint8, device="cuda")
+    C.packet_encode(g, curr, prev, efs[0], 0.9, 0.75, payload)
+    packet = C.packet_compress(g, curr, prev, efs[1], 0.9, 0.75, bytes(range(32)))
+    assert torch.equal(packet[32:], payload) and torch.equal(efs[0], efs[1])
+    head = packet[:32].cpu().numpy().tobytes()
+    assert head[:12] == bytes(range(12)) and head[16:] == bytes(range(16, 32))
+    import zlib
+
+    assert int.from_bytes(head[12:16], "little") == zlib.crc32(payload.cpu().numpy().tobytes())

@@ -28,8 +28,9 @@ def _reference(row_ptr, col, val, x):
     return y
 
 
+# ("bulk" is the default route: matrices of short rows only, "short" and "empty_rows", take the thread-per-row kernel there)
 @pytest.mark.parametrize("plain", [False, True], ids=["bulk", "plain"])
-@pytest.mark.parametrize("case", ["short", "mixed", "long", "empty_rows", "dense_ish"])
+@pytest.mark.parametrize("case", ["short", "mixed", "long", "empty_rows", "empty_and_long_rows", "dense_ish"])
 def test_spmv_matches_host(case, plain):
     from nangila_spice.gpu import DeviceCsr
 
@@ -44,6 +45,8 @@ def test_spmv_matches_host(case, plain):
         lens[[7, 2500, n - 1]] = [3000, 5003, 2049]  # rows longer than one block's capacity
     elif case == "empty_rows":
         lens = np.where(rng.random(n) < 0.7, 0, 3)
+    elif case == "empty_and_long_rows":
+        lens = np.where(rng.random(n) < 0.7, 0, 30)  # staged: rows above 16 entries
     else:
         n = 600
         lens = rng.integers(100, 400, n)
@@ -67,7 +70,7 @@ def test_spmv_matches_host(case, plain):
 
 @pytest.mark.parametrize("n", [200_000, 200_001, 7, 2])
 def test_tridiagonal_like_reference_benchmark(n):
-    """Banded pattern at even, odd and tiny sizes."""
+    """Banded pattern at even, odd and tiny sizes (one thread per row)."""
     from nangila_spice.gpu import DeviceCsr, tridiagonal
 
     row_ptr, col, val = tridiagonal(n)
@@ -87,6 +90,37 @@ def test_tridiagonal_like_reference_benchmark(n):
     torch.cuda.synchronize()
     m.check_status()
     assert np.abs(yd.cpu().numpy() - ref).max() < 1e-14
+
+
+@pytest.mark.parametrize("tile", ["", "1024"])
+@pytest.mark.parametrize("n", [200_000, 200_001, 257, 9])
+def test_wide_band_on_the_staged_kernel(monkeypatch, n, tile):
+    """Nine diagonals: too many entries a row for one thread each, so slices are staged by bulk copies, in either tile size."""
+    from nangila_spice.gpu import DeviceCsr
+
+    monkeypatch.setenv("NANGILA_SPMV_TILE", tile)
+    rng = np.random.default_rng(n)
+    first, last = np.maximum(np.arange(n) - 4, 0), np.minimum(np.arange(n) + 4, n - 1)
+    lens = last - first + 1
+    row_ptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    rows = np.repeat(np.arange(n), lens)
+    col = (first[rows] + np.arange(row_ptr[-1]) - row_ptr[rows]).astype(np.int32)
+    val, x = rng.standard_normal(col.size), rng.standard_normal(n)
+    assert n < 50 or col.size > 6 * n
+    prod = val * x[col]
+    ref = np.bincount(rows, prod, minlength=n)
+    bound = 2.3e-16 * 2 * (lens + 1) * np.bincount(rows, np.abs(prod), minlength=n)  # a rounding per product and per sum, on either side
+    m = DeviceCsr(row_ptr, col, val)
+    assert (np.abs(m.matvec(x) - ref) <= bound).all()
+    # an x vector that is only 8-byte aligned
+    buf = torch.zeros(n + 1, dtype=torch.float64, device="cuda")
+    buf[1:] = torch.from_numpy(x).cuda()
+    yd = torch.full((n,), float("nan"), dtype=torch.float64, device="cuda")
+    m.matvec_device(buf[1:], yd, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    m.check_status()
+    assert (np.abs(yd.cpu().numpy() - ref) <= bound).all()
+    m.close()
 
 
 def test_device_bicgstab_solves_rc_ladder_system():
@@ -140,21 +174,21 @@ def test_transient_simulation_with_the_device_linear_solver():
     assert np.abs(np.array(dev["values"]) - np.array(ref["values"])).max() < 1e-6
 
 
-def test_graph_captured_iteration_agrees_with_the_host_driven_loop(monkeypatch):
-    """The CUDA-graph form of the BiCGSTAB iteration (scalars on the device, convergence read every 4th
-    iteration) against the loop whose scalars go through the host."""
+def test_one_launch_solve_agrees_with_the_host_driven_loop(monkeypatch):
+    """The solver kernel (the whole solve in one launch, convergence tested every 4th iteration) against the loop whose
+    scalars go through the host."""
     from nangila_spice.gpu import DeviceCsr, tridiagonal
 
     n = 30_001
     row_ptr, col, val = tridiagonal(n, diag=2.2, off=-1.0)
     b = np.random.default_rng(5).standard_normal(n)
     m = DeviceCsr(row_ptr, col, val)
-    x_graph, it_graph, rel_graph, ok_graph = m.solve(b, tol=1e-10, max_iter=400)
+    x_one, it_one, rel_one, ok_one = m.solve(b, tol=1e-10, max_iter=400)
     monkeypatch.setenv("NANGILA_SPMV_GRAPH", "0")
     x_host, it_host, rel_host, ok_host = m.solve(b, tol=1e-10, max_iter=400)
-    assert ok_graph and ok_host and rel_graph < 1e-10 and rel_host < 1e-10
-    assert abs(it_graph - it_host) <= 4  # the graph form tests convergence every 4th iteration
-    assert np.abs(x_graph - x_host).max() < 1e-8 * (np.abs(x_host).max() + 1.0)
+    assert ok_one and ok_host and rel_one < 1e-10 and rel_host < 1e-10
+    assert abs(it_one - it_host) <= 4  # the kernel tests convergence every 4th iteration
+    assert np.abs(x_one - x_host).max() < 1e-8 * (np.abs(x_host).max() + 1.0)
     # a right-hand side of zeros is solved before the first iteration; an unreachable tolerance stops at max_iter
     monkeypatch.delenv("NANGILA_SPMV_GRAPH")
     x0, it0, _, ok0 = m.solve(np.zeros(n))
