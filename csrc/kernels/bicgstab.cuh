@@ -19,8 +19,8 @@
 // a grid-wide sum on 148 CTAs 2.4 (one value) to 3.3 us (five): two block reductions, one counter that one thread per CTA polls,
 // one slot of partial sums read per thread. (A flag per CTA that every CTA polls: 8 us; the slots of all CTAs read by one warp,
 // their values interleaved in shared lines: 4.5 to 9 us.) So a CTA's slice of the matrix stays in shared memory over all iterations where it fits,
-// and small systems run on few CTAs, or on one. Measured on B200, us per iteration, against one CUDA graph of 13 kernels per
-// iteration: mesh of 400 nodes 59 -> 3.8, 2500: 57 -> 6.2, 65 536: 70 -> 8.6, 400 000: 83 -> 22, 10^6: 180 -> 67.
+// and small systems run on few CTAs, or on one. Measured on B200, us per iteration of whole calls, copies included, against
+// one CUDA graph of 13 kernels per iteration: mesh of 400 nodes 59 -> 3.9, 2500: 57 -> 7.0, 65 536: 70 -> 9.0, 400 000: 83 -> 22, 10^6: 180 -> 69.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

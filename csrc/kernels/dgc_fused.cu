@@ -27,9 +27,9 @@
 // with ties the list can be longer than k (it is cut at the capacity; what is cut stays in v).
 //
 // What bounds it: phase 1 is HBM (20 bytes an element with a bf16 bucket); what follows is latency, about 2.5 us a barrier and 1.5
-// a selection. Measured on B200, one rank, bf16, launch included: 13.1 M elements 155 -> 100 us while the threshold grows, 195 -> 84 once it
-// has settled; 1.05 M 80 -> 53. Before, phase 1 also voted every element into a histogram, the selections walked their bins with
-// one warp (45 us), there were eight barriers, and the settled list (36 k entries) often had no room.
+// a selection. Measured on B200, one rank, bf16, launch included, against phase 1 voting every element into a histogram, selections
+// that walk their bins with one warp, and eight barriers: 13.1 M elements, first step 209 -> 160 us, the next four, which have no room on the
+// list, 206 -> 180 to 200, settled 195 -> 87; 1.05 M: 94 -> 52, 89 -> 60, 80 -> 47.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

@@ -5,18 +5,21 @@
 // behind four C calls: init / load_matrix / spmv / free, with the vectors copied over PCIe on every
 // call). Here the product is a hand-written kernel and the vectors can stay on the device.
 //
-// Kernel design ("row blocks"): at load time the host packs consecutive rows into blocks of at most
+// Two designs. Matrices of short rows only (ladders and meshes) take one thread per row: spmv_short_rows_kernel, where the rule
+// stands. All others take "row blocks", as do arrays that the caller owns (nangila_spmv_launch) and matrices loaded under
+// NANGILA_SPMV_PLAIN=1: at load time the host packs consecutive rows into blocks of at most
 // kCap non-zeros. A CTA streams its block's values and column indices with coalesced loads, gathers
 // x through the read-only path, parks the products in shared memory and then reduces each row from
-// there with 1..32 lanes per row (chosen from the block's mean row length), so short rows
-// (3 entries for an RC ladder) cost no idle lanes and long rows still reduce in parallel. A row
+// there with 1..32 lanes per row (chosen from the block's mean row length), so that rows of a few
+// entries cost no idle lanes and long rows still reduce in parallel. A row
 // longer than kCap gets a block of its own and a CTA-wide strided reduction.
 //
-// Two variants of the staging step. The context-owned matrix (nangila_spmv_load) is stored padded
+// Row blocks have two variants of the staging step. The context-owned matrix (nangila_spmv_load) is stored padded
 // to a multiple of four entries, so a CTA fetches its slice of `val` and `col` with two
 // cp.async.bulk copies completing on an mbarrier: the copy engine keeps 24 KB per CTA in flight
 // without spending registers or issue slots, where the plain-load variant was bound by load latency
-// (long-scoreboard stalls at 41 % of DRAM throughput). A further variant that also staged the
+// (long-scoreboard stalls at 41 % of DRAM throughput; tridiagonal, before those took the other design.
+// Nine diagonals, 10^6 rows: 51 us, plain loads 53, blocks of 1024 entries 47). A further variant that also staged the
 // block's window of x in shared memory was measured and dropped: 41 KB and 48 registers per CTA cut
 // residency from 8 to 5 CTAs per SM and the 16 M-row product went from 0.199 ms to 0.254 ms; with
 // one copy per CTA the overlap comes from resident CTAs, so residency matters more than the
@@ -178,10 +181,15 @@ __global__ void __launch_bounds__(T) spmv_row_blocks_bulk_kernel(const int* __re
 // Bound by HBM where the matrix does not fit L2, by the chain row_ptr -> col -> x otherwise; the staged kernel adds to that chain
 // the block table, a barrier initialisation, a copy of the slice and two block barriers, and gives a CTA so much of the matrix that a
 // ladder of 10^6 rows is 1.2 waves of CTAs. Products are rounded and added in the staged kernel's order for two and four lanes a row, so
-// that ladders and meshes keep their bits. Measured on B200, vectors on the device: ladder of 10^6 rows 24 -> 14 us, of 4 10^6 59 -> 41 us
-// (5.5 TB/s); mesh of 10^6 nodes 35 -> 19, of 4 10^6 100 -> 56 us.
-constexpr int kShortRow = 16;   // longest row of a matrix that takes this path
-constexpr int kShortMean = 6;   // and its mean row length: beyond, a lane's serial share outweighs what the staging costs
+// that ladders and meshes keep their bits. Measured on B200, staged kernel and this one, repeated products (10^6 rows lie in L2, 4 10^6 do not):
+// ladder of 10^6 rows 24 -> 14 us, of 4 10^6 59 -> 41 us (5.5 TB/s); mesh of 10^6 nodes 35 -> 19, of 4 10^6 100 -> 56 us. With nothing in L2:
+// rows of 1, 3, 5, 6 entries near the diagonal, 10^6 rows: 23 -> 16, 39 -> 23, 52 -> 35, 55 -> 39 us; anywhere: 31 -> 17, 56 -> 28, 77 -> 39, 83 -> 45.
+//
+// The rule: no row above 16 entries, and at most 6 on average. Uneven rows cost a warp the time of its longest; at the corner of the rule
+// (rows of 1 and of 16, mean 6) what is left is 43.5 -> 41.4 us near the diagonal and 150 -> 142 for 4 10^6 rows, so longer rows and higher means
+// stay with the staged kernel; within it this kernel was the faster one for means 1 to 6, even and uneven, 10^4 to 4 10^6 rows.
+constexpr int kShortRow = 16;
+constexpr int kShortMean = 6;
 __global__ void __launch_bounds__(kThreads) spmv_short_rows_kernel(const int* __restrict__ row_ptr, const int* __restrict__ col,
                                                                    const double* __restrict__ val, const double* __restrict__ x,
                                                                    double* __restrict__ y, int n) {
@@ -271,7 +279,7 @@ struct NangilaSpmv {
     int* d_status = nullptr;  // set by a kernel whose bulk copy timed out
     bool plain_loads = false;  // NANGILA_SPMV_PLAIN=1: use the plain-load kernel
     bool short_rows = false;   // every row suits one thread: spmv_short_rows_kernel
-    int cap = kCap;            // non-zeros per row block: 2048 (256 threads) or 1024 (128 threads, NANGILA_SPMV_TILE=1024)
+    int cap = kCap;            // non-zeros per staged row block: 2048 (256 threads) or 1024 (128 threads, NANGILA_SPMV_TILE=1024)
     double* d_work = nullptr;   // solver vectors (kWorkVectors), allocated on first solve
     double* d_partial = nullptr;  // partial sums, then results and counter of the solver kernel
     std::vector<double> h_inv_diag;

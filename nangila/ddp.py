@@ -156,7 +156,7 @@ class NangilaDDPHook(LivenessMixin):
     Args mirror the reference (ddp.py:100-112). ``num_layers`` is only the size of the all-Driver
     mask of the host-side state machine; device state is created per bucket on first use.
     Extra keyword-only knobs: ``momentum``, ``error_feedback``, ``stochastic`` (rounding of the INT4 codes;
-    default: round to nearest with error feedback, stochastic without), ``dgc_momentum`` (momentum correction factor of the DGC path).
+    default: round to nearest with error feedback, stochastic without; BF16 buckets round to nearest while their gain is 0), ``dgc_momentum`` (momentum correction factor of the DGC path).
     """
 
     def __init__(

@@ -82,9 +82,9 @@ class DGCEngine:
         z = lambda m, dt: torch.zeros(m, dtype=dt, device=self.device)  # noqa: E731
         st = DGCBucket(n=n, k=k, capacity=capacity, region=region, recv_off=recv_off, flag_off=flag_off,
                        u=[z(n, torch.float32) for _ in range(self.nvr)], v=[z(n, torch.float32) for _ in range(self.nvr)],
-                       # fixed words + the candidate list (index, bits) of the list-based selection. Unsent entries
-                       # pile up just below the threshold (about 17 k of them within 4 % of it), and every CTA owns an
-                       # equal segment of the list, hence the slack.
+                       # fixed words + the candidate list (index, bits) of the list-based selection. 4 k candidates are aimed
+                       # at, but unsent entries pile up just below the threshold and layers differ in size, so that a CTA's own
+                       # segment may be full early: half of the list is segments, half takes what finds its segment full.
                        scratch=[z(scratch_words + 2 * (32 * k + 128 * _LIST_CTAS), torch.int32) for _ in range(self.nvr)],
                        out_count=[z(2, torch.int32) for _ in range(self.nvr)])
         self.buckets[index] = st

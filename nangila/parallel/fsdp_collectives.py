@@ -1,7 +1,7 @@
 """Compressed collectives for fully-sharded data parallelism (FSDP2 ``fully_shard``).
 
 * :class:`NangilaReduceScatter` — the gradient reduce-scatter as one fused kernel: every rank
-  block-INT4 quantizes the whole unsharded gradient (stochastic rounding, optional error feedback),
+  block-INT4 quantizes the whole unsharded gradient (optional error feedback; rounding: see the class),
   stores each shard's chunks straight into the owning rank's slots over NVLink, and the owner
   dequantize-accumulates its shard. Each rank receives only its shard: (W-1)/W * 0.53 bytes per
   element cross the links instead of (W-1)/W * 2.
@@ -18,8 +18,8 @@ leaves the parameter all-gather alone.
 By default the momentum predictor is not used here: the sender must know the prediction to subtract
 it, so the history of the averaged gradient would have to live, full size, on every rank, which is
 the memory FSDP exists to avoid (``predictor=True`` buys the reference's behaviour at that price).
-Error feedback is optional for the same reason (off by default; stochastic rounding keeps the
-quantizer unbiased). All state is per FSDP unit.
+Error feedback is optional for the same reason (off by default; for FP32 and FP16 gradients stochastic rounding keeps
+the quantizer unbiased). All state is per FSDP unit.
 """
 from __future__ import annotations
 
@@ -115,6 +115,9 @@ class NangilaReduceScatter(_Base, ReduceScatter):
     memory, a function of the size alone) is shared. The key of the stochastic rounding is
     ``(seed, step + calls of the unit, unit index, rank)``, so it changes every time a unit is reduced
     whether or not anybody advances ``step``.
+
+    ``stochastic`` applies to FP32 and FP16 gradients and to the last, partial chunk of a shard. Whole chunks of BF16 gradients go
+    through packed-BF16 arithmetic, which rounds to nearest whatever it says: there, ``error_feedback=True`` is what removes the bias.
 
     ``predictor=True`` selects the prediction-residual form of the reference's FSDP hook
     (python/nangila/fsdp.py:107-236): every rank keeps the two-step history of the unit's *averaged full*
