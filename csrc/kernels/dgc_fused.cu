@@ -21,15 +21,15 @@
 //   5  wait (bounded) for every rank's list, add value / W into the bucket, list by list in rank order
 // Without a previous threshold, or if the list does not hold the k largest for sure (fewer than k candidates,
 // no room for all of them, a threshold above twice the bound), the threshold comes from a three-pass radix select over
-// the dense state (bits [30:20], [19:9], [8:0]; the first histogram is built in phase 1 if there is no previous threshold, and by a CTA
-// whose list is full from there on).
+// the dense state (bits [30:20], [19:9], [8:0]; the first histogram is built in phase 1 if there is no previous threshold or it came
+// from the dense state itself, and by a CTA whose list is full from there on).
 // The selection is exact either way: tau is the k-th largest |v|. Elements equal to tau are all selected, so
 // with ties the list can be longer than k (it is cut at the capacity; what is cut stays in v).
 //
 // What bounds it: phase 1 is HBM (20 bytes an element with a bf16 bucket); what follows is latency, about 2.5 us a barrier and 1.5
 // a selection. Measured on B200, one rank, bf16, launch included, against phase 1 voting every element into a histogram, selections
-// that walk their bins with one warp, and eight barriers: 13.1 M elements, first step 209 -> 160 us, the next four, which have no room on the
-// list, 206 -> 180 to 200, settled 195 -> 87; 1.05 M: 94 -> 52, 89 -> 60, 80 -> 47.
+// that walk their bins with one warp, and eight barriers: 13.1 M elements, first step 209 -> 160 us, the next five, which have no room on the
+// list, 206 -> 170 to 183, settled 195 -> 87; 1.05 M: 94 -> 52, 89 -> 57, 80 -> 48.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -63,7 +63,8 @@ constexpr int kCoarse = kCursor + 8;        // candidates by distance from the b
 constexpr int kStepBits = 12, kCoarseBins = 2048, kFineBins = 1 << kStepBits;
 constexpr int kFine = kCoarse + kCoarseBins;  // the selected step's candidates by distance
 constexpr int kClearWords = kFine + kFineBins;
-// kept from launch to launch (whatever is there at first does no harm): a threshold, and the bound for the launch after it
+// kept from launch to launch (whatever is there at first does no harm): a threshold, the bound for the launch after it, and the threshold
+// if it came from the dense state
 constexpr int kKept = kClearWords;
 constexpr int kScratchWords = kClearWords + 8;
 constexpr uint32_t kBand = 4;  // candidates wanted, in multiples of k
@@ -160,6 +161,9 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
     cand_thr = __float_as_uint(__uint_as_float(tau_prev) * 0.96f);
     if (scratch[kKept] == tau_prev && scratch[kKept + 1] <= tau_prev) cand_thr = max(cand_thr, scratch[kKept + 1]);
   }
+  // A launch after one that went over the dense state may well have to do so too (the second to seventh step of a large bucket), with a
+  // list that fills up only near the end: it counts top bits from the start, while it collects (67 M fp32 elements, sixth step: 1057 -> 811 us).
+  const bool doubt = use_list && scratch[kKept + 2] == tau_prev;
   // Half of the list is cut into a segment per CTA, which fills it without asking anybody; the candidates are not spread evenly (layers
   // have gradients of different size), so what finds its segment full goes to the other half, place by place.
   const uint32_t seg_cap = cand_cap / 2 / gridDim.x;
@@ -178,7 +182,7 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
   // The candidates among a lane's eight entries, from `first` on; all lanes of a warp come here. Space is reserved once for the
   // warp's 256 entries. Where far more entries qualify than the list holds (the first steps of a bucket, gradients that have jumped) the
   // selection goes over the dense state whatever is collected, so a CTA that has found the list full stops: without that, 13.1 M entries
-  // that all qualify made as many reservations in one word (455 us a step; 180 to 200 this way, 33 M: 1100 to 1200 and 410 to 490). From
+  // that all qualify made as many reservations in one word (455 us a step; 170 to 183 this way, 33 M: 1100 to 1200 and 400 to 430). From
   // there on its warps count bits [30:20] instead, as they do without a previous threshold, so that less is left to be read again.
   // Returns false if the entries were not collected because the list is full.
   volatile uint32_t* list_full = &sh_list_full;
@@ -234,7 +238,7 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
   };
   const int64_t n8 = n / 8, groups8 = (n + 7) / 8, groups8_rounded = (groups8 + 31) / 32 * 32;
   bool collecting = use_list;
-  int64_t vote_from = use_list ? groups8_rounded : 0;  // this lane's groups from here on are in the first histogram (the same iteration for a warp)
+  int64_t vote_from = use_list && !doubt ? groups8_rounded : 0;  // this lane's groups from here on are in the first histogram (the same iteration for a warp)
   for (int64_t q = tid0; q < groups8_rounded; q += stride) {
     float vn[8];
     int valid = 0;
@@ -270,9 +274,9 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
     }
     if (collecting && !collect(q * 8, vn, valid)) {
       collecting = false;
-      vote_from = q;
+      vote_from = min(vote_from, q);
     }
-    if (!collecting) vote_top(vn, valid);
+    if (!collecting || doubt) vote_top(vn, valid);
   }
   __syncthreads();
   auto add_top = [&] {
@@ -282,9 +286,8 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
   if (use_list) {
     for (int i = threadIdx.x; i < kCoarseBins; i += kThreads)
       if (sh_hist[i]) atomicAdd(&scratch[kCoarse + i], sh_hist[i]);
-  } else {
-    add_top();
   }
+  if (!use_list || doubt) add_top();
   const uint32_t my_cand = min(sh_cand_cnt, seg_cap);  // entries of this CTA's segment
   if (threadIdx.x == 0) atomicAdd(&scratch[kCandCount], my_cand);
   if (!gsync()) return;
@@ -374,7 +377,7 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
       }
     };
 
-    if (use_list) {
+    if (use_list && !doubt) {
       // ---- bits [30:20] of what phase 1 went through while it still collected ----
       for (int64_t q = tid0; q < vote_from; q += stride) {
         float x[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
@@ -428,6 +431,7 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
     if (!ssync()) return;
     select_bin<kBins2>(scratch + kHist2, want, bin2, sh_sel);
     tau = (prefix << 9) | bin2;  // bit pattern of the k-th largest |v|
+    if (blockIdx.x == 0 && threadIdx.x == 0) scratch[kKept + 2] = tau;
 
     even_out();
 
