@@ -1,0 +1,76 @@
+// The meeting of the ranks between two kernels of a collective: what the kernel before it in the stream has stored into peers' memory
+// is complete (that kernel has ended), so one word per rank says so, and when every rank's word has arrived the kernel after it
+// may read. A launch of one CTA: while it waits for a peer the rest of the GPU belongs to whatever else is queued, the kernels
+// around it need no flags, no fences and no residency, and the wait is paid once and not by each of their CTAs (1536 CTAs that each
+// looked at four words themselves added 7 us to the reduce-scatter's sum; all of them releasing the words as well, 45 us). All words of the launch's ranks are released before any wait
+// begins, so ranks that are emulated in one launch do not depend on one another's progress. A wait that runs out is recorded in the
+// rank's status block, which the kernel after it reads first.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "nangila_kernels.h"
+#include "signal.cuh"
+
+namespace nangila {
+namespace comm {
+
+struct MeetArgs {
+  uint8_t* region[NANGILA_MAX_RANKS];
+  uint32_t* status[NANGILA_MAX_VRANKS];
+  uint64_t flag_off;  // of the words, one per rank, in every region
+  uint64_t timeout_ns;
+  int32_t world, rank0, nvr;
+  uint32_t epoch, code, phase;
+};
+constexpr int kMeetThreads = NANGILA_MAX_RANKS * NANGILA_MAX_VRANKS;
+
+// The three kernels are launched so that each is set up while the one before it ends (programmatic dependent launch): `follow` waits until
+// that one is complete and its writes are visible, `may_follow` lets the next one be set up from here on.
+__device__ __forceinline__ void follow() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void may_follow() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... Args>
+cudaError_t launch_following(void (*kernel)(Args...), dim3 grid, int threads, cudaStream_t stream, const Args&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+static __global__ void __launch_bounds__(kMeetThreads) meet_kernel(const __grid_constant__ MeetArgs a) {
+  follow();
+  const int v = int(threadIdx.x) / a.world, r = int(threadIdx.x) % a.world;
+  if (v < a.nvr) st_release_sys(reinterpret_cast<uint32_t*>(a.region[r] + a.flag_off) + a.rank0 + v, a.epoch);
+  __syncthreads();
+  if (v < a.nvr && *reinterpret_cast<volatile uint32_t*>(&a.status[v][kStatusCode]) == 0u)
+    wait_flag(reinterpret_cast<const uint32_t*>(a.region[a.rank0 + v] + a.flag_off) + r, a.epoch, a.timeout_ns, a.status[v], a.code,
+              uint32_t(a.rank0 + v), uint32_t(r), a.phase, 0u);
+}
+
+// P: a parameter block with the members that all exchange kernels share.
+template <typename P>
+cudaError_t launch_meet(const P& p, uint64_t flag_off, uint32_t code, uint32_t phase, cudaStream_t stream) {
+  MeetArgs a{};
+  for (int r = 0; r < p.world; ++r) a.region[r] = p.region[r];
+  for (int v = 0; v < p.nvr; ++v) a.status[v] = p.status[v];
+  a.flag_off = flag_off;
+  a.timeout_ns = p.timeout_ns;
+  a.world = p.world;
+  a.rank0 = p.rank0;
+  a.nvr = p.nvr;
+  a.epoch = p.epoch;
+  a.code = code;
+  a.phase = phase;
+  return launch_following(meet_kernel, dim3(1), kMeetThreads, stream, a);
+}
+
+}  // namespace comm
+}  // namespace nangila

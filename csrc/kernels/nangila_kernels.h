@@ -29,7 +29,8 @@ enum NangilaDType { NANGILA_F32 = 0, NANGILA_F16 = 1, NANGILA_BF16 = 2 };
  * Multi-GPU: nvr = 1, rank0 = this rank, `region[r]` = rank r's mapping of the bucket's symmetric
  * region. Single-GPU loopback: nvr = world, rank0 = 0, grid.y = nvr, launched cooperatively.
  * grid_x is clamped to the number of CTAs of the chosen variant that the device can hold at once
- * (occupancy x SM count, divided by nvr); grid_x <= 0 asks for exactly that number.
+ * (occupancy x SM count, divided by nvr); grid_x <= 0 asks for exactly that number. The reduce-scatter (mode 2) has kernels of its
+ * own that need no residency: there grid_x below nchunks is a cap, anything else means as many CTAs as there is work for.
  */
 typedef struct NangilaPredResParams {
   void* grad[NANGILA_MAX_VRANKS];      /* in/out: bucket, n elements of grad_dtype */

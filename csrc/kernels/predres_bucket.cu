@@ -27,6 +27,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "bucket_slots.cuh"
+#include "fsdp_reduce_scatter.cuh"
 #include "launch_util.cuh"
 #include "nangila_kernels.h"
 #include "ptx_sm100.cuh"
@@ -39,29 +41,6 @@ namespace {
 using namespace dev;
 using namespace comm;
 
-constexpr int kThreads = 256;
-constexpr int kE = kElems8;                       // elements per thread per iteration
-constexpr int kElemsPerIter = kThreads * kE;      // 2048
-
-// packed nibbles, then one bf16 scale per 64 elements, then a 16-byte trailer whose first word is the
-// sender's prediction gain (phase 1) or the mean gain of all senders (phase 2)
-__host__ __device__ inline uint64_t compressed_trailer_off(int chunk) {
-  return uint64_t(chunk) / 2 + uint64_t(chunk) / kQuantBlock * 2;
-}
-__host__ __device__ inline uint64_t compressed_slot_bytes(int chunk) { return compressed_trailer_off(chunk) + 16; }
-
-// Slot layout (compressed modes), warp-major so that everything one warp needs from a chunk is
-// contiguous and can be fetched with one bulk copy: packed nibbles [warp][iteration][lane] (4 bytes per
-// lane = 8 elements), then bf16 scales [warp][iteration][4] (one per 64 elements), then the trailer.
-__device__ __forceinline__ uint32_t* packed_ptr(uint8_t* slot, int C, int it, int tid) {
-  const int iters = C / kElemsPerIter;
-  return reinterpret_cast<uint32_t*>(slot) + ((tid >> 5) * iters + it) * 32 + (tid & 31);
-}
-__device__ __forceinline__ uint16_t* scale_ptr(uint8_t* slot, int C, int it, int tid) {
-  const int iters = C / kElemsPerIter;
-  return reinterpret_cast<uint16_t*>(slot + uint64_t(C) / 2) + ((tid >> 5) * iters + it) * 4 + ((tid & 31) >> 3);
-}
-
 struct TaskInfo {
   int phase;      // 1, 2, 3 or 0 (padding task: nothing to do)
   int c;          // chunk id (flag index)
@@ -71,12 +50,11 @@ struct TaskInfo {
   int64_t limit;  // elements at or beyond this index do not belong to the chunk's range
 };
 // All-reduce modes: chunk c covers [c C, (c+1) C) and belongs to rank c % W.
-// Reduce-scatter mode: the bucket is W equal shards; rank o owns shard o, cut into `cps` chunks.
 // Gather mode: every rank pushes each of its packed chunks to all ranks and later sums all W
 // contributions of every chunk itself: tasks are NC quantize tasks followed by NC sum tasks.
-template <bool RS, bool GATHER>
+template <bool GATHER>
 __device__ __forceinline__ TaskInfo decode_task(int task, int me, int W, int NC, int T1, int my_owned, int C,
-                                                int64_t n, int cps, int64_t shard) {
+                                                int64_t n) {
   TaskInfo t;
   if (GATHER) {
     t.phase = task < NC ? 1 : 2;
@@ -90,12 +68,12 @@ __device__ __forceinline__ TaskInfo decode_task(int task, int me, int W, int NC,
     const int k = task / W, d = task % W;
     t.o = (me + 1 + d) % W;  // remote owners first, own chunk last in each round
     t.j = k;
-    t.c = RS ? t.o * cps + k : k * W + t.o;
+    t.c = k * W + t.o;
     t.phase = t.c < NC ? 1 : 0;
   } else if (task < T1 + my_owned) {
     t.j = task - T1;
     t.o = me;
-    t.c = RS ? me * cps + t.j : t.j * W + me;
+    t.c = t.j * W + me;
     t.phase = 2;
   } else {
     t.c = task - T1 - my_owned;
@@ -103,13 +81,8 @@ __device__ __forceinline__ TaskInfo decode_task(int task, int me, int W, int NC,
     t.o = t.c % W;
     t.phase = 3;
   }
-  if (RS) {
-    t.base = int64_t(t.o) * shard + int64_t(t.j) * C;
-    t.limit = int64_t(t.o + 1) * shard;
-  } else {
-    t.base = int64_t(t.c) * C;
-    t.limit = n;
-  }
+  t.base = int64_t(t.c) * C;
+  t.limit = n;
   return t;
 }
 
@@ -398,18 +371,16 @@ constexpr int kSlots = 4;  // completion counters in flight per CTA
 // task's flag (system-scope fence + release store). A block barrier here would leave every warp idle,
 // with no loads in flight, until the slowest one and the fence were done. A warp may run at most
 // kSlots - 1 tasks ahead of the slowest warp of its CTA (the counters are reused round-robin).
-// MODE 0: exact all-reduce; 1: compressed all-reduce; 2: compressed reduce-scatter (phases 1 and 2
-// only: the owner writes the mean of its shard to out_shard, nothing is broadcast, no history);
+// MODE 0: exact all-reduce; 1: compressed all-reduce;
 // 3: compressed all-reduce, lean phase 1 (this rank's gain is zero and no statistics are wanted);
-// (a world of one rank has a kernel of its own: predres_single_kernel;)
+// (a world of one rank has a kernel of its own, predres_single_kernel, and so has the reduce-scatter, fsdp_reduce_scatter.cu;)
 // 6 / 7: gather mode, full / lean (small worlds): phase 1 pushes the packed chunk to every rank, and
 // every rank sums the W contributions of every chunk itself: one quantization, two phases.
 template <typename T, typename S, int MODE>
 __global__ void __launch_bounds__(kThreads, 4)
 predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
   constexpr bool COMPRESSED = MODE != 0;
-  constexpr bool RS = MODE == 2;
-  constexpr bool LEAN = MODE == 2 || MODE == 3 || MODE == 7;
+  constexpr bool LEAN = MODE == 3 || MODE == 7;
   constexpr bool GATHER = MODE == 6 || MODE == 7;
   const int vr = blockIdx.y;
   const int me = p.rank0 + vr;
@@ -418,10 +389,8 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
   const int iters = C / kElemsPerIter;
   const int NC = p.nchunks;
   const int64_t n = p.n;
-  const int64_t shard = RS ? n / W : 0;
-  const int cps = RS ? NC / W : 0;
-  const int owned_max = RS ? cps : (NC + W - 1) / W;
-  const int my_owned = RS ? cps : (NC > me ? (NC - me + W - 1) / W : 0);
+  const int owned_max = (NC + W - 1) / W;
+  const int my_owned = NC > me ? (NC - me + W - 1) / W : 0;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const uint64_t slot = COMPRESSED ? compressed_slot_bytes(C) : uint64_t(C) * sizeof(T);
@@ -429,14 +398,11 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
   uint32_t* status = p.status[vr];
   uint8_t* myreg = p.region[me];
   const int T1 = owned_max * W;
-  const int ntasks = GATHER ? 2 * NC : T1 + my_owned + (RS ? 0 : NC);
-  // Reduce-scatter has no phase 3 to prove that the owner is done reading, so its slots alternate
-  // between two sets by launch parity (a rank cannot get two launches ahead of a peer: its phase 2 of
-  // the launch in between needs that peer's flags).
-  // (gather mode alternates for the same reason: a rank may start the next launch while a peer still sums)
-  const uint64_t recv1 = p.recv1_off + (RS       ? uint64_t(epoch & 1u) * uint64_t(cps) * W * slot
-                                        : GATHER ? uint64_t(epoch & 1u) * uint64_t(NC) * W * slot
-                                                 : 0);
+  const int ntasks = GATHER ? 2 * NC : T1 + my_owned + NC;
+  // Gather mode has no phase 3 to prove that a rank is done reading (it may start the next launch while a peer still sums), so its slots
+  // alternate between two sets by launch parity; a rank cannot get two launches ahead of a peer: its phase 2 of the launch in between
+  // needs that peer's flags.
+  const uint64_t recv1 = p.recv1_off + (GATHER ? uint64_t(epoch & 1u) * uint64_t(NC) * W * slot : 0);
 
   __shared__ int s_count[kSlots];   // warps that have finished the task in this slot
   __shared__ int s_done;            // tasks of this CTA whose flag has been published
@@ -464,7 +430,7 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
   bool failed = false;
 
   const float mu = p.mu;
-  const float kappa = RS ? 0.0f : p.pred_gain[vr];  // this rank's prediction gain for the bucket, in [0, 1]
+  const float kappa = p.pred_gain[vr];  // this rank's prediction gain for the bucket, in [0, 1]
   T* __restrict__ grad = static_cast<T*>(p.grad[vr]);
   S* __restrict__ prev = static_cast<S*>(p.prev[vr]);
   const S* __restrict__ curr = static_cast<const S*>(p.curr[vr]);
@@ -475,7 +441,7 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
   const bool stochastic = p.stochastic != 0;
   // With a zero gain the history only matters for the statistics that steer the gain; the host asks
   // for them on probe steps (p.measure) and the loads are skipped otherwise.
-  const bool use_history = !RS && (kappa != 0.0f || p.measure != 0);
+  const bool use_history = kappa != 0.0f || p.measure != 0;
   // The new history may be left unwritten only where nothing will read it: the caller asks for that
   // while the gain is 0 and no probe is near. A non-zero gain or a probe always writes it.
   const bool keep_history = !COMPRESSED || p.skip_history == 0 || use_history;
@@ -491,7 +457,7 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
 
   int local = 0;  // number of the task within this CTA
   for (int task = task_begin + int(blockIdx.x); task < task_end; task += gridDim.x, ++local) {
-    const TaskInfo t = decode_task<RS, GATHER>(task, me, W, NC, T1, my_owned, C, n, cps, shard);
+    const TaskInfo t = decode_task<GATHER>(task, me, W, NC, T1, my_owned, C, n);
     const int c = t.c, j = t.j;
     const int64_t lim = t.limit;
     // ---- entry (per warp): stop if this rank has failed; do not run too far ahead; wait for inputs ----
@@ -575,7 +541,7 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
           gbar += *reinterpret_cast<const float*>(src0 + uint64_t(r) * slot + compressed_trailer_off(C));
         gbar *= inv_w;
       }
-      if (COMPRESSED && !RS && !GATHER && tid < W) {
+      if (COMPRESSED && !GATHER && tid < W) {
         // mean prediction gain of the senders: every rank applies the same value in phase 3
         float kbar = 0.0f;
         for (int r = 0; r < W; ++r)
@@ -587,12 +553,8 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
       // what happens to the sum of one iteration (8 elements of this lane)
       auto finish = [&](int it, float (&acc)[kE]) {
 #pragma unroll
-        for (int i = 0; i < kE; ++i) acc[i] *= RS ? p.out_scale : inv_w;
-        if constexpr (RS) {
-          // reduce-scatter: the mean of this rank's shard is the result; nothing is broadcast
-          const int64_t local_i = int64_t(j) * C + int64_t(it) * kElemsPerIter + tid * kE;
-          store8_guarded<T>(static_cast<T*>(p.out_shard[vr]), local_i, shard, acc);
-        } else if constexpr (GATHER) {
+        for (int i = 0; i < kE; ++i) acc[i] *= inv_w;
+        if constexpr (GATHER) {
           // the mean of the W dequantized residuals plus the prediction is the result on every rank
           const int64_t base = t.base + int64_t(it) * kElemsPerIter + tid * kE;
           if (base < n) {
@@ -634,17 +596,14 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
           }
         }
       };
-      // packed-bf16 form of the same (quant.cuh): the mean's factor 1 / W (or out_scale) is folded into each
+      // packed-bf16 form of the same (quant.cuh): the mean's factor 1 / W is folded into each
       // rank's block scale, so the sum of the dequantized codes is already the result
       [[maybe_unused]] const bool fast2 = kFastBf16<T, S, LEAN> && t.base + C <= lim && (!GATHER || gbar == 0.0f) &&
-                                          (RS || GATHER || ef2 == nullptr);
+                                          (GATHER || ef2 == nullptr);
       [[maybe_unused]] auto finish_fast = [&](int it, uint32_t (&acc)[4]) {
         if constexpr (kFastBf16<T, S, LEAN>) {
           const uint4 o = make_uint4(acc[0], acc[1], acc[2], acc[3]);
-          if constexpr (RS) {
-            const int64_t local_i = int64_t(j) * C + int64_t(it) * kElemsPerIter + tid * kE;
-            *reinterpret_cast<uint4*>(static_cast<T*>(p.out_shard[vr]) + local_i) = o;
-          } else if constexpr (GATHER) {
+          if constexpr (GATHER) {
             const int64_t base = t.base + int64_t(it) * kElemsPerIter + tid * kE;
             *reinterpret_cast<uint4*>(grad + base) = o;
             if (keep_history) *reinterpret_cast<uint4*>(prev + base) = o;
@@ -661,7 +620,6 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
           }
         }
       };
-      [[maybe_unused]] const float mulw = RS ? p.out_scale : inv_w;
       bool batched = false;
       if constexpr (COMPRESSED) {
         const int ib = min(iters, kHalf / (W * kIterBytes)) & ~1;
@@ -700,7 +658,7 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
                   for (int r = 0; r < W; ++r) {
                     const uint32_t pk = reinterpret_cast<const uint32_t*>(buf + r * ib * 128)[i * 32 + lane];
                     const uint16_t sc = reinterpret_cast<const uint16_t*>(buf + W * ib * 128 + r * ib * 8)[i * 4 + (lane >> 3)];
-                    dequant8_bf16_fma(pk, bf16_rn_bits(bf16_bits_to_float(sc) * mulw), acc2);
+                    dequant8_bf16_fma(pk, bf16_rn_bits(bf16_bits_to_float(sc) * inv_w), acc2);
                   }
                   finish_fast(it0 + i, acc2);
                   continue;
@@ -874,7 +832,7 @@ predres_bucket_kernel(const __grid_constant__ NangilaPredResParams p) {
         } else if (t.phase == 1) {
           __threadfence_system();
           st_release_sys(reinterpret_cast<uint32_t*>(p.region[t.o] + p.flag1_off) + (uint64_t(j) * W + me), epoch);
-        } else if (t.phase == 2 && !RS && !GATHER) {
+        } else if (t.phase == 2 && !GATHER) {
           __threadfence_system();
           for (int r = 0; r < W; ++r)
             st_release_sys(reinterpret_cast<uint32_t*>(p.region[(me + 1 + r) % W] + p.flag2_off) + c, epoch);
@@ -978,7 +936,7 @@ __global__ void __launch_bounds__(kThreads) predres_single_kernel(const __grid_c
 
 template <typename T, typename S, int MODE>
 cudaError_t launch_mode(const NangilaPredResParams& p, cudaStream_t stream) {
-  constexpr bool LEAN = MODE == 2 || MODE == 3 || MODE == 7;
+  constexpr bool LEAN = MODE == 3 || MODE == 7;
   constexpr int smem = MODE == 0 ? 0 : kWarps * Ring<T, S, LEAN>::BYTES_PER_WARP;
   static_assert(Ring<T, S, LEAN>::D <= kMaxDepth, "ring depth");
   const void* fn = reinterpret_cast<const void*>(&predres_bucket_kernel<T, S, MODE>);
@@ -1015,8 +973,7 @@ cudaError_t launch_ts(const NangilaPredResParams& p, cudaStream_t stream) {
   if (p.mode == 0 && p.world == 1) return lean ? launch_single<T, S, true>(p, stream) : launch_single<T, S, false>(p, stream);
   if (p.mode == 0 && p.gather != 0) return lean ? launch_mode<T, S, 7>(p, stream) : launch_mode<T, S, 6>(p, stream);
   if (p.mode == 0) return lean ? launch_mode<T, S, 3>(p, stream) : launch_mode<T, S, 1>(p, stream);
-  if (p.mode == 1) return launch_mode<T, S, 0>(p, stream);
-  return launch_mode<T, S, 2>(p, stream);
+  return launch_mode<T, S, 0>(p, stream);  // mode 1
 }
 
 }  // namespace
@@ -1042,21 +999,6 @@ extern "C" uint64_t nangila_predres_region_bytes(int64_t n, int32_t world, int32
   off = align(off + std::max<uint64_t>(owned_max, gather_ok ? nchunks : 0) * world * 4);
   if (flag2_off) *flag2_off = off;
   off = align(off + nchunks * 4);
-  return off;
-}
-
-// Reduce-scatter mode (mode 2): only the phase-1 slots and flags are needed.
-extern "C" uint64_t nangila_rs_region_bytes(int64_t n, int32_t world, int32_t chunk_elems, uint64_t* recv1_off,
-                                            uint64_t* flag1_off, int32_t* nchunks) {
-  auto align = [](uint64_t x) { return (x + 255) & ~uint64_t(255); };
-  const int64_t shard = n / world;
-  const uint64_t cps = uint64_t((shard + chunk_elems - 1) / chunk_elems);
-  if (nchunks) *nchunks = int32_t(cps * world);
-  uint64_t off = 0;
-  if (recv1_off) *recv1_off = off;
-  off = align(off + 2 * cps * world * nangila::compressed_slot_bytes(chunk_elems));
-  if (flag1_off) *flag1_off = off;
-  off = align(off + cps * world * 4);
   return off;
 }
 
@@ -1098,6 +1040,7 @@ extern "C" int nangila_predres_launch(const NangilaPredResParams* p, cudaStream_
   cudaError_t e;
   const bool s32 = p->state_dtype == NANGILA_F32;
   if (!s32 && p->state_dtype != NANGILA_BF16) return int(cudaErrorInvalidValue);
+  if (p->mode == 2) return int(launch_reduce_scatter(*p, stream));
   switch (p->grad_dtype) {
     case NANGILA_F32:
       e = s32 ? launch_ts<float, float>(*p, stream) : launch_ts<float, __nv_bfloat16>(*p, stream);

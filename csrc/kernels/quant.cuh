@@ -304,14 +304,25 @@ __device__ __forceinline__ bool maybe_nonfinite8(const uint32_t (&w)[4]) {
   return ((t + 0x00800080u) & 0x80008000u) != 0u;
 }
 
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Largest magnitude of eight finite bf16 values.
+__device__ __forceinline__ float absmax8_bf16(const uint32_t (&x)[4]) {
+  const uint32_t m01 = as_u32(__hmax2(__habs2(as_bf162(x[0])), __habs2(as_bf162(x[1]))));
+  const uint32_t m23 = as_u32(__hmax2(__habs2(as_bf162(x[2])), __habs2(as_bf162(x[3]))));
+  const uint32_t m = as_u32(__hmax2(as_bf162(m01), as_bf162(m23)));
+  return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u));
+}
+
 // x[0..3]: eight values as bf16x2 words (element 2j in the low half of word j). On return x holds the error
 // x - q * scale, `qs` the dequantized values q * scale, `packed` the eight codes, `scale_bits` the block's
 // bf16 scale. The eight lanes holding one 64-element block call it together; all values must be finite.
 __device__ __forceinline__ void quantize8_bf16(uint32_t (&x)[4], uint32_t& packed, uint32_t& scale_bits, uint32_t (&qs)[4]) {
-  const uint32_t m01 = as_u32(__hmax2(__habs2(as_bf162(x[0])), __habs2(as_bf162(x[1]))));
-  const uint32_t m23 = as_u32(__hmax2(__habs2(as_bf162(x[2])), __habs2(as_bf162(x[3]))));
-  const uint32_t m = as_u32(__hmax2(as_bf162(m01), as_bf162(m23)));
-  float amax = fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u));
+  float amax = absmax8_bf16(x);
   amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
   amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
   amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
@@ -319,7 +330,10 @@ __device__ __forceinline__ void quantize8_bf16(uint32_t (&x)[4], uint32_t& packe
   const float s = bf16_bits_to_float(scale_bits);
   const bool live = s > 1e-30f;
   if (!live) scale_bits = 0u;
-  const uint32_t inv_bits = live ? (__float_as_uint(__frcp_rn(s)) >> 16) : 0u;  // truncated: never above 1 / s
+  // 1 / s truncated to bf16, never above it. The approximate reciprocal (within 1 ulp) has the same upper 16 bits as the exact one: s has 8 significant
+  // bits, so 1 / s is at least 2^-16 of itself away from every bf16 number unless s is a power of two, and it never is one: no bf16 number
+  // lies in [6.98, 7) and 7 fl(1/7) is above 1.
+  const uint32_t inv_bits = live ? (__float_as_uint(rcp_approx(s)) >> 16) : 0u;
   const bf162 inv2 = as_bf162(inv_bits | (inv_bits << 16));
   const uint32_t s2_bits = scale_bits | (scale_bits << 16);
   const bf162 s2 = as_bf162(s2_bits), neg_s2 = as_bf162(s2_bits ^ 0x80008000u);
@@ -356,23 +370,28 @@ __device__ __forceinline__ uint32_t bf16_rn_bits(float f) {
   return (u + 0x7fffu + ((u >> 16) & 1u)) >> 16;
 }
 
-// acc[j] += q * scale for the eight codes in `packed` (two's complement nibbles), as bf16x2 words.
-__device__ __forceinline__ void dequant8_bf16_fma(uint32_t packed, uint32_t scale_bits, uint32_t (&acc)[4]) {
+// The eight codes in `packed` (two's complement nibbles) as bf16x2 words: element 2j in the low half of word j.
+__device__ __forceinline__ void codes8_bf16(uint32_t packed, bf162 (&q)[4]) {
   const uint32_t w = packed ^ 0x88888888u;                 // offset codes n = q + 8 in [0, 15]
   const uint32_t lo = w & 0x0F0F0F0Fu;                     // elements 0, 2, 4, 6
   const uint32_t hi = (w >> 4) & 0x0F0F0F0Fu;              // elements 1, 3, 5, 7
-  const bf162 s2 = as_bf162(scale_bits | (scale_bits << 16));
   const bf162 off = as_bf162(0x43084308u);                 // 136 = 128 + 8
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    // bytes {lo.byte j, 0, hi.byte j, 0} (selector nibbles 8..15 replicate the byte's sign bit, which is 0 here)
-    const uint32_t sel = uint32_t(j) | (uint32_t(8 + j) << 4) | (uint32_t(4 + j) << 8) | (uint32_t(12 + j) << 12);
-    uint32_t v;  // prmt in PTX: the CUDA intrinsic ignores bit 3 of a selector nibble (the sign-replicate flag)
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(v) : "r"(lo), "r"(hi), "r"(sel));
-    v |= 0x43004300u;                                       // 128 + n in both halves
-    const bf162 q = __hsub2(as_bf162(v), off);              // exact
-    acc[j] = as_u32(__hfma2(q, s2, as_bf162(acc[j])));
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t four = __byte_perm(lo, hi, h == 0 ? 0x5140 : 0x7362);  // elements 4h .. 4h + 3
+    q[2 * h] = __hsub2(as_bf162(__byte_perm(four, 0x43434343u, 0x4140)), off);      // 128 + n in both halves, less 136: exact
+    q[2 * h + 1] = __hsub2(as_bf162(__byte_perm(four, 0x43434343u, 0x4342)), off);
   }
+}
+// acc[j] += q * scale for the eight codes in `packed`, as bf16x2 words; s2: the scale in both halves.
+__device__ __forceinline__ void dequant8_bf16_fma2(uint32_t packed, bf162 s2, uint32_t (&acc)[4]) {
+  bf162 q[4];
+  codes8_bf16(packed, q);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) acc[j] = as_u32(__hfma2(q[j], s2, as_bf162(acc[j])));
+}
+__device__ __forceinline__ void dequant8_bf16_fma(uint32_t packed, uint32_t scale_bits, uint32_t (&acc)[4]) {
+  dequant8_bf16_fma2(packed, as_bf162(scale_bits | (scale_bits << 16)), acc);
 }
 
 template <typename T, bool GUARD>

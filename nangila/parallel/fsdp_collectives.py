@@ -1,6 +1,6 @@
 """Compressed collectives for fully-sharded data parallelism (FSDP2 ``fully_shard``).
 
-* :class:`NangilaReduceScatter` — the gradient reduce-scatter as one fused kernel: every rank
+* :class:`NangilaReduceScatter` — the gradient reduce-scatter as fused kernels: every rank
   block-INT4 quantizes the whole unsharded gradient (optional error feedback; rounding: see the class),
   stores each shard's chunks straight into the owning rank's slots over NVLink, and the owner
   dequantize-accumulates its shard. Each rank receives only its shard: (W-1)/W * 0.53 bytes per
