@@ -1,25 +1,34 @@
 // Quantizing parameter all-gather for fully-sharded training (sm_100a): every rank quantizes its
-// parameter shard to INT8 (default) or INT4 with one bf16 scale per 64 elements, stores the packed
-// chunks straight into every rank's staging slots over NVLink, and every rank dequantizes all W
-// shards directly into the unsharded parameter buffer the next layer reads. One launch replaces
-// all-gather + copy-out; 1.03 (INT8) or 0.53 (INT4) bytes per element cross the links instead of 2.
+// parameter shard to INT8 (default) or INT4 with one bf16 scale per 64 elements, stores the codes
+// straight into every other rank's staging slots over NVLink, and every rank dequantizes the shards
+// straight into the unsharded parameter buffer the next layer reads. 1.03 (INT8) or 0.53 (INT4) bytes per
+// element cross the links instead of 2.
 //
 // The owner of a shard also consumes the dequantized form of its own shard, so all ranks compute
 // with bit-identical parameters. Rounding is to nearest (parameters must not pick up random noise).
+//
+// Three launches, one behind the other: ag_quantize (codes to the peers, this rank's own part of the result; it may be the
+// buffer the shard is read from), the meeting of the ranks (meet.cuh), ag_expand (the other ranks' parts). Grids of short CTAs
+// without flags or fences that the hardware hands out as SMs come free.
+// What bounds them: HBM and L2 traffic. Measured on B200, four ranks on one device, 3.1 M bf16 elements each, INT8 (25 MB in, 39 MB of codes, 100 MB
+// out): 17 us (5.2 TB/s) + 21 us (5.5 TB/s), 42.6 us for the call; as one resident kernel with block barriers and a flag per chunk 49.3 us.
+// The arithmetic is kept out of the way: with divisions by the chunk size, conversions and clamps (250 instructions per eight elements, now 90; 132 and now 35
+// to expand them) the two took 19 and 45 us.
 //
 // The reference leaves the FSDP parameter all-gather untouched (python/nangila/fsdp.py:80-236 only
 // hooks the gradient path).
 //
 // Staging slots are double-buffered by launch parity: a rank may start launch t+1 while a slower
 // peer still dequantizes launch t, but it cannot finish t+1 (and so cannot start t+2) before that
-// peer has started t+1, because it needs the peer's flags of t+1.
+// peer has started t+1, because it needs the peer's word of t+1.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
-#include "launch_util.cuh"
+#include "meet.cuh"
 #include "nangila_kernels.h"
 #include "quant.cuh"
 #include "signal.cuh"
@@ -43,139 +52,178 @@ template <typename T>
 struct __align__(16) Raw {
   T v[kE];
 };
+template <int BITS>
+using Packed = std::conditional_t<BITS == 8, uint2, uint32_t>;  // eight codes
+
+constexpr int kTile = 4;  // iterations of 2048 elements whose loads are issued together
+
+// A rank's shard in the exchange region: its codes one behind the other, then its scales.
+struct AgSlot {
+  uint64_t codes, scales;  // offsets of lane `tid` of iteration `it`; the next iterations follow kThreads lanes, kPerIter / 64 scales further
+  __device__ __forceinline__ AgSlot(const NangilaAgParams& p, int bits, int owner, int it, int tid) {
+    const int C = p.chunk_elems;
+    const uint64_t cps = uint64_t((p.shard_elems + C - 1) / C), bytes = cps * ag_slot_bytes(C, bits);
+    const uint64_t base = p.recv_off + (uint64_t(p.epoch & 1u) * p.world + owner) * bytes;
+    codes = base + (uint64_t(it) * kPerIter + tid * kE) * bits / 8;
+    scales = base + cps * C * bits / 8 + (uint64_t(it) * (kPerIter / kQuantBlock) + tid / 8) * 2;
+  }
+};
+
+// Eight values from their codes. For bf16 in packed arithmetic: a code and a scale have 8 significant bits, so their product is rounded
+// once either way.
+template <typename T, int BITS>
+__device__ __forceinline__ void expand8(const Packed<BITS>& w, uint16_t scale, T* dst) {
+  if constexpr (std::is_same_v<T, __nv_bfloat16>) {
+    const uint32_t bits = scale;
+    const bf162 s2 = as_bf162(bits | (bits << 16));
+    bf162 q[4];
+    if constexpr (BITS == 8) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        // 0x43nn: 128 + the low seven bits, less 128 or (code below zero) 256
+        const uint32_t v = __byte_perm(j < 2 ? w.x : w.y, 0x43434343u, (j & 1) == 0 ? 0x4140 : 0x4342);
+        q[j] = __hsub2(as_bf162(v & 0xff7fff7fu), as_bf162(v & 0xff80ff80u));
+      }
+    } else {
+      codes8_bf16(w, q);
+    }
+    *reinterpret_cast<uint4*>(dst) = make_uint4(as_u32(__hmul2(q[0], s2)), as_u32(__hmul2(q[1], s2)), as_u32(__hmul2(q[2], s2)), as_u32(__hmul2(q[3], s2)));
+  } else {
+    const float s = bf16_bits_to_float(scale);
+    float y[kE];
+#pragma unroll
+    for (int i = 0; i < kE; ++i) {
+      // the code plus 128 (or 8) as the low bits of a float near 2^23: one permutation and one exact subtraction, no conversion
+      if constexpr (BITS == 8) y[i] = (__uint_as_float(__byte_perm((i < 4 ? w.x : w.y) ^ 0x80808080u, 0x4B000000u, 0x7440u + uint32_t(i & 3))) - 8388736.0f) * s;
+      else y[i] = (__uint_as_float((((w ^ 0x88888888u) >> (4 * i)) & 0xfu) | 0x4B000000u) - 8388616.0f) * s;
+    }
+    Vec8<T>::store(dst, y);
+  }
+}
 
 template <typename T, int BITS>
-__global__ void __launch_bounds__(kThreads, 4) fsdp_ag_kernel(const __grid_constant__ NangilaAgParams p) {
-  const int vr = blockIdx.y;
-  const int me = p.rank0 + vr;
-  const int W = p.world;
-  const int C = p.chunk_elems;
-  const int iters = C / kPerIter;
-  const int64_t shard = p.shard_elems;
-  const int cps = int((shard + C - 1) / C);
-  const int tid = threadIdx.x;
-  const uint64_t slot = ag_slot_bytes(C, BITS);
-  const uint64_t set_bytes = uint64_t(W) * cps * slot;
-  const uint64_t recv = p.recv_off + uint64_t(p.epoch & 1u) * set_bytes;
-  const T* __restrict__ in = static_cast<const T*>(p.in_shard[vr]);
-  T* __restrict__ out = static_cast<T*>(p.out_full[vr]);
-  uint32_t* status = p.status[vr];
-  uint8_t* myreg = p.region[me];
-  constexpr float kQmax = BITS == 8 ? 127.0f : 7.0f;
+__global__ void __launch_bounds__(kThreads, 5) ag_quantize_kernel(const __grid_constant__ NangilaAgParams p) {
+  may_follow();
+  const int vr = blockIdx.y, me = p.rank0 + vr, W = p.world, tid = threadIdx.x;
+  const int total = int((p.shard_elems + kPerIter - 1) / kPerIter);
+  // A rank that has failed does nothing more. The word is looked at when the first data are there, so it costs no latency.
+  const uint32_t failed = *reinterpret_cast<volatile uint32_t*>(&p.status[vr][kStatusCode]);
+  const T* in = static_cast<const T*>(p.in_shard[vr]);
+  T* own = static_cast<T*>(p.out_full[vr]) + int64_t(me) * p.shard_elems;  // may be `in`: a lane writes where it has read
   constexpr float kInvQmax = BITS == 8 ? 0.0078740157f : 0.14285715f;
-
-  const int ntasks = cps + W * cps;
-  for (int task = blockIdx.x; task < ntasks; task += gridDim.x) {
-    if (*reinterpret_cast<volatile uint32_t*>(&status[kStatusCode]) != 0u) break;
-    if (task < cps) {
-      // ---- quantize chunk `task` of my shard and store it into every rank's slot [me][task] ----
-      const int j = task;
-      auto quantize = [&](int it, const Raw<T>& raw) {
-        float x[kE];
-        Vec8<T>::load(reinterpret_cast<const T*>(&raw), x);
-        float amax = 0.0f;
+  for (int it0 = blockIdx.x * kTile; it0 < total; it0 += gridDim.x * kTile) {
+    const int64_t at0 = int64_t(it0) * kPerIter + tid * kE, left = p.shard_elems - at0;  // the shard is a multiple of 8: a lane has eight values or none
+    Raw<T> raw[kTile];
+#pragma unroll
+    for (int b = 0; b < kTile; ++b) raw[b] = b * kPerIter < left ? *reinterpret_cast<const Raw<T>*>(in + at0 + b * kPerIter) : Raw<T>{};
+    if (failed != 0u) return;
+    Packed<BITS> w[kTile];
+    uint16_t sb[kTile];
+#pragma unroll
+    for (int b = 0; b < kTile; ++b) {
+      float x[kE], amax = 0.0f;
+      bool clean = false;
+      if constexpr (std::is_same_v<T, __nv_bfloat16>) {
+        const uint4 v = *reinterpret_cast<const uint4*>(&raw[b]);
+        const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+        words_to_float8(words, x);
+        clean = !__any_sync(0xffffffffu, maybe_nonfinite8(words));
+        if (clean) amax = absmax8_bf16(words);
+      } else {
+        Vec8<T>::load(reinterpret_cast<const T*>(&raw[b]), x);
+      }
+      if (!clean) {
 #pragma unroll
         for (int i = 0; i < kE; ++i) {
           x[i] = sanitize(x[i]);
           amax = fmaxf(amax, fabsf(x[i]));
         }
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-        uint32_t sb = bf16_ceil_bits(__fmul_rn(amax, kInvQmax));
-        const float s = bf16_bits_to_float(sb);
-        const bool live = s > 1e-30f;
-        const float inv = live ? __frcp_rn(s) : 0.0f;
-        if (!live) sb = 0;
-        uint32_t w0 = 0, w1 = 0;
-#pragma unroll
-        for (int i = 0; i < kE; ++i) {
-          const int q = int(fminf(fmaxf(rintf(x[i] * inv), -kQmax - 1.0f), kQmax));
-          if (BITS == 8) {
-            if (i < 4) w0 |= (uint32_t(q) & 0xffu) << (8 * i); else w1 |= (uint32_t(q) & 0xffu) << (8 * (i - 4));
-          } else {
-            w0 |= (uint32_t(q) & 0xfu) << (4 * i);
-          }
-        }
-        int rr = me + 1 == W ? 0 : me + 1;  // peers first, this rank last; no division in the loop
-        for (int r = 0; r < W; ++r, rr = (rr + 1 == W ? 0 : rr + 1)) {
-          uint8_t* dst = p.region[rr] + recv + (uint64_t(me) * cps + j) * slot;
-          if (BITS == 8) reinterpret_cast<uint2*>(dst + uint64_t(it) * kPerIter)[tid] = make_uint2(w0, w1);
-          else reinterpret_cast<uint32_t*>(dst + uint64_t(it) * (kPerIter / 2))[tid] = w0;
-          if ((tid & 7) == 0)
-            reinterpret_cast<uint16_t*>(dst + uint64_t(C) * BITS / 8)[it * (kPerIter / kQuantBlock) + tid / 8] = uint16_t(sb);
-        }
-      };
-      // The loads of kBatch iterations are issued before the first is used (the stores into the slots may alias the shard as far as
-      // the compiler knows). The shard is a multiple of 8: a lane has eight values or none.
-      constexpr int kBatch = sizeof(T) == 2 ? 4 : 2;
-      for (int it0 = 0; it0 < iters; it0 += kBatch) {
-        Raw<T> raw[kBatch];
-#pragma unroll
-        for (int b = 0; b < kBatch; ++b) {
-          const int64_t local = int64_t(j) * C + int64_t(it0 + b) * kPerIter + tid * kE;
-          raw[b] = it0 + b < iters && local < shard ? *reinterpret_cast<const Raw<T>*>(in + local) : Raw<T>{};
-        }
-#pragma unroll
-        for (int b = 0; b < kBatch; ++b)
-          if (it0 + b < iters) quantize(it0 + b, raw[b]);
       }
-      __syncthreads();
-      if (tid < W) {
-        __threadfence_system();
-        st_release_sys(reinterpret_cast<uint32_t*>(p.region[tid] + p.flag_off) + (uint64_t(me) * cps + j), p.epoch);
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+      const uint32_t scale = bf16_ceil_bits(__fmul_rn(amax, kInvQmax));
+      const float s = bf16_bits_to_float(scale);
+      const bool live = s > 1e-30f;
+      const float inv = live ? __frcp_rn(s) : 0.0f;
+      sb[b] = uint16_t(live ? scale : 0u);
+      // To the nearest integer, ties to even, by adding 1.5 2^23: the code is in the low bits (conversions run at a quarter of the rate).
+      // The scale is rounded up, so that |x / s| stays below 127.5 (7.5) and needs no clamp.
+      uint32_t q[kE];
+#pragma unroll
+      for (int i = 0; i < kE; ++i) q[i] = __float_as_uint(__fadd_rn(__fmul_rn(x[i], inv), 12582912.0f));
+      const uint32_t lo = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
+      const uint32_t hi = __byte_perm(__byte_perm(q[4], q[5], 0x0040), __byte_perm(q[6], q[7], 0x0040), 0x5410);
+      if constexpr (BITS == 8) {
+        w[b] = make_uint2(lo, hi);
+      } else {
+        const uint32_t a = lo & 0x0F0F0F0Fu, c = hi & 0x0F0F0F0Fu;
+        w[b] = __byte_perm(a | (a >> 4), c | (c >> 4), 0x6420);
       }
-    } else {
-      // ---- dequantize chunk j of owner o into the unsharded buffer ----
-      const int idx = task - cps;
-      const int o = (me + idx / cps) % W;  // own shard first
-      const int j = idx % cps;
-      bool ok = true;
-      if (tid == 0)
-        ok = wait_flag(reinterpret_cast<const uint32_t*>(myreg + p.flag_off) + (uint64_t(o) * cps + j), p.epoch,
-                       p.timeout_ns, status, kTimeoutPhase3, uint32_t(me), uint32_t(o), 3u, uint32_t(j));
-      if (!__syncthreads_and(ok ? 1 : 0)) break;
-      const uint8_t* src = myreg + recv + (uint64_t(o) * cps + j) * slot;
-      // The packed words and scales of kB iterations are fetched before any of them is expanded: the
-      // stores to `out` may alias the slot as far as the compiler knows, so without this every load
-      // would wait for the previous iteration's stores.
-      constexpr int kB = 4;
-      for (int it0 = 0; it0 < iters; it0 += kB) {
-        uint2 w[kB];
-        uint16_t sc[kB];
+    }
+    const AgSlot slot(p, BITS, me, it0, tid);
+    for (int d = 1, r = me + 1; d < W; ++d, ++r) {
+      if (r == W) r = 0;
+      Packed<BITS>* codes = reinterpret_cast<Packed<BITS>*>(p.region[r] + slot.codes);
+      uint16_t* scales = reinterpret_cast<uint16_t*>(p.region[r] + slot.scales);
 #pragma unroll
-        for (int b = 0; b < kB; ++b) {
-          const int it = it0 + b;
-          w[b] = make_uint2(0u, 0u);
-          sc[b] = 0;
-          if (it < iters && int64_t(j) * C + int64_t(it) * kPerIter + tid * kE < shard) {
-            sc[b] = reinterpret_cast<const uint16_t*>(src + uint64_t(C) * BITS / 8)[it * (kPerIter / kQuantBlock) + tid / 8];
-            if (BITS == 8) w[b] = reinterpret_cast<const uint2*>(src + uint64_t(it) * kPerIter)[tid];
-            else w[b].x = reinterpret_cast<const uint32_t*>(src + uint64_t(it) * (kPerIter / 2))[tid];
-          }
-        }
-#pragma unroll
-        for (int b = 0; b < kB; ++b) {
-          const int it = it0 + b;
-          const int64_t local = int64_t(j) * C + int64_t(it) * kPerIter + tid * kE;
-          if (it >= iters || local >= shard) continue;
-          const float s = bf16_bits_to_float(sc[b]);
-          float y[kE];
-          if (BITS == 8) {
-#pragma unroll
-            for (int i = 0; i < kE; ++i) {
-              const uint32_t ww = i < 4 ? w[b].x : w[b].y;
-              y[i] = float(int(ww << (24 - 8 * (i & 3))) >> 24) * s;
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < kE; ++i) y[i] = float(int(w[b].x << (28 - 4 * i)) >> 28) * s;
-          }
-          store8_guarded<T>(out + int64_t(o) * shard, local, shard, y);
+      for (int b = 0; b < kTile; ++b) {
+        if (it0 + b < total) {
+          codes[b * kThreads] = w[b];
+          if ((tid & 7) == 0) scales[b * (kPerIter / kQuantBlock)] = sb[b];
         }
       }
     }
+    // this rank's own part of the result: what the others make of the codes
+#pragma unroll
+    for (int b = 0; b < kTile; ++b)
+      if (b * kPerIter < left) expand8<T, BITS>(w[b], sb[b], own + at0 + b * kPerIter);
   }
+}
+
+template <typename T, int BITS>
+__global__ void __launch_bounds__(kThreads, 8) ag_expand_kernel(const __grid_constant__ NangilaAgParams p, int tiles) {
+  const int vr = blockIdx.z, me = p.rank0 + vr, W = p.world, tid = threadIdx.x;
+  int o = me + 1 + int(blockIdx.y);  // the other ranks' shards
+  if (o >= W) o -= W;
+  follow();
+  const uint32_t failed = *reinterpret_cast<volatile uint32_t*>(&p.status[vr][kStatusCode]);  // not 0: a rank's data did not come
+  const uint8_t* myreg = p.region[me];
+  T* __restrict__ out = static_cast<T*>(p.out_full[vr]) + int64_t(o) * p.shard_elems;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int64_t at0 = int64_t(tile) * (kTile * kPerIter) + tid * kE, left = p.shard_elems - at0;
+    const AgSlot slot(p, BITS, o, tile * kTile, tid);
+    const Packed<BITS>* codes = reinterpret_cast<const Packed<BITS>*>(myreg + slot.codes);
+    const uint16_t* scales = reinterpret_cast<const uint16_t*>(myreg + slot.scales);
+    Packed<BITS> w[kTile];
+    uint16_t sc[kTile];
+#pragma unroll
+    for (int b = 0; b < kTile; ++b) {
+      if (b * kPerIter < left) {
+        w[b] = codes[b * kThreads];
+        sc[b] = scales[b * (kPerIter / kQuantBlock)];
+      }
+    }
+    if (failed != 0u) return;
+#pragma unroll
+    for (int b = 0; b < kTile; ++b)
+      if (b * kPerIter < left) expand8<T, BITS>(w[b], sc[b], out + at0 + b * kPerIter);
+  }
+}
+
+template <typename T, int BITS>
+cudaError_t launch(const NangilaAgParams& p, cudaStream_t stream) {
+  const int64_t total = (p.shard_elems + kPerIter - 1) / kPerIter, tiles = (total + kTile - 1) / kTile;
+  if (total > 0x3fffffff) return cudaErrorInvalidValue;
+  // fewer CTAs asked for than chunks to quantize and to expand: a cap
+  const int64_t cps = (p.shard_elems + p.chunk_elems - 1) / p.chunk_elems;
+  const int64_t cap = p.grid_x > 0 && p.grid_x < cps * (p.world + 1) ? p.grid_x : 0x7fffffff;
+  ag_quantize_kernel<T, BITS><<<dim3(unsigned(std::min(cap, tiles)), unsigned(p.nvr)), kThreads, 0, stream>>>(p);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || p.world == 1) return e;
+  if ((e = launch_meet(p, p.flag_off, kTimeoutPhase3, 3u, stream)) != cudaSuccess) return e;
+  const dim3 grid(unsigned(std::min(std::max<int64_t>(1, cap / (p.world - 1)), tiles)), unsigned(p.world - 1), unsigned(p.nvr));
+  return launch_following(ag_expand_kernel<T, BITS>, grid, kThreads, stream, p, int(tiles));
 }
 
 }  // namespace
@@ -193,11 +241,9 @@ extern "C" uint64_t nangila_ag_region_bytes(int64_t shard_elems, int32_t world, 
   return off;
 }
 
-// Chunk size for a shard. A rank has one quantize task per chunk and W dequantize tasks, walked by the CTAs a whole device holds at
-// once (`resident` per rank, from NANGILA_LAYOUT_CTAS: 64 registers and 256 threads make four an SM): the largest chunk that still gives every CTA a quantize task, in whole iterations, since each
-// task ends in a block barrier and a system-wide flag (four ranks, 3.1 M bf16 elements each: chunks of 4096 elements 120 us,
-// 8192 78, 24576 59, 32768 64; the rule gives 22528 there, one rank alone 6144). Not below 4096 elements, where a task is nearly all barrier and flag (131 072 elements on four ranks:
-// 19.7 us, 21.4 with 2048), except for shards of less than four such chunks.
+// Chunk size for a shard: what a rank's slot is rounded up to, and the unit of the caller's cap on CTAs. About one chunk for each of the `resident`
+// CTAs that a device holds at once per rank (NANGILA_LAYOUT_CTAS), not below 4096 elements except for shards of less than four
+// such chunks. The same on every rank, whatever its device: peers write into one another's slots.
 extern "C" int32_t nangila_ag_chunk_elems(int64_t shard_elems, int32_t resident) {
   const int64_t g = resident > 0 ? resident : 1, most = 131072;
   const int64_t waves = std::max<int64_t>(1, (shard_elems + g * most - 1) / (g * most));
@@ -213,22 +259,10 @@ extern "C" int nangila_ag_launch(const NangilaAgParams* p, cudaStream_t stream) 
       (p->nvr > 1 && p->nvr != p->world) || p->chunk_elems <= 0 || p->chunk_elems % kPerIter != 0 || p->epoch == 0 ||
       (p->bits != 8 && p->bits != 4))
     return int(cudaErrorInvalidValue);
-  const void* fn = nullptr;
-#define NANGILA_AG_PICK(TYPE)                                                                  \
-  fn = p->bits == 8 ? reinterpret_cast<const void*>(&fsdp_ag_kernel<TYPE, 8>)                  \
-                    : reinterpret_cast<const void*>(&fsdp_ag_kernel<TYPE, 4>)
   switch (p->dtype) {
-    case NANGILA_F32: NANGILA_AG_PICK(float); break;
-    case NANGILA_BF16: NANGILA_AG_PICK(__nv_bfloat16); break;
-    case NANGILA_F16: NANGILA_AG_PICK(__half); break;
+    case NANGILA_F32: return int(p->bits == 8 ? launch<float, 8>(*p, stream) : launch<float, 4>(*p, stream));
+    case NANGILA_BF16: return int(p->bits == 8 ? launch<__nv_bfloat16, 8>(*p, stream) : launch<__nv_bfloat16, 4>(*p, stream));
+    case NANGILA_F16: return int(p->bits == 8 ? launch<__half, 8>(*p, stream) : launch<__half, 4>(*p, stream));
     default: return int(cudaErrorInvalidValue);
   }
-#undef NANGILA_AG_PICK
-  int grid_x = 0;
-  const cudaError_t ce = clamp_grid(fn, kThreads, 0, p->grid_x, p->nvr, &grid_x);
-  if (ce != cudaSuccess) return int(ce);
-  dim3 grid(unsigned(grid_x), unsigned(p->nvr)), block(kThreads);
-  void* args[] = {const_cast<NangilaAgParams*>(p)};
-  if (p->nvr > 1) return int(cudaLaunchCooperativeKernel(fn, grid, block, args, 0, stream));
-  return int(cudaLaunchKernel(fn, grid, block, args, 0, stream));
 }
