@@ -455,6 +455,8 @@ PYBIND11_MODULE(_C, m) {
         s.record(id, static_cast<const float*>(bi.ptr), size_t(bi.size));
       })
       .def("record_norm", &Sculptor::record_norm)
+      .def("note_size", &Sculptor::note_size)
+      .def("schedule_needs_norms", &Sculptor::schedule_needs_norms)
       .def("end_step", &Sculptor::end_step)
       .def("note_step", &Sculptor::note_step)
       .def("set_pair_result", &Sculptor::set_pair_result)

@@ -58,6 +58,11 @@ class Sculptor {
     stats_[id].update(l2_norm);
   }
 
+  // The size alone, for a caller that schedules pairs before it knows the norms.
+  void note_size(LayerId id, size_t numel) { layer_sizes_[id] = numel; }
+  // Whether `scheduled_pairs` depends on the norms of the step.
+  bool schedule_needs_norms() const { return strategy_.kind == SamplingStrategy::KNearestNeighbors; }
+
   void end_step() {
     std::vector<LayerId> ids;
     for (auto& kv : current_) ids.push_back(kv.first);  // map order = ascending id

@@ -9,6 +9,7 @@ scalars (reference: nangila-core/src/sculptor.rs:238-550, all on the host there)
 """
 from __future__ import annotations
 
+import math
 from typing import Dict, List, Tuple
 
 import torch
@@ -42,9 +43,35 @@ class DeviceSculptor:
             return
         ids = sorted(self._current)
         tensors = [self._current[i] for i in ids]
-        sumsq = self._glue.sculptor_layer_sumsq(tensors).sqrt().tolist()
-        for i, norm in zip(ids, sumsq):
-            self.core.record_norm(i, norm, self._current[i].numel())
+        # The norms come to the host while the pair statistics, which do not depend on them, are queued and run; only the nearest-neighbour
+        # schedule has to wait for them. (28 pairs of eight 589 824-element bf16 layers, a step: 176 us with the host reading the norms first, 126 so.)
+        sumsq = self._glue.sculptor_layer_sumsq(tensors)
+        host = torch.empty(len(ids), dtype=torch.float64, pin_memory=True)
+        with torch.cuda.device(sumsq.device):
+            host.copy_(sumsq, non_blocking=True)
+            arrived = torch.cuda.Event()
+            arrived.record()
+
+        def record_norms() -> None:
+            arrived.synchronize()
+            for i, ss in zip(ids, host.tolist()):
+                self.core.record_norm(i, math.sqrt(ss), self._current[i].numel())
+
+        if self.core.schedule_needs_norms():
+            record_norms()
+            self._update_pairs(ids, tensors)
+        else:
+            for i in ids:
+                self.core.note_size(i, self._current[i].numel())
+            try:
+                self._update_pairs(ids, tensors)
+            finally:
+                record_norms()
+        self.core.note_step()
+        self._steps += 1
+        self._current.clear()
+
+    def _update_pairs(self, ids: List[int], tensors: List[torch.Tensor]) -> None:
         pairs = self.core.scheduled_pairs(ids)
         if pairs:
             xi, xj, st, cnt = [], [], [], []
@@ -72,9 +99,6 @@ class DeviceSculptor:
             for batch in batches:
                 self._glue.sculptor_pair_update([xi[k] for k in batch], [xj[k] for k in batch], [st[k] for k in batch],
                                                 [cnt[k] for k in batch])
-        self.core.note_step()
-        self._steps += 1
-        self._current.clear()
 
     def _finalize(self) -> None:
         keys = [k for k, c in self._pair_count.items() if c >= 2]
