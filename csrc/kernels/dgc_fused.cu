@@ -26,10 +26,11 @@
 // The selection is exact either way: tau is the k-th largest |v|. Elements equal to tau are all selected, so
 // with ties the list can be longer than k (it is cut at the capacity; what is cut stays in v).
 //
-// What bounds it: phase 1 is HBM (20 bytes an element with a bf16 bucket); what follows is latency, about 2.5 us a barrier and 1.5
-// a selection. Measured on B200, one rank, bf16, launch included, against phase 1 voting every element into a histogram, selections
-// that walk their bins with one warp, and eight barriers: 13.1 M elements, first step 209 -> 160 us, the next five, which have no room on the
-// list, 206 -> 170 to 183, settled 195 -> 87; 1.05 M: 94 -> 52, 89 -> 57, 80 -> 48.
+// What bounds it: phase 1 is HBM (20 bytes an element with a bf16 bucket); what follows is latency, about 2.5 us a barrier and 1.5 to 2
+// a selection. Measured on B200, one rank, bf16, copy of the gradient into the bucket included: 13.1 M elements, settled, 73 us (87 with selections that read
+// the histograms a word at a time, 195 with phase 1 voting every element and eight barriers). Without that copy, before the selections were
+// mended: first step 160 us, the next five, which have no room on the list, 170 to 183; 1.05 M: 52, 57, settled 48.
+
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -340,20 +341,10 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
     };
     for (uint32_t j = threadIdx.x; j < my_cand; j += kThreads) count_fine(cand_bits[j]);
     for (uint32_t j = uint32_t(tid0); j < nspill; j += uint32_t(stride)) count_fine(__ldcg(spill_bits + j));
-    uint32_t next_bound = 0;
-    if (blockIdx.x == 0) {
-      uint32_t rank = min(kBand * p.k, ncand), bin;
-      select_bin<kCoarseBins>(scratch + kCoarse, rank, bin, sh_sel);
-      next_bound = cand_thr + (bin << kStepBits);
-    }
     if (!ssync()) return;
     uint32_t fine;
     select_bin<kFineBins>(scratch + kFine, want, fine, sh_sel);
     tau = cand_thr + (coarse << kStepBits) + fine;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {  // every CTA has read the old pair before the first barrier
-      scratch[kKept] = tau;
-      scratch[kKept + 1] = next_bound;
-    }
     even_out();
     const uint32_t nc_rounded = (my_cand + 31u) / 32u * 32u;
     for (uint32_t j = threadIdx.x; j < nc_rounded; j += kThreads) {
@@ -364,6 +355,14 @@ __global__ void __launch_bounds__(kThreads, 3) dgc_fused_kernel(const __grid_con
     for (uint32_t j = uint32_t(tid0); j < ns_rounded; j += uint32_t(stride)) {
       const bool sel = j < nspill && __ldcg(spill_bits + j) >= tau && p.k > 0;
       append(sel, sel ? int64_t(__ldcg(spill_idx + j)) : 0);
+    }
+    if (blockIdx.x == 0) {  // nobody waits for this; every CTA has read the old pair before the first barrier
+      uint32_t rank = min(kBand * p.k, ncand), bin;
+      select_bin<kCoarseBins>(scratch + kCoarse, rank, bin, sh_sel);
+      if (threadIdx.x == 0) {
+        scratch[kKept] = tau;
+        scratch[kKept + 1] = cand_thr + (bin << kStepBits);
+      }
     }
   } else {
     // bit patterns of |v| for one group (0 beyond the end: never selected, never counted)
