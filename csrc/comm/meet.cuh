@@ -10,6 +10,7 @@
 
 #include <cstdint>
 
+#include "follow.cuh"
 #include "nangila_kernels.h"
 #include "signal.cuh"
 
@@ -25,25 +26,6 @@ struct MeetArgs {
   uint32_t epoch, code, phase;
 };
 constexpr int kMeetThreads = NANGILA_MAX_RANKS * NANGILA_MAX_VRANKS;
-
-// The three kernels are launched so that each is set up while the one before it ends (programmatic dependent launch): `follow` waits until
-// that one is complete and its writes are visible, `may_follow` lets the next one be set up from here on.
-__device__ __forceinline__ void follow() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void may_follow() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-template <typename... Args>
-cudaError_t launch_following(void (*kernel)(Args...), dim3 grid, int threads, cudaStream_t stream, const Args&... args) {
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(unsigned(threads));
-  cfg.stream = stream;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
 
 static __global__ void __launch_bounds__(kMeetThreads) meet_kernel(const __grid_constant__ MeetArgs a) {
   follow();
@@ -69,7 +51,7 @@ cudaError_t launch_meet(const P& p, uint64_t flag_off, uint32_t code, uint32_t p
   a.epoch = p.epoch;
   a.code = code;
   a.phase = phase;
-  return launch_following(meet_kernel, dim3(1), kMeetThreads, stream, a);
+  return launch_following(meet_kernel, dim3(1), kMeetThreads, 0, stream, a);
 }
 
 }  // namespace comm

@@ -400,6 +400,12 @@ void psgd_gemm(const at::Tensor& M, const at::Tensor& Bt, bool transposed, at::T
     }
     for (size_t r = 0; r < push_region_ptrs.size(); ++r) push.region[r] = as_ptr(push_region_ptrs[r]);
   }
+  if (!pushing && push_rank > 0) {  // no exchange, but only the factor's columns are wanted
+    check_launch(nangila_psgd_gemm_columns(M.data_ptr(), int32_t(m), int32_t(n), Bt.data_ptr(), transposed ? 1 : 0, out.data_ptr<float>(),
+                                           int32_t(push_rank), reinterpret_cast<uint32_t*>(status.data_ptr<int32_t>()),
+                                           uint64_t(timeout_s * 1e9), at::cuda::getCurrentCUDAStream()), "psgd_gemm");
+    return;
+  }
   check_launch(nangila_psgd_gemm_push(M.data_ptr(), int32_t(m), int32_t(n), Bt.data_ptr(), transposed ? 1 : 0, out.data_ptr<float>(),
                                       pushing ? &push : nullptr, reinterpret_cast<uint32_t*>(status.data_ptr<int32_t>()),
                                       uint64_t(timeout_s * 1e9), at::cuda::getCurrentCUDAStream()), "psgd_gemm");

@@ -223,7 +223,7 @@ cudaError_t launch(const NangilaAgParams& p, cudaStream_t stream) {
   if (e != cudaSuccess || p.world == 1) return e;
   if ((e = launch_meet(p, p.flag_off, kTimeoutPhase3, 3u, stream)) != cudaSuccess) return e;
   const dim3 grid(unsigned(std::min(std::max<int64_t>(1, cap / (p.world - 1)), tiles)), unsigned(p.world - 1), unsigned(p.nvr));
-  return launch_following(ag_expand_kernel<T, BITS>, grid, kThreads, stream, p, int(tiles));
+  return launch_following(ag_expand_kernel<T, BITS>, grid, kThreads, 0, stream, p, int(tiles));
 }
 
 }  // namespace

@@ -242,7 +242,7 @@ cudaError_t launch(const NangilaPredResParams& p, cudaStream_t stream) {
     if (e == cudaSuccess) e = launch_meet(p, p.flag1_off, kTimeoutPhase2, 2u, stream);
     if (e != cudaSuccess) return e;
     const dim3 grid(unsigned(cap > 0 ? std::min(tiles, cap) : tiles), unsigned(p.nvr));
-    return launch_following(rs_sum_kernel<T, kPackedBf16<T, S>>, grid, kThreads, stream, p, tiles);
+    return launch_following(rs_sum_kernel<T, kPackedBf16<T, S>>, grid, kThreads, 0, stream, p, tiles);
   }
   return cudaGetLastError();
 }

@@ -114,6 +114,9 @@ int nangila_ag_launch(const NangilaAgParams* p, cudaStream_t stream);
  * (transposed = 1, rows = n). M: m x n bf16 row-major, m and n multiples of 8. Bt: 16 x K bf16. */
 int nangila_psgd_gemm(const void* M, int32_t m, int32_t n, const void* Bt, int32_t transposed, float* out,
                       uint32_t* status, uint64_t timeout_ns, cudaStream_t stream);
+/* The same GEMM where only the first `columns` (1 to 16) columns of `out` are wanted: the others may be left as they are. */
+int nangila_psgd_gemm_columns(const void* M, int32_t m, int32_t n, const void* Bt, int32_t transposed, float* out, int32_t columns,
+                              uint32_t* status, uint64_t timeout_ns, cudaStream_t stream);
 /* The same GEMM with the cross-rank exchange of its result started from the epilogue: the CTA that completes a
  * 128-row tile of `out` (the last of the tile's K splits to arrive) stores the tile's first `rank` columns, column-major,
  * into slot [me] of EVERY rank's exchange region (peer stores over NVLink, this rank's own region included), and the CTA

@@ -26,6 +26,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "follow.cuh"
 #include "nangila_kernels.h"
 #include "ptx_sm100.cuh"
 #include "quant.cuh"
@@ -57,7 +58,7 @@ constexpr int kGemmSmem = kStages * kStageBytes + 1024 /*alignment slack*/ + 256
 template <bool A_MN>
 __global__ void __launch_bounds__(kGemmThreads)
 psgd_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 float* __restrict__ out, int rows_out, int k_total, int k_per_split, int use_atomics,
+                 float* __restrict__ out, int rows_out, int k_total, int k_per_split, int use_atomics, int columns,
                  uint32_t* status, uint64_t timeout_ns, const __grid_constant__ NangilaPsgdPush push) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -90,6 +91,8 @@ psgd_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  may_follow();
+  follow();
 
   if (nslabs > 0) {
     if (warp == 0 && lane == 0) {
@@ -152,11 +155,10 @@ psgd_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (row < rows_out) {
         float* dst = out + int64_t(row) * kCols;
         if (use_atomics) {
-          // four columns per reduction; with a push only the factor's columns are ever read
-          const int cols = push.counters != nullptr ? push.rank : kCols;
+          // four columns per reduction, and none that nobody reads
 #pragma unroll
           for (int c = 0; c < kCols; c += 4)
-            if (c < cols)
+            if (c < columns)
               asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + c), "f"(v[c]), "f"(v[c + 1]), "f"(v[c + 2]), "f"(v[c + 3])
                            : "memory");
         } else {
@@ -227,6 +229,7 @@ __global__ void __launch_bounds__(256) psgd_prep_kernel(const T* __restrict__ gr
                                                        __nv_bfloat16* __restrict__ mef, int64_t numel,
                                                        float* __restrict__ z0, int64_t n0, float* __restrict__ z1,
                                                        int64_t n1) {
+  may_follow();
   const int64_t t0 = int64_t(blockIdx.x) * 256 + threadIdx.x, stride = int64_t(gridDim.x) * 256;
   // Eight elements a thread where the addresses allow it (bound by HBM; one element a thread was bound by latency: 2.4 M elements
   // 4.7 -> 3.6 us).
@@ -255,6 +258,7 @@ __global__ void __launch_bounds__(256) psgd_reconstruct_kernel(T* __restrict__ g
                                                               const __nv_bfloat16* __restrict__ mef,
                                                               const float* __restrict__ P, const float* __restrict__ Q,
                                                               int m, int n, int r) {
+  follow();
   const int col = (blockIdx.x * 256 + threadIdx.x) * 8;
   if (col >= n) return;  // n is a multiple of 8
   float q[RQ > 0 ? RQ : 1][8];
@@ -320,6 +324,8 @@ __global__ void __launch_bounds__(256) psgd_reconstruct_kernel(T* __restrict__ g
 // two cluster barriers and two factorisations per launch and no trip to L2. Measured on B200, rank 4, 2048 rows: 23.5 -> 9.9 us;
 // rank 8 (four factors of 512 to 4608 rows at once): 72 -> 18 us each. Before, every pass went through memory, and one thread
 // factorised with its matrices in local memory.
+// A rank on its own reads the factor where the GEMM left it. The GEMM then needs no counters, no second look at its tiles and no flag (11 -> 5.5 us), and
+// with every kernel of the chain set up while the one before it ends, the four matrices of a ResNet-50 bucket (2.4 to 1.0 M elements, rank 4) take 49 us and not 67.
 constexpr int kXCtas = 8;
 constexpr int kXThreads = 512;
 constexpr int kXWarps = kXThreads / 32;
@@ -393,6 +399,9 @@ __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_c
   const int W = p.world, rows = p.rows, r = p.rank;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint64_t slot_bytes = (uint64_t(rows) * r * 4 + 255) & ~uint64_t(255);
+  follow();
+  // nobody to exchange with: the factor is read where the GEMM left it, four columns at a time
+  const bool alone = W == 1 && p.pushed == 0 && (reinterpret_cast<uintptr_t>(p.local[vr]) & 15u) == 0;
   const uint32_t epoch = p.epoch_dev != nullptr ? *p.epoch_dev : p.epoch;
   const uint64_t base = p.recv_off + uint64_t(epoch & 1u) * W * slot_bytes;  // two slot sets, by launch parity
   uint32_t* status = p.status[vr];
@@ -411,7 +420,7 @@ __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_c
 
   // 1. store my rows of my factor (r columns, column-major) into every rank's slot [me] (unless the GEMM's
   //    epilogue has done that already)
-  if (p.pushed == 0) {
+  if (p.pushed == 0 && !alone) {
     for (int d = 0; d < W; ++d) {
       float* dst = reinterpret_cast<float*>(p.region[(me + d) % W] + base + uint64_t(me) * slot_bytes);
       for (int c = 0; c < r; ++c)
@@ -428,19 +437,39 @@ __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_c
   //    the cluster barriers below, doing no work)
   if (tid == 0) s_ok = 1;
   __syncthreads();
-  if (tid < W) {
+  if (tid < W && !alone) {
     if (!wait_flag(reinterpret_cast<const uint32_t*>(p.region[me] + p.flag_off) + tid, epoch, p.timeout_ns, status,
                    kTimeoutPhase2, uint32_t(me), uint32_t(tid), 8u, 0u))
       s_ok = 0;
   }
   __syncthreads();
   const bool ok = s_ok != 0;
+  if (p.orth_mean != 0) may_follow();  // a GEMM of a few CTAs comes next; the reconstruction after the other exchange would fill the device
   // 3. mean in rank order (identical on every rank); columns >= r are zero
   float* work = SMEM ? s_rows : (p.orth_mean ? mean : p.scratch[vr]) + r0;
   const int pitch = SMEM ? per : rows;  // element (row r0 + i, c) at work[c * pitch + i]
   if (ok) {
     const float inv_w = 1.0f / float(W);
-    for (int c = 0; c < r; ++c)
+    if (alone) {
+      for (int i = tid; i < mine; i += kXThreads) {
+        const float4* row = reinterpret_cast<const float4*>(local + int64_t(r0 + i) * kCols);
+#pragma unroll
+        for (int c4 = 0; c4 < RMAX; c4 += 4) {
+          if (c4 < r) {
+            const float4 q = __ldcg(row + c4 / 4);
+            const float v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              if (c4 + k < r) {
+                if (!p.orth_mean) mean[int64_t(c4 + k) * rows + r0 + i] = v[k];
+                work[int64_t(c4 + k) * pitch + i] = v[k];
+              }
+            }
+          }
+        }
+      }
+    }
+    for (int c = alone ? r : 0; c < r; ++c)
       for (int i = tid; i < mine; i += kXThreads) {
         float acc = 0.0f;
         for (int src = 0; src < W; ++src)
@@ -584,9 +613,23 @@ extern "C" int nangila_psgd_gemm(const void* M, int32_t m, int32_t n, const void
   return nangila_psgd_gemm_push(M, m, n, Bt, transposed, out, nullptr, status, timeout_ns, stream);
 }
 
+static int launch_gemm(const void* M, int32_t m, int32_t n, const void* Bt, int32_t transposed, float* out, int32_t columns,
+                       const NangilaPsgdPush* push_in, uint32_t* status, uint64_t timeout_ns, cudaStream_t stream);
+
+extern "C" int nangila_psgd_gemm_columns(const void* M, int32_t m, int32_t n, const void* Bt, int32_t transposed, float* out, int32_t columns,
+                                         uint32_t* status, uint64_t timeout_ns, cudaStream_t stream) {
+  if (columns < 1 || columns > 16) return int(cudaErrorInvalidValue);
+  return launch_gemm(M, m, n, Bt, transposed, out, columns, nullptr, status, timeout_ns, stream);
+}
+
 extern "C" int nangila_psgd_gemm_push(const void* M, int32_t m, int32_t n, const void* Bt, int32_t transposed, float* out,
                                       const NangilaPsgdPush* push_in, uint32_t* status, uint64_t timeout_ns,
                                       cudaStream_t stream) {
+  return launch_gemm(M, m, n, Bt, transposed, out, push_in != nullptr ? push_in->rank : 16, push_in, status, timeout_ns, stream);
+}
+
+static int launch_gemm(const void* M, int32_t m, int32_t n, const void* Bt, int32_t transposed, float* out, int32_t columns,
+                       const NangilaPsgdPush* push_in, uint32_t* status, uint64_t timeout_ns, cudaStream_t stream) {
   using namespace nangila;
   NangilaPsgdPush push;
   std::memset(&push, 0, sizeof push);
@@ -615,27 +658,15 @@ extern "C" int nangila_psgd_gemm_push(const void* M, int32_t m, int32_t n, const
   int k_per_split = (k_total + splits - 1) / splits;
   k_per_split = (k_per_split + kSlabK - 1) / kSlabK * kSlabK;
   const int nsplit = (k_total + k_per_split - 1) / k_per_split;
-  dim3 grid{unsigned(tiles), unsigned(nsplit), 1u}, block{unsigned(kGemmThreads), 1u, 1u};
-  cudaError_t e;
-  if (transposed) {
-    static bool attr1 = false;
-    if (!attr1) {
-      cudaFuncSetAttribute(psgd_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
-      attr1 = true;
-    }
-    psgd_gemm_kernel<true><<<grid, block, kGemmSmem, stream>>>(tmA, tmB, out, rows, k_total, k_per_split, nsplit > 1, status,
-                                                              timeout_ns, push);
-  } else {
-    static bool attr0 = false;
-    if (!attr0) {
-      cudaFuncSetAttribute(psgd_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
-      attr0 = true;
-    }
-    psgd_gemm_kernel<false><<<grid, block, kGemmSmem, stream>>>(tmA, tmB, out, rows, k_total, k_per_split, nsplit > 1, status,
-                                                               timeout_ns, push);
+  const dim3 grid{unsigned(tiles), unsigned(nsplit), 1u};
+  auto* kernel = transposed ? psgd_gemm_kernel<true> : psgd_gemm_kernel<false>;
+  static bool opted_in[2] = {false, false};  // shared memory above the default limit
+  if (!opted_in[transposed ? 1 : 0]) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
+    opted_in[transposed ? 1 : 0] = true;
   }
-  e = cudaGetLastError();
-  return int(e);
+  return int(launch_following(kernel, grid, kGemmThreads, kGemmSmem, stream, tmA, tmB, out, rows, k_total, k_per_split, int(nsplit > 1),
+                              int(columns), status, timeout_ns, push));
 }
 
 extern "C" int nangila_psgd_prep(const void* grad, int32_t dtype, const void* ef, void* mef, int64_t numel, float* z0,
@@ -664,8 +695,9 @@ extern "C" int nangila_psgd_reconstruct(void* grad, int32_t dtype, void* ef, con
   const unsigned gy = unsigned(std::max<int64_t>(1, std::min<int64_t>(m, (148 * 8 + gx - 1) / gx)));
   const dim3 grid{gx, gy};
   auto* e = static_cast<__nv_bfloat16*>(ef);
+  cudaError_t err = cudaSuccess;
   auto* f = static_cast<const __nv_bfloat16*>(mef);
-#define NANGILA_RECON(T, RQ) psgd_reconstruct_kernel<T, RQ><<<grid, 256, 0, stream>>>(static_cast<T*>(grad), e, f, P, Q, m, n, r)
+#define NANGILA_RECON(T, RQ) err = launch_following(psgd_reconstruct_kernel<T, RQ>, grid, 256, 0, stream, static_cast<T*>(grad), e, f, P, Q, int(m), int(n), int(r))
   switch (dtype) {
     case NANGILA_F32: if (r <= 4) NANGILA_RECON(float, 4); else NANGILA_RECON(float, 0); break;
     case NANGILA_BF16: if (r <= 4) NANGILA_RECON(__nv_bfloat16, 4); else NANGILA_RECON(__nv_bfloat16, 0); break;
@@ -673,7 +705,7 @@ extern "C" int nangila_psgd_reconstruct(void* grad, int32_t dtype, void* ef, con
     default: return int(cudaErrorInvalidValue);
   }
 #undef NANGILA_RECON
-  return int(cudaGetLastError());
+  return int(err);
 }
 
 extern "C" uint64_t nangila_psgd_exchange_region_bytes(int32_t rows, int32_t rank, int32_t world, uint64_t* recv_off,
@@ -708,10 +740,15 @@ extern "C" int nangila_psgd_exchange(const NangilaPsgdExchangeParams* p, cudaStr
   attrs[0].val.clusterDim.z = 1;
   // several emulated ranks in one launch wait for one another: ask for a cooperative launch so that
   // all their clusters are resident together
-  attrs[1].id = cudaLaunchAttributeCooperative;
-  attrs[1].val.cooperative = 1;
+  if (p->nvr > 1) {
+    attrs[1].id = cudaLaunchAttributeCooperative;
+    attrs[1].val.cooperative = 1;
+  } else {
+    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  }
   cfg.attrs = attrs;
-  cfg.numAttrs = p->nvr > 1 ? 2 : 1;
+  cfg.numAttrs = 2;
   const NangilaPsgdExchangeParams params = *p;
   cudaError_t e;
   if (p->rank <= 4)

@@ -149,20 +149,21 @@ class PowerSGDEngine:
         # The GEMMs start the exchange of their result from the epilogue: the CTA that completes a 128-row tile stores
         # it into every rank's slot over NVLink, the one that completes the last tile releases the flags; the exchange
         # kernel then only waits, averages and orthonormalises (NANGILA_PSGD_PUSH=0: it also does the stores).
-        push = self.push_from_gemm
+        # A rank on its own has nobody to exchange with: the exchange kernel reads the factor where the GEMM left it.
+        push = self.push_from_gemm and self.world > 1
         for v in range(self.nvr):
             G.psgd_prep(flat[v], st.ef[v], st.mef[v], st.p_full[v], st.q_full[v])  # also clears accumulators and counters
             G.psgd_gemm(st.mef[v], st.qt[v], False, st.p_local[v], self.status[v], self.timeout_s, False,
                         **(dict(counters=st.p_cnt[v], push_region_ptrs=st.region_p.ptrs, push_recv_off=st.lay_p[0],
                                 push_flag_off=st.lay_p[1], push_me=rank0 + v, push_rank=st.r, push_epoch=st.epoch,
-                                push_epoch_word=epoch_word) if push else {}))
+                                push_epoch_word=epoch_word) if push else dict(push_rank=st.r)))
         G.psgd_exchange(st.p_local, st.p_mean, [s[:m] for s in st.scratch], st.pt, self.status, st.region_p.ptrs,
                         st.lay_p[0], st.lay_p[1], m, st.r, rank0, True, st.epoch, self.timeout_s, epoch_word, push)
         for v in range(self.nvr):
             G.psgd_gemm(st.mef[v], st.pt[v], True, st.q_local[v], self.status[v], self.timeout_s, False,
                         **(dict(counters=st.q_cnt[v], push_region_ptrs=st.region_q.ptrs, push_recv_off=st.lay_q[0],
                                 push_flag_off=st.lay_q[1], push_me=rank0 + v, push_rank=st.r, push_epoch=st.epoch,
-                                push_epoch_word=epoch_word) if push else {}))
+                                push_epoch_word=epoch_word) if push else dict(push_rank=st.r)))
         G.psgd_exchange(st.q_local, st.q_mean, [s[:n] for s in st.scratch], st.qt, self.status, st.region_q.ptrs,
                         st.lay_q[0], st.lay_q[1], n, st.r, rank0, False, st.epoch, self.timeout_s, epoch_word, push)
         for v in range(self.nvr):
@@ -230,7 +231,8 @@ class PowerSGDEngine:
             if not self._branches:
                 self._branches = [torch.cuda.Stream(device=self.device) for _ in range(self.graph_branches)]
             with torch.cuda.graph(graph, stream=self._capture_stream, capture_error_mode="thread_local"):
-                epoch_word.add_(1)
+                if self.world > 1:  # (a rank on its own waits for nothing)
+                    epoch_word.add_(1)
                 # The matrices are independent of one another: each one's chain of six kernels is recorded on one
                 # of a few branch streams, so the graph has that many parallel chains and the small kernels of
                 # different matrices overlap instead of queueing behind one another.
