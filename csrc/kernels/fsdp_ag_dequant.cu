@@ -11,7 +11,7 @@
 // buffer the shard is read from), the meeting of the ranks (meet.cuh), ag_expand (the other ranks' parts). Grids of short CTAs
 // without flags or fences that the hardware hands out as SMs come free.
 // What bounds them: HBM and L2 traffic. Measured on B200, four ranks on one device, 3.1 M bf16 elements each, INT8 (25 MB in, 39 MB of codes, 100 MB
-// out): 17 us (5.2 TB/s) + 21 us (5.5 TB/s), 42.6 us for the call; as one resident kernel with block barriers and a flag per chunk 49.3 us.
+// out): 17 us (5.2 TB/s) + 21 us (5.5 TB/s), 42.4 us for the call; as one resident kernel with block barriers and a flag per chunk 49.3 us.
 // The arithmetic is kept out of the way: with divisions by the chunk size, conversions and clamps (250 instructions per eight elements, now 90; 132 and now 35
 // to expand them) the two took 19 and 45 us.
 //
@@ -57,15 +57,26 @@ using Packed = std::conditional_t<BITS == 8, uint2, uint32_t>;  // eight codes
 
 constexpr int kTile = 4;  // iterations of 2048 elements whose loads are issued together
 
-// A rank's shard in the exchange region: its codes one behind the other, then its scales.
-struct AgSlot {
-  uint64_t codes, scales;  // offsets of lane `tid` of iteration `it`; the next iterations follow kThreads lanes, kPerIter / 64 scales further
-  __device__ __forceinline__ AgSlot(const NangilaAgParams& p, int bits, int owner, int it, int tid) {
+// A rank's shard in the exchange region: its codes one behind the other, then its scales. Worked out on the host: the number of chunks is a
+// division of 64-bit numbers, which costs a thread more than quantizing eight elements.
+struct AgShape {
+  uint64_t base, per_owner, to_scales;
+  AgShape(const NangilaAgParams& p, int bits) {
     const int C = p.chunk_elems;
-    const uint64_t cps = uint64_t((p.shard_elems + C - 1) / C), bytes = cps * ag_slot_bytes(C, bits);
-    const uint64_t base = p.recv_off + (uint64_t(p.epoch & 1u) * p.world + owner) * bytes;
-    codes = base + (uint64_t(it) * kPerIter + tid * kE) * bits / 8;
-    scales = base + cps * C * bits / 8 + (uint64_t(it) * (kPerIter / kQuantBlock) + tid / 8) * 2;
+    const uint64_t cps = uint64_t((p.shard_elems + C - 1) / C);
+    per_owner = cps * ag_slot_bytes(C, bits);
+    base = p.recv_off + uint64_t(p.epoch & 1u) * uint64_t(p.world) * per_owner;
+    to_scales = cps * uint64_t(C) * uint64_t(bits) / 8;
+  }
+};
+// Offsets of lane `tid` of iteration `it`; the next iterations follow kThreads lanes, kPerIter / 64 scales further.
+template <int BITS>
+struct AgSlot {
+  uint64_t codes, scales;
+  __device__ __forceinline__ AgSlot(const AgShape& sh, int owner, int it, int tid) {
+    const uint64_t own = sh.base + uint64_t(owner) * sh.per_owner;
+    codes = own + (uint64_t(it) * kPerIter + tid * kE) * BITS / 8;
+    scales = own + sh.to_scales + (uint64_t(it) * (kPerIter / kQuantBlock) + tid / 8) * 2;
   }
 };
 
@@ -102,7 +113,7 @@ __device__ __forceinline__ void expand8(const Packed<BITS>& w, uint16_t scale, T
 }
 
 template <typename T, int BITS>
-__global__ void __launch_bounds__(kThreads, 5) ag_quantize_kernel(const __grid_constant__ NangilaAgParams p) {
+__global__ void __launch_bounds__(kThreads, 5) ag_quantize_kernel(const __grid_constant__ NangilaAgParams p, const __grid_constant__ AgShape sh) {
   may_follow();
   const int vr = blockIdx.y, me = p.rank0 + vr, W = p.world, tid = threadIdx.x;
   const int total = int((p.shard_elems + kPerIter - 1) / kPerIter);
@@ -161,7 +172,7 @@ __global__ void __launch_bounds__(kThreads, 5) ag_quantize_kernel(const __grid_c
         w[b] = __byte_perm(a | (a >> 4), c | (c >> 4), 0x6420);
       }
     }
-    const AgSlot slot(p, BITS, me, it0, tid);
+    const AgSlot<BITS> slot(sh, me, it0, tid);
     for (int d = 1, r = me + 1; d < W; ++d, ++r) {
       if (r == W) r = 0;
       Packed<BITS>* codes = reinterpret_cast<Packed<BITS>*>(p.region[r] + slot.codes);
@@ -182,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, 5) ag_quantize_kernel(const __grid_c
 }
 
 template <typename T, int BITS>
-__global__ void __launch_bounds__(kThreads, 8) ag_expand_kernel(const __grid_constant__ NangilaAgParams p, int tiles) {
+__global__ void __launch_bounds__(kThreads, 8) ag_expand_kernel(const __grid_constant__ NangilaAgParams p, const __grid_constant__ AgShape sh, int tiles) {
   const int vr = blockIdx.z, me = p.rank0 + vr, W = p.world, tid = threadIdx.x;
   int o = me + 1 + int(blockIdx.y);  // the other ranks' shards
   if (o >= W) o -= W;
@@ -192,7 +203,7 @@ __global__ void __launch_bounds__(kThreads, 8) ag_expand_kernel(const __grid_con
   T* __restrict__ out = static_cast<T*>(p.out_full[vr]) + int64_t(o) * p.shard_elems;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t at0 = int64_t(tile) * (kTile * kPerIter) + tid * kE, left = p.shard_elems - at0;
-    const AgSlot slot(p, BITS, o, tile * kTile, tid);
+    const AgSlot<BITS> slot(sh, o, tile * kTile, tid);
     const Packed<BITS>* codes = reinterpret_cast<const Packed<BITS>*>(myreg + slot.codes);
     const uint16_t* scales = reinterpret_cast<const uint16_t*>(myreg + slot.scales);
     Packed<BITS> w[kTile];
@@ -215,15 +226,16 @@ template <typename T, int BITS>
 cudaError_t launch(const NangilaAgParams& p, cudaStream_t stream) {
   const int64_t total = (p.shard_elems + kPerIter - 1) / kPerIter, tiles = (total + kTile - 1) / kTile;
   if (total > 0x3fffffff) return cudaErrorInvalidValue;
+  const AgShape sh(p, BITS);
   // fewer CTAs asked for than chunks to quantize and to expand: a cap
   const int64_t cps = (p.shard_elems + p.chunk_elems - 1) / p.chunk_elems;
   const int64_t cap = p.grid_x > 0 && p.grid_x < cps * (p.world + 1) ? p.grid_x : 0x7fffffff;
-  ag_quantize_kernel<T, BITS><<<dim3(unsigned(std::min(cap, tiles)), unsigned(p.nvr)), kThreads, 0, stream>>>(p);
+  ag_quantize_kernel<T, BITS><<<dim3(unsigned(std::min(cap, tiles)), unsigned(p.nvr)), kThreads, 0, stream>>>(p, sh);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || p.world == 1) return e;
   if ((e = launch_meet(p, p.flag_off, kTimeoutPhase3, 3u, stream)) != cudaSuccess) return e;
   const dim3 grid(unsigned(std::min(std::max<int64_t>(1, cap / (p.world - 1)), tiles)), unsigned(p.world - 1), unsigned(p.nvr));
-  return launch_following(ag_expand_kernel<T, BITS>, grid, kThreads, 0, stream, p, int(tiles));
+  return launch_following(ag_expand_kernel<T, BITS>, grid, kThreads, 0, stream, p, sh, int(tiles));
 }
 
 }  // namespace

@@ -11,7 +11,7 @@
 // between needs that peer's word.
 //
 // What bounds it: rs_quantize the issue rate, about as much as HBM (the gradient in), rs_sum latency (its input lies in L2). Measured on B200, four ranks on one
-// device, 12.6 M bf16 elements each: 28 us (100 MB in, 27 MB of codes out: 4.5 TB/s) + 13 us, 45 us for the call; before, one resident kernel that walked a
+// device, 12.6 M bf16 elements each: 26 us (100 MB in, 27 MB of codes out: 4.8 TB/s) + 12 us, 43 us for the call; before, one resident kernel that walked a
 // task per chunk with a ring of bulk copies, a fence and a flag each: 99 us. Tiles of four iterations: their loads are issued together,
 // and the index arithmetic is paid once.
 //
@@ -38,12 +38,14 @@ using namespace comm;
 // Iterations of 2048 elements a CTA takes; their loads are issued together.
 constexpr int kTile = 4;
 
+// What follows from the parameters, worked out once on the host: two of them are divisions of 64-bit numbers, which cost a thread more than
+// quantizing eight elements (the call above: 45.2 us with them in every CTA).
 struct RsShape {
-  int W, C, iters, cps, sub;
+  int W, C, iters, cps, sub, tiles;  // sub: tiles of a chunk; tiles: of a shard
   int64_t shard;
   uint64_t slot, recv;
-  __device__ __forceinline__ explicit RsShape(const NangilaPredResParams& p)
-      : W(p.world), C(p.chunk_elems), iters(C / kElemsPerIter), cps(p.nchunks / p.world), sub((iters + kTile - 1) / kTile),
+  explicit RsShape(const NangilaPredResParams& p)
+      : W(p.world), C(p.chunk_elems), iters(C / kElemsPerIter), cps(p.nchunks / p.world), sub((iters + kTile - 1) / kTile), tiles(cps * sub),
         shard(p.n / p.world), slot(compressed_slot_bytes(C)), recv(p.recv1_off + uint64_t(p.epoch & 1u) * uint64_t(cps) * W * slot) {}
 };
 
@@ -53,9 +55,8 @@ constexpr bool kPackedBf16 = std::is_same_v<T, __nv_bfloat16> && std::is_same_v<
 
 // LOOP: the launch has fewer CTAs than tiles. (The loop's invariants cost registers; without it 64 are enough for four CTAs an SM.)
 template <typename T, typename S, bool EF, bool LOOP>
-__global__ void __launch_bounds__(kThreads, LOOP ? 2 : kPackedBf16<T, S> && !EF ? 6 : 4) rs_quantize_kernel(const __grid_constant__ NangilaPredResParams p, int tiles) {
+__global__ void __launch_bounds__(kThreads, LOOP ? 2 : kPackedBf16<T, S> && !EF ? 6 : 4) rs_quantize_kernel(const __grid_constant__ NangilaPredResParams p, const __grid_constant__ RsShape sh) {
   may_follow();
-  const RsShape sh(p);
   const int vr = blockIdx.z, me = p.rank0 + vr, W = sh.W, C = sh.C, tid = threadIdx.x;
   int o = me + 1 + int(blockIdx.y);  // remote owners first, this rank's own shard last
   if (o >= W) o -= W;
@@ -145,18 +146,17 @@ __global__ void __launch_bounds__(kThreads, LOOP ? 2 : kPackedBf16<T, S> && !EF 
       fp32_tile(std::false_type{});
     }
     tile += gridDim.x;
-  } while (LOOP && tile < tiles);
+  } while (LOOP && tile < sh.tiles);
 }
 
 template <typename T, bool PACKED>
-__global__ void __launch_bounds__(kThreads, 4) rs_sum_kernel(const __grid_constant__ NangilaPredResParams p, int tiles) {
-  const RsShape sh(p);
+__global__ void __launch_bounds__(kThreads, 4) rs_sum_kernel(const __grid_constant__ NangilaPredResParams p, const __grid_constant__ RsShape sh) {
   const int vr = blockIdx.y, me = p.rank0 + vr, W = sh.W, C = sh.C, tid = threadIdx.x;
   uint8_t* myreg = p.region[me];
   follow();
   if (*reinterpret_cast<volatile uint32_t*>(&p.status[vr][kStatusCode]) != 0u) return;  // a rank's data did not come
   T* __restrict__ out = static_cast<T*>(p.out_shard[vr]);
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+  for (int tile = blockIdx.x; tile < sh.tiles; tile += gridDim.x) {
     const int j = int(unsigned(tile) / unsigned(sh.sub)), it0 = (tile - j * sh.sub) * kTile;
     uint8_t* src = myreg + sh.recv + uint64_t(j) * W * sh.slot;
     const uint32_t* codes = packed_ptr(src, C, it0, tid);
@@ -217,32 +217,32 @@ __global__ void __launch_bounds__(kThreads, 4) rs_sum_kernel(const __grid_consta
 }
 
 template <typename T, typename S, bool EF>
-void launch_quantize(const NangilaPredResParams& p, dim3 grid, int tiles, cudaStream_t stream) {
-  if (grid.x < unsigned(tiles)) rs_quantize_kernel<T, S, EF, true><<<grid, kThreads, 0, stream>>>(p, tiles);
-  else rs_quantize_kernel<T, S, EF, false><<<grid, kThreads, 0, stream>>>(p, tiles);
+void launch_quantize(const NangilaPredResParams& p, const RsShape& sh, dim3 grid, cudaStream_t stream) {
+  if (grid.x < unsigned(sh.tiles)) rs_quantize_kernel<T, S, EF, true><<<grid, kThreads, 0, stream>>>(p, sh);
+  else rs_quantize_kernel<T, S, EF, false><<<grid, kThreads, 0, stream>>>(p, sh);
 }
 
 template <typename T, typename S>
 cudaError_t launch(const NangilaPredResParams& p, cudaStream_t stream) {
   const int64_t sub = (p.chunk_elems / kElemsPerIter + kTile - 1) / kTile, all = p.nchunks / p.world * sub;
   if (all > 0x3fffffff) return cudaErrorInvalidValue;
-  const int tiles = int(all);  // of one shard
+  const RsShape sh(p);
   // fewer CTAs than chunks asked for: a cap for all destinations together
   const int cap = p.grid_x > 0 && p.grid_x < p.nchunks ? p.grid_x : 0;
   const int phases = (p.phase_mask & 7) == 0 ? 7 : p.phase_mask;
   if (phases & 1) {
     bool ef = false;
     for (int v = 0; v < p.nvr; ++v) ef = ef || p.ef[v] != nullptr;
-    const dim3 grid(unsigned(cap > 0 ? std::min(tiles, std::max(1, cap / p.world)) : tiles), unsigned(p.world), unsigned(p.nvr));
-    if (ef) launch_quantize<T, S, true>(p, grid, tiles, stream);
-    else launch_quantize<T, S, false>(p, grid, tiles, stream);
+    const dim3 grid(unsigned(cap > 0 ? std::min(sh.tiles, std::max(1, cap / p.world)) : sh.tiles), unsigned(p.world), unsigned(p.nvr));
+    if (ef) launch_quantize<T, S, true>(p, sh, grid, stream);
+    else launch_quantize<T, S, false>(p, sh, grid, stream);
   }
   if (phases & 2) {
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = launch_meet(p, p.flag1_off, kTimeoutPhase2, 2u, stream);
     if (e != cudaSuccess) return e;
-    const dim3 grid(unsigned(cap > 0 ? std::min(tiles, cap) : tiles), unsigned(p.nvr));
-    return launch_following(rs_sum_kernel<T, kPackedBf16<T, S>>, grid, kThreads, 0, stream, p, tiles);
+    const dim3 grid(unsigned(cap > 0 ? std::min(sh.tiles, cap) : sh.tiles), unsigned(p.nvr));
+    return launch_following(rs_sum_kernel<T, kPackedBf16<T, S>>, grid, kThreads, 0, stream, p, sh);
   }
   return cudaGetLastError();
 }
