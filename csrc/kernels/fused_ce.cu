@@ -16,6 +16,9 @@
 namespace {
 
 constexpr int kT = 256;
+// Loads of a thread that the forward pass has on their way. It is bound by HBM (824 MB of GPT-2 logits, 8192 rows: 139 us with one, 134 with four, 6.2 TB/s);
+// one exponential an element is not far behind.
+constexpr int kAhead = 4;
 
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
     const uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -41,9 +44,9 @@ __global__ void __launch_bounds__(kT) ce_forward_kernel(const __nv_bfloat16* __r
     const int tid = threadIdx.x;
     const int v8 = v & ~7;
     float m = -INFINITY, s = 0.0f;
-    for (int i = tid * 8; i < v8; i += kT * 8) {
+    auto add8 = [&](const uint4& u) {
         float f[8];
-        unpack8(__ldg(reinterpret_cast<const uint4*>(p + i)), f);
+        unpack8(u, f);
         float mx = f[0];
 #pragma unroll
         for (int k = 1; k < 8; ++k) mx = fmaxf(mx, f[k]);
@@ -53,7 +56,16 @@ __global__ void __launch_bounds__(kT) ce_forward_kernel(const __nv_bfloat16* __r
         for (int k = 0; k < 8; ++k) acc += __expf(f[k] - mn);
         s = s * __expf(m - mn) + acc;  // exp(-inf) = 0 on the first pass
         m = mn;
+    };
+    int i = tid * 8;
+    for (; i + (kAhead - 1) * kT * 8 < v8; i += kAhead * kT * 8) {
+        uint4 u[kAhead];
+#pragma unroll
+        for (int a = 0; a < kAhead; ++a) u[a] = __ldg(reinterpret_cast<const uint4*>(p + i + a * kT * 8));
+#pragma unroll
+        for (int a = 0; a < kAhead; ++a) add8(u[a]);
     }
+    for (; i < v8; i += kT * 8) add8(__ldg(reinterpret_cast<const uint4*>(p + i)));
     if (tid < v - v8) {
         const float x = __bfloat162float(p[v8 + tid]);
         merge(m, s, x, 1.0f);
