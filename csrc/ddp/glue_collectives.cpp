@@ -1,6 +1,7 @@
 // Bindings of the kernels other than the prediction-residual bucket exchange; kept in its own
 // translation unit so the glue compiles in parallel.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
@@ -145,9 +146,11 @@ at::Tensor packet_compress(const at::Tensor& grad, const c10::optional<at::Tenso
                                        sums.data_ptr<float>(), at::cuda::getCurrentCUDAStream()), "packet_compress");
   return packet;
 }
-// What the host has to know of a packet before it decodes it: the first (up to) 44 bytes and, if asked for, the CRC32 of everything
-// behind the header. One synchronisation for both.
-py::tuple packet_inspect(const at::Tensor& packet, bool checksum) {
+// What the host has to know of a packet: the first (up to) 44 bytes and, if asked for, the CRC32 of everything behind the header. One
+// synchronisation for both. With `out` the decoder is queued behind them, so that the device need not wait for the host's verdict; it
+// checks the header itself. The last part of the answer says whether it was queued.
+py::tuple packet_inspect(const at::Tensor& packet, bool checksum, int64_t layer, const c10::optional<at::Tensor>& curr,
+                         const c10::optional<at::Tensor>& prev, double mu, const c10::optional<at::Tensor>& out) {
   TORCH_CHECK(packet.is_cuda() && packet.scalar_type() == at::kByte && packet.is_contiguous() && packet.numel() > 32,
               "nangila: packet_inspect wants a contiguous uint8 CUDA packet");
   const int64_t fixed = std::min<int64_t>(packet.numel(), 44);
@@ -156,22 +159,32 @@ py::tuple packet_inspect(const at::Tensor& packet, bool checksum) {
   auto host = at::empty({48}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
   uint8_t* h = host.data_ptr<uint8_t>();
   at::Tensor word;
+  uint32_t* w = nullptr;
   if (checksum) {
     word = at::empty({1}, packet.options().dtype(at::kInt));
-    auto* w = reinterpret_cast<uint32_t*>(word.data_ptr<int32_t>());
+    w = reinterpret_cast<uint32_t*>(word.data_ptr<int32_t>());
     check_launch(nangila_crc32(packet.data_ptr<uint8_t>() + 32, packet.numel() - 32, w, w, stream), "crc32");
-    check_launch(int(cudaMemcpyAsync(h + 44, w, 4, cudaMemcpyDeviceToHost, stream)), "packet_inspect");
   }
-  check_launch(int(cudaMemcpyAsync(h, packet.data_ptr<uint8_t>(), size_t(fixed), cudaMemcpyDeviceToHost, stream)), "packet_inspect");
-  cudaError_t e;
+  check_launch(nangila_packet_report(packet.data_ptr<uint8_t>(), int32_t(fixed), w, h, stream), "packet_inspect");
+  at::cuda::CUDAEvent reported;
+  reported.record(stream);
+  bool queued = false;
+  if (out.has_value() && layer >= 0 && layer <= 0xffffffffll) {
+    const int64_t n = out->numel();
+    TORCH_CHECK(out->is_cuda() && out->scalar_type() == at::kFloat && out->is_contiguous(), "nangila: out must be FP32 CUDA");
+    const float* c = curr.has_value() ? curr->data_ptr<float>() : nullptr;
+    const float* p = prev.has_value() ? prev->data_ptr<float>() : nullptr;
+    if (c) TORCH_CHECK(curr->numel() == n && prev.has_value() && prev->numel() == n, "nangila: history size mismatch");
+    // (refused: too short or misaligned for what is expected; the host will say what is wrong with it)
+    queued = nangila_packet_decode_expected(packet.data_ptr<uint8_t>(), packet.numel(), uint32_t(layer), c, p, float(mu), n, out->data_ptr<float>(), stream) == 0;
+  }
   {
     py::gil_scoped_release release;
-    e = cudaStreamSynchronize(stream);
+    reported.synchronize();
   }
-  check_launch(int(e), "packet_inspect");
   uint32_t crc = 0;
   if (checksum) std::memcpy(&crc, h + 44, 4);
-  return py::make_tuple(py::bytes(reinterpret_cast<const char*>(h), size_t(fixed)), crc);
+  return py::make_tuple(py::bytes(reinterpret_cast<const char*>(h), size_t(fixed)), crc, queued);
 }
 void packet_decode(const at::Tensor& payload, int64_t ndim, const c10::optional<at::Tensor>& curr,
                    const c10::optional<at::Tensor>& prev, double mu, double gain, at::Tensor out) {
@@ -493,7 +506,8 @@ void register_more(py::module_& m) {
         py::arg("gain"), py::arg("payload"));
   m.def("packet_compress", &packet_compress, py::arg("grad"), py::arg("curr"), py::arg("prev"), py::arg("ef"), py::arg("mu"),
         py::arg("gain"), py::arg("header"));
-  m.def("packet_inspect", &packet_inspect, py::arg("packet"), py::arg("checksum"));
+  m.def("packet_inspect", &packet_inspect, py::arg("packet"), py::arg("checksum"), py::arg("layer") = -1, py::arg("curr") = py::none(),
+        py::arg("prev") = py::none(), py::arg("mu") = 0.0, py::arg("out") = py::none());
   m.def("packet_decode", &packet_decode, py::arg("payload"), py::arg("ndim"), py::arg("curr"), py::arg("prev"), py::arg("mu"),
         py::arg("gain"), py::arg("out"));
   m.def("dgc_region_layout", &dgc_region_layout);

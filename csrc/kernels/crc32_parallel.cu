@@ -170,7 +170,8 @@ uint32_t x_pow_bytes(uint64_t n) {
   return r;
 }
 
-cudaError_t launch_crc(const void* data, int64_t nbytes, uint32_t* out, cudaStream_t stream) {
+// cleared: *out is zero when the kernel starts.
+cudaError_t launch_crc(const void* data, int64_t nbytes, uint32_t* out, bool cleared, cudaStream_t stream) {
   CrcArgs a;
   a.data = static_cast<const uint8_t*>(data);
   a.head = int64_t((16u - (reinterpret_cast<uintptr_t>(data) & 15u)) & 15u);
@@ -187,7 +188,7 @@ cudaError_t launch_crc(const void* data, int64_t nbytes, uint32_t* out, cudaStre
   a.tail_factor = x_pow_bytes(uint64_t(a.tail));
   a.fixed = mulmod(0xFFFFFFFFu, x_pow_bytes(uint64_t(nbytes))) ^ 0xFFFFFFFFu;
   a.out = out;
-  if (ctas > 1) {
+  if (ctas > 1 && !cleared) {
     const cudaError_t e = cudaMemsetAsync(out, 0, 4, stream);
     if (e != cudaSuccess) return e;
   }
@@ -207,7 +208,13 @@ extern "C" int nangila_crc32(const void* data, int64_t nbytes, uint32_t* scratch
   if (out == nullptr || nbytes < 0 || (nbytes > 0 && (data == nullptr || scratch == nullptr)))
     return int(cudaErrorInvalidValue);
   if (nbytes == 0) return int(cudaMemsetAsync(out, 0, 4, stream));
-  return int(nangila::launch_crc(data, nbytes, out, stream));
+  return int(nangila::launch_crc(data, nbytes, out, false, stream));
+}
+
+// The same with *out known to be zero: one launch instead of a memset and a launch where several CTAs add to it.
+extern "C" int nangila_crc32_cleared(const void* data, int64_t nbytes, uint32_t* out, cudaStream_t stream) {
+  if (out == nullptr || nbytes <= 0 || data == nullptr) return int(cudaErrorInvalidValue);
+  return int(nangila::launch_crc(data, nbytes, out, true, stream));
 }
 
 // Allocation-free entry point (declared in nangila_noalloc.h; the reference has nothing like it).
@@ -217,5 +224,5 @@ extern "C" int nangila_crc32_noalloc(const void* data, int64_t nbytes, uint32_t*
   if (out == nullptr || nbytes < 0 || (nbytes > 0 && data == nullptr)) return int(cudaErrorInvalidValue);
   if (nbytes > nangila_crc32_noalloc_max_bytes()) return int(cudaErrorInvalidValue);
   if (nbytes == 0) return int(cudaMemsetAsync(out, 0, 4, stream));
-  return int(nangila::launch_crc(data, nbytes, out, stream));
+  return int(nangila::launch_crc(data, nbytes, out, false, stream));
 }

@@ -217,6 +217,7 @@ int nangila_state_hash(const void* data, int64_t nbytes, uint64_t seed, uint64_t
 /* `scratch` of nangila_crc32 is no longer written (the result word is all the kernel needs); it must still not be NULL. */
 int64_t nangila_crc32_scratch_words(int64_t nbytes);
 int nangila_crc32(const void* data, int64_t nbytes, uint32_t* scratch, uint32_t* out, cudaStream_t stream);
+int nangila_crc32_cleared(const void* data, int64_t nbytes, uint32_t* out, cudaStream_t stream); /* *out is zero, nbytes above 0 */
 uint32_t nangila_absmax_scratch_words(void);
 int nangila_absmax_hist(const void* x, int32_t dtype, int64_t n, uint32_t k, float qmax, uint32_t* scratch, float* out,
                         uint32_t* hist256, cudaStream_t stream);
@@ -246,6 +247,12 @@ int nangila_packet_compress(const void* grad, int32_t dtype, const float* curr, 
  * payload's dimension count (its third word), which fixes where the gain, scales and nibbles start. */
 int nangila_packet_decode(const uint8_t* payload, int64_t payload_bytes, int32_t ndim, const float* curr, const float* prev,
                           float mu, float gain, int64_t n, float* out, cudaStream_t stream);
+/* The decoder for a packet whose header the host has not seen yet: runs if it is a driver's one-dimensional packet of layer `layer` with n elements in blocks
+ * of 64 (and not one without a prediction, if curr is given), and leaves `out` alone otherwise. */
+int nangila_packet_decode_expected(const uint8_t* packet, int64_t packet_bytes, uint32_t layer, const float* curr, const float* prev, float mu,
+                                   int64_t n, float* out, cudaStream_t stream);
+/* The first `bytes` (at most 44) of a packet and, at byte 44, *crc (unless NULL) into 48 bytes of pinned HOST memory. */
+int nangila_packet_report(const uint8_t* packet, int32_t bytes, const uint32_t* crc, uint8_t* host, cudaStream_t stream);
 /* runtime helpers for callers that bind this library without linking the CUDA runtime themselves */
 int nangila_copy_to_host(void* dst, const void* src, int64_t nbytes, cudaStream_t stream);   /* copies, then synchronises */
 int nangila_copy_to_device(void* dst, const void* src, int64_t nbytes, cudaStream_t stream); /* asynchronous */

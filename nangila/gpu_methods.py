@@ -17,7 +17,7 @@ The history (two FP32 tensors per layer) and the error memory live on the device
 object; the host-side state machine supplies step numbers, warm-up and momentum. Nothing synchronises
 unless ``sync_mode`` says so: 0 (ASYNC) never, 1 (ALWAYS) after every call, 2 (PERIODIC) every 100th call.
 ``decompress_gpu`` reads the 44 fixed bytes of the packet on the host (one synchronisation, which brings the checksum of
-the payload with it unless ``sync_mode`` is 0) and validates them before anything is decoded.
+the payload with it unless ``sync_mode`` is 0) and validates them before anything decoded is handed out.
 """
 from __future__ import annotations
 
@@ -121,8 +121,19 @@ def decompress_gpu(self: NangilaHook, layer_id: int, compressed: torch.Tensor, o
     if packet.numel() < _HEADER + 8:
         raise RuntimeError(f"decompress_gpu: packet of {packet.numel()} bytes is too small")
     dev = packet.device
+    n = int(output_size)
+    # A layer that is known is decoded while the host still looks at the packet; the kernel checks the header by itself, and what it
+    # has written is handed out only if the host finds nothing wrong.
+    known = _state(self)["layers"].get(layer_id)
+    out, predicted = None, False
     with torch.cuda.device(dev):
-        fixed, got = _glue().packet_inspect(packet, sync_mode != 0)
+        if known is not None and known.n == n and known.curr.device == dev:
+            out = torch.empty(n, dtype=torch.float32, device=dev)
+            predicted = known.updates >= 2
+            fixed, got, queued = _glue().packet_inspect(packet, sync_mode != 0, layer_id, known.curr if predicted else None,
+                                                        known.prev if predicted else None, float(self.momentum()), out)
+        else:
+            fixed, got, queued = _glue().packet_inspect(packet, sync_mode != 0)
     magic, version, flags, _step, layer, crc, _hash, _s, _e = struct.unpack("<HBBIIIQII", fixed[:_HEADER])
     if magic != _MAGIC or version != _VERSION:
         raise RuntimeError("decompress_gpu: not a nangila packet (bad magic or version)")
@@ -132,7 +143,8 @@ def decompress_gpu(self: NangilaHook, layer_id: int, compressed: torch.Tensor, o
         glue = _glue()
         if sync_mode != 0 and got != crc:
             raise RuntimeError(f"decompress_gpu: checksum mismatch on layer {layer_id} ({got:#x} != {crc:#x})")
-        out = torch.empty(int(output_size), dtype=torch.float32, device=dev)
+        if out is None:
+            out = torch.empty(n, dtype=torch.float32, device=dev)
         if not flags & _FLAG_DRIVER:
             # raw tensor payload: u32 numel, u32 ndim, u32 dims[ndim], f32 data
             numel, ndim = struct.unpack("<II", fixed[_HEADER:_HEADER + 8])
@@ -154,8 +166,9 @@ def decompress_gpu(self: NangilaHook, layer_id: int, compressed: torch.Tensor, o
                 raise RuntimeError(f"decompress_gpu: packet holds {numel} elements, expected {output_size}")
             ls = _layer(self, layer_id, numel, dev)
             use_pred = not (flags & _FLAG_NO_PREDICTION) and ls.updates >= 2
-            glue.packet_decode(packet[_HEADER:], int(ndim), ls.curr if use_pred else None, ls.prev if use_pred else None,
-                               float(self.momentum()), -1.0 if use_pred else 0.0, out)
+            if not (queued and ndim == 1 and use_pred == predicted):  # else the decoder has seen what it expected
+                glue.packet_decode(packet[_HEADER:], int(ndim), ls.curr if use_pred else None, ls.prev if use_pred else None,
+                                   float(self.momentum()), -1.0 if use_pred else 0.0, out)
     _maybe_sync(self, sync_mode)
     return out
 
