@@ -30,9 +30,11 @@ constexpr int kMeetThreads = NANGILA_MAX_RANKS * NANGILA_MAX_VRANKS;
 static __global__ void __launch_bounds__(kMeetThreads) meet_kernel(const __grid_constant__ MeetArgs a) {
   follow();
   const int v = int(threadIdx.x) / a.world, r = int(threadIdx.x) % a.world;
-  if (v < a.nvr) st_release_sys(reinterpret_cast<uint32_t*>(a.region[r] + a.flag_off) + a.rank0 + v, a.epoch);
+  // a rank that has failed before has stored nothing: its word stays away, and the others' waits for it run out
+  const bool sound = v < a.nvr && *reinterpret_cast<volatile uint32_t*>(&a.status[v][kStatusCode]) == 0u;
+  if (sound) st_release_sys(reinterpret_cast<uint32_t*>(a.region[r] + a.flag_off) + a.rank0 + v, a.epoch);
   __syncthreads();
-  if (v < a.nvr && *reinterpret_cast<volatile uint32_t*>(&a.status[v][kStatusCode]) == 0u)
+  if (sound)
     wait_flag(reinterpret_cast<const uint32_t*>(a.region[a.rank0 + v] + a.flag_off) + r, a.epoch, a.timeout_ns, a.status[v], a.code,
               uint32_t(a.rank0 + v), uint32_t(r), a.phase, 0u);
 }

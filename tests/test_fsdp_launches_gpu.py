@@ -135,3 +135,28 @@ def test_a_rank_that_does_not_come(what):
     assert (out[0][-4096:] == 3.0).all()  # nothing was made of data that did not come
     assert torch.ones(4, device=DEV).sum().item() == 4.0
     assert int(obj._status[0][0].item()) == 0  # cleared by the check
+
+
+@pytest.mark.parametrize("what", ["reduce_scatter", "all_gather"])
+def test_a_rank_that_has_failed_before_is_missed(what):
+    """A status that nobody has looked at: the rank sends nothing more, and the others find out instead of taking what lies in its slots."""
+    from nangila.parallel import fsdp_collectives as F
+
+    x = [torch.randn(8192, device=DEV) for _ in range(2)]
+    obj = (F.NangilaAllGather if what == "all_gather" else F.NangilaReduceScatter)(arena=_loopback(2), timeout_s=0.2)
+    size = 2 * 8192 if what == "all_gather" else 4096
+    outs = [torch.zeros(size, device=DEV) for _ in range(2)]
+    call = (lambda: obj.gather(outs, x)) if what == "all_gather" else (lambda: obj.reduce(outs, x, 0.5))
+    call()
+    obj.check_status()
+    obj._status[1][0] = 3
+    for o in outs:
+        o.fill_(3.0)
+    call()
+    with pytest.raises(RuntimeError, match="waiting for rank 1"):
+        obj.check_status()
+    assert (outs[0][-4096:] == 3.0).all()
+    obj._status[1].zero_()
+    call()
+    obj.check_status()
+    assert not (outs[0] == 3.0).any()
