@@ -243,6 +243,9 @@ int nangila_packet_encode(const void* grad, int32_t dtype, const float* curr, co
  * aligned) holds 32 + nangila_packet_payload_bytes(n) bytes, `sums` (device) two floats of scratch. */
 int nangila_packet_compress(const void* grad, int32_t dtype, const float* curr, const float* prev, float* ef, float mu, float gain, int64_t n,
                             const uint8_t* header, uint8_t* packet, float* sums, cudaStream_t stream);
+/* The same with room for the inner products in 64 bits. */
+int nangila_packet_compress_f64(const void* grad, int32_t dtype, const float* curr, const float* prev, float* ef, float mu, float gain, int64_t n,
+                                const uint8_t* header, uint8_t* packet, double* sums, cudaStream_t stream);
 /* decode: out = q scale + kappa (curr + mu (curr - prev)); gain < 0 takes kappa from the payload. `ndim` is the
  * payload's dimension count (its third word), which fixes where the gain, scales and nibbles start. */
 int nangila_packet_decode(const uint8_t* payload, int64_t payload_bytes, int32_t ndim, const float* curr, const float* prev,

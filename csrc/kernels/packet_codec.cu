@@ -84,10 +84,11 @@ __device__ __forceinline__ void store8_f32(float* p, int64_t base, int64_t n, co
 }
 
 // sums[0] += <g + ef, g_hat>, sums[1] += <g_hat, g_hat>
-template <typename T>
+// The CTAs' parts meet in 64 bits where the caller has room for that (Sum): a thousand of them added in FP32, in any order, moved the gain by 1e-7 to 1e-6.
+template <typename T, typename Sum>
 __global__ void __launch_bounds__(kThreads) packet_gain_kernel(const T* __restrict__ grad, const float* __restrict__ curr,
                                                                const float* __restrict__ prev, const float* __restrict__ ef,
-                                                               float mu, int64_t n, float* __restrict__ sums) {
+                                                               float mu, int64_t n, Sum* __restrict__ sums) {
   float xp = 0.0f, pp = 0.0f;
   const int64_t stride = int64_t(gridDim.x) * kThreads * kPer;
   for (int64_t base = (int64_t(blockIdx.x) * kThreads + threadIdx.x) * kPer; base < n; base += stride) {
@@ -115,18 +116,19 @@ __global__ void __launch_bounds__(kThreads) packet_gain_kernel(const T* __restri
   }
   __syncthreads();
   if (threadIdx.x < 2) {
-    float a = 0.0f;
+    Sum a = Sum(0);
 #pragma unroll
-    for (int i = 0; i < kThreads / 32; ++i) a += red[threadIdx.x][i];
+    for (int i = 0; i < kThreads / 32; ++i) a += Sum(red[threadIdx.x][i]);
     atomicAdd(&sums[threadIdx.x], a);
   }
 }
 
 // kappa: fixed (>= 0) or taken from the inner products in `sums` (fixed < 0). Thread 0 of block 0 writes the value
 // it used into the payload's gain field.
-__device__ __forceinline__ float resolve_gain(float fixed, const float* sums) {
+template <typename Sum>
+__device__ __forceinline__ float resolve_gain(float fixed, const Sum* sums) {
   if (fixed >= 0.0f) return fixed;
-  const float xp = sums[0], pp = sums[1];
+  const float xp = float(sums[0]), pp = float(sums[1]);
   return pp > 0.0f ? fminf(fmaxf(xp / pp, 0.0f), 1.0f) : 0.0f;
 }
 
@@ -136,10 +138,10 @@ struct PacketHead {
   uint32_t* dst;  // NULL: none
 };
 
-template <typename T>
+template <typename T, typename Sum>
 __global__ void __launch_bounds__(kThreads) packet_encode_kernel(const T* __restrict__ grad, const float* __restrict__ curr,
                                                                  const float* __restrict__ prev, float* __restrict__ ef,
-                                                                 float mu, float fixed_gain, const float* __restrict__ sums,
+                                                                 float mu, float fixed_gain, const Sum* __restrict__ sums,
                                                                  int64_t n, float* __restrict__ gain_out,
                                                                  float* __restrict__ scales, uint8_t* __restrict__ packed,
                                                                  const __grid_constant__ PacketHead head) {
@@ -259,23 +261,24 @@ extern "C" int64_t nangila_packet_payload_bytes(int64_t n) { return 20 + 4 * ((n
 
 namespace nangila {
 namespace {
-// `sums`: two floats for the inner products, used when the gain is to be derived.
+// `sums`: two numbers for the inner products, used when the gain is to be derived.
+template <typename Sum>
 cudaError_t launch_encode(const void* grad, int32_t dtype, const float* curr, const float* prev, float* ef, float mu, float gain, int64_t n,
-                          uint8_t* payload, float* sums, const PacketHead& head, cudaStream_t stream) {
+                          uint8_t* payload, Sum* sums, const PacketHead& head, cudaStream_t stream) {
   float* gain_out = reinterpret_cast<float*>(payload + 16);
   float* scales = reinterpret_cast<float*>(payload + 20);
   uint8_t* packed = payload + 20 + 4 * ((n + 63) / 64);
   const int grid = grid_for(n);
   if (curr == nullptr) gain = 0.0f;
   if (gain < 0.0f) {
-    const cudaError_t e = cudaMemsetAsync(sums, 0, 2 * sizeof(float), stream);
+    const cudaError_t e = cudaMemsetAsync(sums, 0, 2 * sizeof(Sum), stream);
     if (e != cudaSuccess) return e;
   }
 #define NANGILA_PACKET_LAUNCH(TYPE)                                                                                  \
   do {                                                                                                               \
     if (gain < 0.0f)                                                                                                 \
-      packet_gain_kernel<TYPE><<<grid, kThreads, 0, stream>>>(static_cast<const TYPE*>(grad), curr, prev, ef, mu, n, sums); \
-    packet_encode_kernel<TYPE><<<tiles_grid(n), kThreads, 0, stream>>>(static_cast<const TYPE*>(grad), curr, prev, ef, mu, gain, \
+      packet_gain_kernel<TYPE, Sum><<<grid, kThreads, 0, stream>>>(static_cast<const TYPE*>(grad), curr, prev, ef, mu, n, sums); \
+    packet_encode_kernel<TYPE, Sum><<<tiles_grid(n), kThreads, 0, stream>>>(static_cast<const TYPE*>(grad), curr, prev, ef, mu, gain, \
                                                               sums, n, gain_out, scales, packed, head);              \
   } while (0)
   switch (dtype) {
@@ -323,9 +326,11 @@ extern "C" int nangila_packet_encode(const void* grad, int32_t dtype, const floa
 // knows from its own parameters, and the checksum kernel puts its result where it belongs. For small layers the call is what
 // costs: 10 007 FP32 elements through compress_gpu, decompress_gpu and update_gpu took 142 us with the header and the checksum copied in by
 // tensor operations and two synchronisations before decoding, 91 us this way.
-extern "C" int nangila_packet_compress(const void* grad, int32_t dtype, const float* curr, const float* prev, float* ef, float mu,
-                                       float gain, int64_t n, const uint8_t* header, uint8_t* packet, float* sums, cudaStream_t stream) {
-  using namespace nangila;
+namespace nangila {
+namespace {
+template <typename Sum>
+int compress(const void* grad, int32_t dtype, const float* curr, const float* prev, float* ef, float mu, float gain, int64_t n, const uint8_t* header,
+             uint8_t* packet, Sum* sums, cudaStream_t stream) {
   if (bad_encode(grad, curr, prev, mu, n, packet) || header == nullptr || sums == nullptr) return int(cudaErrorInvalidValue);
   PacketHead head;
   memcpy(head.word, header, 32);
@@ -336,6 +341,17 @@ extern "C" int nangila_packet_compress(const void* grad, int32_t dtype, const fl
   if (e != cudaSuccess) return int(e);
   uint32_t* crc = reinterpret_cast<uint32_t*>(packet + 12);
   return nangila_crc32_cleared(packet + 32, nangila_packet_payload_bytes(n), crc, stream);  // the encoder has written the header
+}
+}  // namespace
+}  // namespace nangila
+
+extern "C" int nangila_packet_compress(const void* grad, int32_t dtype, const float* curr, const float* prev, float* ef, float mu,
+                                       float gain, int64_t n, const uint8_t* header, uint8_t* packet, float* sums, cudaStream_t stream) {
+  return nangila::compress(grad, dtype, curr, prev, ef, mu, gain, n, header, packet, sums, stream);
+}
+extern "C" int nangila_packet_compress_f64(const void* grad, int32_t dtype, const float* curr, const float* prev, float* ef, float mu,
+                                           float gain, int64_t n, const uint8_t* header, uint8_t* packet, double* sums, cudaStream_t stream) {
+  return nangila::compress(grad, dtype, curr, prev, ef, mu, gain, n, header, packet, sums, stream);
 }
 
 namespace nangila {
