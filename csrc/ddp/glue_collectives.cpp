@@ -233,6 +233,30 @@ at::Tensor sculptor_layer_sumsq(const std::vector<at::Tensor>& layers) {
                                                  at::cuda::getCurrentCUDAStream()), "sculptor_layer_sumsq");
   return out;
 }
+// The sums on their way to the host: queued by begin(), read by result(), which waits for the copy alone and not for what was queued after it.
+class PendingSums {
+ public:
+  explicit PendingSums(const std::vector<at::Tensor>& layers) : sums_(sculptor_layer_sumsq(layers)) {
+    c10::cuda::CUDAGuard guard(sums_.device());
+    host_ = at::empty({sums_.numel()}, at::TensorOptions().dtype(at::kDouble).pinned_memory(true));
+    auto stream = at::cuda::getCurrentCUDAStream();
+    check_launch(int(cudaMemcpyAsync(host_.data_ptr<double>(), sums_.data_ptr<double>(), size_t(sums_.numel()) * sizeof(double), cudaMemcpyDeviceToHost, stream)),
+                 "sculptor_layer_sumsq");
+    arrived_.record(stream);
+  }
+  std::vector<double> result() {
+    {
+      py::gil_scoped_release release;
+      arrived_.synchronize();
+    }
+    const double* p = host_.data_ptr<double>();
+    return std::vector<double>(p, p + host_.numel());
+  }
+
+ private:
+  at::Tensor sums_, host_;
+  at::cuda::CUDAEvent arrived_;
+};
 std::vector<NangilaPairDesc> pair_descs(const std::vector<at::Tensor>& xi, const std::vector<at::Tensor>& xj,
                                         const std::vector<at::Tensor>& state, const std::vector<int64_t>& count_after,
                                         int64_t* mx) {
@@ -530,6 +554,7 @@ void register_more(py::module_& m) {
   m.def("rs_region_layout", &rs_region_layout);
   m.def("rs_launch", &rs_launch);
   m.def("ag_region_layout", &ag_region_layout);
+  py::class_<PendingSums>(m, "PendingSums").def(py::init<const std::vector<at::Tensor>&>(), py::arg("layers")).def("result", &PendingSums::result);
   m.attr("LAYOUT_CTAS") = py::int_(NANGILA_LAYOUT_CTAS);
   m.def("ag_chunk_elems", [](int64_t shard, int64_t resident) { return nangila_ag_chunk_elems(shard, int32_t(resident)); });
   m.def("ag_launch", &ag_launch);
