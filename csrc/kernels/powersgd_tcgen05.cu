@@ -31,6 +31,7 @@
 #include "ptx_sm100.cuh"
 #include "quant.cuh"
 #include "signal.cuh"
+#include "warp_sums.cuh"
 
 namespace nangila {
 namespace {
@@ -503,13 +504,7 @@ __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_c
             for (int j = 0; j <= c; ++j, ++q) acc[q] = __fmaf_rn(w[c], w[j], acc[q]);
         }
       }
-#pragma unroll
-      for (int q = 0; q < kAcc; ++q) {
-        float v = acc[q];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if (lane == 0) s_warp[warp][q] = v;
-      }
+      warp_sums(acc, [&](int q, float v) { s_warp[warp][q] = v; });
     } else {
       // 136 sums are too many for a thread's registers: a warp's lanes share them out, and each lane walks the warp's rows
       __syncthreads();  // rows of other threads: the pass before this one has written them
