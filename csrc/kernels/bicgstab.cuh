@@ -20,7 +20,10 @@
 // one slot of partial sums read per thread. (A flag per CTA that every CTA polls: 8 us; the slots of all CTAs read by one warp,
 // their values interleaved in shared lines: 4.5 to 9 us.) So a CTA's slice of the matrix stays in shared memory over all iterations where it fits,
 // and small systems run on few CTAs, or on one. Measured on B200, us per iteration of whole calls, copies included, against
-// one CUDA graph of 13 kernels per iteration: mesh of 400 nodes 59 -> 3.9, 2500: 57 -> 7.0, 65 536: 70 -> 9.0, 400 000: 83 -> 22, 10^6: 180 -> 69.
+// one CUDA graph of 13 kernels per iteration: mesh of 400 nodes 59 -> 3.9, 2500: 57 -> 7.0, 65 536: 70 -> 8.9, 400 000: 83 -> 22, 10^6: 180 -> 69.
+// With the values of a sum shared out among the lanes while a warp adds them up, a barrier less, and all entries of a row gathered at once:
+// 10 000 nodes 7.11 -> 6.76, 65 536: 8.90 -> 8.38, 300 000: 16.4 -> 15.7. (Partial sums that carry their number, which every CTA looks at itself instead of
+// a counter, took 10 us at 65 536 nodes.)
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -40,6 +43,7 @@ constexpr int kEntriesPerCta = 2048;
 constexpr int kMaxCtas = 512;         // a sum reads the CTAs' slots with one thread each
 constexpr int kLongRow = 64;          // rows above this many entries are summed by a whole warp each
 constexpr int kCheckEvery = 4;        // iterations between two tests of the residual
+constexpr int kAtOnce = 5;            // entries of a row gathered together: a mesh's
 // Below these shares of what they are differences of, <r, r> and <r0, r> are summed from r itself. |r| < 0.1 |s|: an error of about
 // 1e-16 |s|^2 is then 1e-14 of |r|^2. <r0, r> may be small of itself; its line only has to catch what is nothing but rounding.
 constexpr double kCancelled = 1e-2;
@@ -85,27 +89,40 @@ struct GridSum {
   double* partial;
   uint32_t* arrived;
   uint64_t timeout_ns;
-  double (*sh)[kSums];  // [WARPS]
+  double (*twice)[WARPS][kSums];  // by parity of the sum's number: a thread may be a sum ahead of another's last look
   int* failed;
   uint32_t k = 0;
+  // The sum over a warp of each of N values: value i in lane 4 i. The values are shared out among the lanes as they are added up
+  // (nine exchanges for five values; each on its own takes 25).
   template <int N>
-  __device__ __forceinline__ void warp_sum(double (&v)[N]) {
+  static __device__ __forceinline__ double warp_sums(const double (&v)[N]) {
+    const int lane = threadIdx.x & 31;
+    double a[8];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
+    for (int i = 0; i < 8; ++i) a[i] = i < N ? v[i < N ? i : 0] : 0.0;
 #pragma unroll
-      for (int i = 0; i < N; ++i) v[i] += __shfl_down_sync(0xffffffffu, v[i], off);
+    for (int half = 4; half >= 1; half >>= 1) {
+      const bool upper = (lane & (4 * half)) != 0;
+#pragma unroll
+      for (int i = 0; i < half; ++i) {
+        if (i < N) {  // (above N only zeros would meet)
+          const double other = __shfl_xor_sync(0xffffffffu, upper ? a[i] : a[i + half], 4 * half);
+          a[i] = (upper ? a[i + half] : a[i]) + other;
+        }
+      }
     }
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 2);
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
+    return a[0];
   }
   template <int N>
   __device__ __forceinline__ bool operator()(double (&v)[N]) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ctas = int(gridDim.x);
     ++k;
-    warp_sum(v);
-    if (lane == 0) {
-#pragma unroll
-      for (int i = 0; i < N; ++i) sh[warp][i] = v[i];
-    }
+    double (*sh)[kSums] = twice[k & 1u];
+    const double mine = warp_sums(v);
+    if ((lane & 3) == 0 && lane / 4 < N) sh[warp][lane / 4] = mine;
     __syncthreads();
     if (ctas == 1) {
       if (warp == 0 && lane < N) {
@@ -155,11 +172,8 @@ struct GridSum {
           v[i] = w.x;
           if (i + 1 < N) v[i + 1] = w.y;
         }
-        warp_sum(v);
-        if (lane == 0) {
-#pragma unroll
-          for (int i = 0; i < N; ++i) sh[warp][i] = v[i];
-        }
+        const double part = warp_sums(v);
+        if ((lane & 3) == 0 && lane / 4 < N) sh[warp][lane / 4] = part;
       }
       __syncthreads();
     }
@@ -169,7 +183,6 @@ struct GridSum {
 #pragma unroll
       for (int i = 0; i < N; ++i) v[i] += sh[w][i];
     }
-    __syncthreads();  // the next sum writes there again
     return *reinterpret_cast<volatile int*>(failed) == 0;
   }
 };
@@ -178,7 +191,7 @@ template <bool RESIDENT>
 __global__ void __launch_bounds__(solver_threads(RESIDENT), 1) bicgstab_kernel(const __grid_constant__ SolverArgs a) {
   constexpr int kThreads = solver_threads(RESIDENT), kWarps = kThreads / 32;
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double sh[kWarps][kSums];
+  __shared__ double sh[2][kWarps][kSums];
   __shared__ int failed;
   const int tid = threadIdx.x;
   const int r0 = a.first_row[blockIdx.x], r1 = a.first_row[blockIdx.x + 1], rows = r1 - r0;
@@ -231,8 +244,19 @@ __global__ void __launch_bounds__(solver_threads(RESIDENT), 1) bicgstab_kernel(c
       if (mine && lane == 0) own = load(r0 + i);
       double sum = 0.0;
       if (mine) {
-#pragma unroll 4
-        for (int j = s + lane; j < e; j += lanes) sum += val[j] * gather(col[j]);
+        // all gathers of a short row at once, at a valid place whatever its length: the next one would wait for a trip to L2 otherwise
+        for (int j = s + lane; j < e; j += kAtOnce * lanes) {
+          double g[kAtOnce], w[kAtOnce];
+#pragma unroll
+          for (int u = 0; u < kAtOnce; ++u) {
+            const int at = min(j + u * lanes, e - 1);
+            g[u] = gather(col[at]);
+            w[u] = val[at];
+          }
+#pragma unroll
+          for (int u = 0; u < kAtOnce; ++u)
+            if (j + u * lanes < e) sum += w[u] * g[u];
+        }
       }
       for (int off = lanes >> 1; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off, lanes);
       if (mine && lane == 0) finish(r0 + i, own, sum);
