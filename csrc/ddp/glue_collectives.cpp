@@ -140,7 +140,15 @@ at::Tensor packet_compress(const at::Tensor& grad, const c10::optional<at::Tenso
   };
   c10::cuda::CUDAGuard guard(grad.device());
   auto packet = at::empty({32 + nangila_packet_payload_bytes(n)}, grad.options().dtype(at::kByte));
-  auto sums = at::empty({2}, grad.options().dtype(at::kDouble));
+  // The gain's sums: in FP32 where few parts meet (64 CTAs of 2048 elements: off by 1e-7), in 64 bits beyond.
+  const bool few = n <= 64 * 2048;
+  auto sums = at::empty({2}, grad.options().dtype(few ? at::kFloat : at::kDouble));
+  if (few) {
+    check_launch(nangila_packet_compress(grad.data_ptr(), dtype_code(grad), f32(curr, "curr"), f32(prev, "prev"), f32(ef, "ef"), float(mu),
+                                         float(gain), n, reinterpret_cast<const uint8_t*>(header.data()), packet.data_ptr<uint8_t>(),
+                                         sums.data_ptr<float>(), at::cuda::getCurrentCUDAStream()), "packet_compress");
+    return packet;
+  }
   check_launch(nangila_packet_compress_f64(grad.data_ptr(), dtype_code(grad), f32(curr, "curr"), f32(prev, "prev"), f32(ef, "ef"), float(mu),
                                        float(gain), n, reinterpret_cast<const uint8_t*>(header.data()), packet.data_ptr<uint8_t>(),
                                        sums.data_ptr<double>(), at::cuda::getCurrentCUDAStream()), "packet_compress");
