@@ -233,7 +233,7 @@ cudaError_t launch(const NangilaAgParams& p, cudaStream_t stream) {
   ag_quantize_kernel<T, BITS><<<dim3(unsigned(std::min(cap, tiles)), unsigned(p.nvr)), kThreads, 0, stream>>>(p, sh);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || p.world == 1) return e;
-  if ((e = launch_meet(p, p.flag_off, kTimeoutPhase3, 3u, stream)) != cudaSuccess) return e;
+  if ((e = launch_meet(p, p.flag_off, kTimeoutPhase3, 3u, kMeetlessCtas + 1, stream)) != cudaSuccess) return e;
   const dim3 grid(unsigned(std::min(std::max<int64_t>(1, cap / (p.world - 1)), tiles)), unsigned(p.world - 1), unsigned(p.nvr));
   return launch_following(ag_expand_kernel<T, BITS>, grid, kThreads, 0, stream, p, sh, int(tiles));
 }

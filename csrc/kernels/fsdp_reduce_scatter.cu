@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kThreads, 4) rs_sum_kernel(const __grid_consta
   const int vr = blockIdx.y, me = p.rank0 + vr, W = sh.W, C = sh.C, tid = threadIdx.x;
   uint8_t* myreg = p.region[me];
   follow();
-  if (*reinterpret_cast<volatile uint32_t*>(&p.status[vr][kStatusCode]) != 0u) return;  // a rank's data did not come
+  const uint32_t seen = status_seen(p);
   T* __restrict__ out = static_cast<T*>(p.out_shard[vr]);
   for (int tile = blockIdx.x; tile < sh.tiles; tile += gridDim.x) {
     const int j = int(unsigned(tile) / unsigned(sh.sub)), it0 = (tile - j * sh.sub) * kTile;
@@ -188,6 +188,7 @@ __global__ void __launch_bounds__(kThreads, 4) rs_sum_kernel(const __grid_consta
           dequant8_bf16_fma2(packed[b], __floats2bfloat162_rn(s, s), acc[b]);
         }
       }
+      if (!all_came(p, vr, seen, kTimeoutPhase2, 2u)) return;
 #pragma unroll
       for (int b = 0; b < kTile; ++b)
         if (b < left) *reinterpret_cast<uint4*>(out + at0 + b * kElemsPerIter) = make_uint4(acc[b][0], acc[b][1], acc[b][2], acc[b][3]);
@@ -204,6 +205,7 @@ __global__ void __launch_bounds__(kThreads, 4) rs_sum_kernel(const __grid_consta
 #pragma unroll
           for (int b = 0; b < kBatch; ++b) dequant8_add(packed[b], bf16_bits_to_float(scale[b]), acc[b]);
         }
+        if (!all_came(p, vr, seen, kTimeoutPhase2, 2u)) return;
 #pragma unroll
         for (int b = 0; b < kBatch; ++b)
           if (b0 + b < left) {
@@ -239,9 +241,9 @@ cudaError_t launch(const NangilaPredResParams& p, cudaStream_t stream) {
   }
   if (phases & 2) {
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = launch_meet(p, p.flag1_off, kTimeoutPhase2, 2u, stream);
-    if (e != cudaSuccess) return e;
     const dim3 grid(unsigned(cap > 0 ? std::min(sh.tiles, cap) : sh.tiles), unsigned(p.nvr));
+    if (e == cudaSuccess) e = launch_meet(p, p.flag1_off, kTimeoutPhase2, 2u, int64_t(grid.x) * grid.y, stream);
+    if (e != cudaSuccess) return e;
     return launch_following(rs_sum_kernel<T, kPackedBf16<T, S>>, grid, kThreads, 0, stream, p, sh);
   }
   return cudaGetLastError();

@@ -160,3 +160,51 @@ def test_a_rank_that_has_failed_before_is_missed(what):
     call()
     obj.check_status()
     assert not (outs[0] == 3.0).any()
+
+
+class _Rank:
+    """One rank of a group of two whose regions are shared with the other's object."""
+
+    world, provider = 2, "test"
+
+    def __init__(self, rank, region):
+        self.rank, self._region = rank, region
+
+    def allocate(self, nbytes):
+        if not self._region:
+            self._region.append(_loopback(2).allocate(nbytes))
+        return self._region[0]
+
+
+@pytest.mark.parametrize("what", ["reduce_scatter", "all_gather"])
+def test_ranks_of_a_group_meet(what):
+    """Rank 1 first (rank 0's word is put there by hand, so that it has nothing to wait for), then rank 0, which finds rank 1's codes and word: the same
+    bits as with both ranks in one launch. Three launches of both parities."""
+    from nangila.parallel import fsdp_collectives as F
+
+    cls = F.NangilaAllGather if what == "all_gather" else F.NangilaReduceScatter
+    shard = 3 * 8192 - 8
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    region = []
+    ranks = [cls(arena=_Rank(r, region), timeout_s=0.5, **({} if what == "all_gather" else {"stochastic": False})) for r in range(2)]
+    both = cls(arena=_loopback(2), **({} if what == "all_gather" else {"stochastic": False}))
+    size = 2 * shard if what == "all_gather" else shard
+    for epoch in (1, 2, 3):
+        ins = [(torch.randn(shard if what == "all_gather" else 2 * shard, device=DEV, generator=gen) * 0.02).to(torch.bfloat16) for _ in range(2)]
+        want = [torch.empty(size, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+        got = [torch.empty(size, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+        call = (lambda o, w, x: o.gather(w, x)) if what == "all_gather" else (lambda o, w, x: o.reduce(w, x, 0.5))
+        call(both, want, ins)
+        if epoch == 1:  # the regions exist from the first call on: let rank 1's wait for the word run out once
+            call(ranks[1], [got[1]], [ins[1]])
+            with pytest.raises(RuntimeError, match="waiting for rank 0"):
+                ranks[1].check_status()
+        else:
+            st = next(iter(ranks[1]._regions.values()))
+            at = st["f"] if what == "all_gather" else st["f1"]
+            region[0].segment._keepalive[1][at:at + 4].view(torch.int32)[0] = epoch
+            call(ranks[1], [got[1]], [ins[1]])
+            ranks[1].check_status()
+        call(ranks[0], [got[0]], [ins[0]])
+        ranks[0].check_status()
+        assert torch.equal(got[0], want[0])
