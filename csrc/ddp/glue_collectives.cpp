@@ -154,6 +154,34 @@ at::Tensor packet_compress(const at::Tensor& grad, const c10::optional<at::Tenso
                                        sums.data_ptr<double>(), at::cuda::getCurrentCUDAStream()), "packet_compress");
   return packet;
 }
+// Pinned memory that work queued on `stream` writes. It goes back to its pool, which knows nothing of such writes, only when they are done: also where an
+// exception ends the call, or nobody asks for what was written.
+class Landing {
+ public:
+  Landing(int64_t n, at::ScalarType type, at::cuda::CUDAStream stream)
+      : stream_(stream), block_(at::empty({n}, at::TensorOptions().dtype(type).pinned_memory(true))) {}
+  Landing(const Landing&) = delete;
+  Landing& operator=(const Landing&) = delete;
+  ~Landing() {
+    if (!arrived_ && cudaStreamSynchronize(stream_) != cudaSuccess) (void)cudaGetLastError();
+  }
+  const at::Tensor& block() const { return block_; }
+  // All writes have been queued: wait() waits for nothing that is queued from here on.
+  void complete() { written_.record(stream_); }
+  void wait() {
+    {
+      py::gil_scoped_release release;
+      written_.synchronize();
+    }
+    arrived_ = true;
+  }
+
+ private:
+  at::cuda::CUDAStream stream_;
+  at::Tensor block_;
+  at::cuda::CUDAEvent written_;
+  bool arrived_ = false;
+};
 // What the host has to know of a packet: the first (up to) 44 bytes and, if asked for, the CRC32 of everything behind the header. One
 // synchronisation for both. With `out` the decoder is queued behind them, so that the device need not wait for the host's verdict; it
 // checks the header itself. The last part of the answer says whether it was queued.
@@ -161,11 +189,23 @@ py::tuple packet_inspect(const at::Tensor& packet, bool checksum, int64_t layer,
                          const c10::optional<at::Tensor>& prev, double mu, const c10::optional<at::Tensor>& out) {
   TORCH_CHECK(packet.is_cuda() && packet.scalar_type() == at::kByte && packet.is_contiguous() && packet.numel() > 32,
               "nangila: packet_inspect wants a contiguous uint8 CUDA packet");
+  // (nothing is queued before all that may be refused has been looked at)
+  const bool queue = out.has_value() && layer >= 0 && layer <= 0xffffffffll;
+  const float *c = nullptr, *p = nullptr;
+  if (queue) {
+    auto f32 = [&](const at::Tensor& t, const char* what) -> float* {
+      TORCH_CHECK(t.device() == packet.device() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.numel() == out->numel(), "nangila: ", what,
+                  " must be a contiguous FP32 tensor on the packet's device, of the size of the result");
+      return t.data_ptr<float>();
+    };
+    f32(*out, "out");
+    if (curr.has_value()) c = f32(*curr, "curr");
+    if (prev.has_value()) p = f32(*prev, "prev");
+    TORCH_CHECK(c == nullptr || p != nullptr, "nangila: a history has two parts");
+  }
   const int64_t fixed = std::min<int64_t>(packet.numel(), 44);
   c10::cuda::CUDAGuard guard(packet.device());
   auto stream = at::cuda::getCurrentCUDAStream();
-  auto host = at::empty({48}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
-  uint8_t* h = host.data_ptr<uint8_t>();
   at::Tensor word;
   uint32_t* w = nullptr;
   if (checksum) {
@@ -173,23 +213,14 @@ py::tuple packet_inspect(const at::Tensor& packet, bool checksum, int64_t layer,
     w = reinterpret_cast<uint32_t*>(word.data_ptr<int32_t>());
     check_launch(nangila_crc32(packet.data_ptr<uint8_t>() + 32, packet.numel() - 32, w, w, stream), "crc32");
   }
+  Landing host(48, at::kByte, stream);
+  uint8_t* h = host.block().data_ptr<uint8_t>();
   check_launch(nangila_packet_report(packet.data_ptr<uint8_t>(), int32_t(fixed), w, h, stream), "packet_inspect");
-  at::cuda::CUDAEvent reported;
-  reported.record(stream);
-  bool queued = false;
-  if (out.has_value() && layer >= 0 && layer <= 0xffffffffll) {
-    const int64_t n = out->numel();
-    TORCH_CHECK(out->is_cuda() && out->scalar_type() == at::kFloat && out->is_contiguous(), "nangila: out must be FP32 CUDA");
-    const float* c = curr.has_value() ? curr->data_ptr<float>() : nullptr;
-    const float* p = prev.has_value() ? prev->data_ptr<float>() : nullptr;
-    if (c) TORCH_CHECK(curr->numel() == n && prev.has_value() && prev->numel() == n, "nangila: history size mismatch");
-    // (refused: too short or misaligned for what is expected; the host will say what is wrong with it)
-    queued = nangila_packet_decode_expected(packet.data_ptr<uint8_t>(), packet.numel(), uint32_t(layer), c, p, float(mu), n, out->data_ptr<float>(), stream) == 0;
-  }
-  {
-    py::gil_scoped_release release;
-    reported.synchronize();
-  }
+  host.complete();
+  // (not queued: too short or misaligned for what is expected; the host will say what is wrong with it)
+  const bool queued = queue && nangila_packet_decode_expected(packet.data_ptr<uint8_t>(), packet.numel(), uint32_t(layer), c, p, float(mu), out->numel(),
+                                                              out->data_ptr<float>(), stream) == 0;
+  host.wait();
   uint32_t crc = 0;
   if (checksum) std::memcpy(&crc, h + 44, 4);
   return py::make_tuple(py::bytes(reinterpret_cast<const char*>(h), size_t(fixed)), crc, queued);
@@ -244,26 +275,22 @@ at::Tensor sculptor_layer_sumsq(const std::vector<at::Tensor>& layers) {
 // The sums on their way to the host: queued by begin(), read by result(), which waits for the copy alone and not for what was queued after it.
 class PendingSums {
  public:
-  explicit PendingSums(const std::vector<at::Tensor>& layers) : sums_(sculptor_layer_sumsq(layers)) {
+  explicit PendingSums(const std::vector<at::Tensor>& layers)
+      : sums_(sculptor_layer_sumsq(layers)), host_(sums_.numel(), at::kDouble, at::cuda::getCurrentCUDAStream(sums_.device().index())) {
     c10::cuda::CUDAGuard guard(sums_.device());
-    host_ = at::empty({sums_.numel()}, at::TensorOptions().dtype(at::kDouble).pinned_memory(true));
-    auto stream = at::cuda::getCurrentCUDAStream();
-    check_launch(int(cudaMemcpyAsync(host_.data_ptr<double>(), sums_.data_ptr<double>(), size_t(sums_.numel()) * sizeof(double), cudaMemcpyDeviceToHost, stream)),
-                 "sculptor_layer_sumsq");
-    arrived_.record(stream);
+    check_launch(int(cudaMemcpyAsync(host_.block().data_ptr<double>(), sums_.data_ptr<double>(), size_t(sums_.numel()) * sizeof(double),
+                                     cudaMemcpyDeviceToHost, at::cuda::getCurrentCUDAStream())), "sculptor_layer_sumsq");
+    host_.complete();
   }
   std::vector<double> result() {
-    {
-      py::gil_scoped_release release;
-      arrived_.synchronize();
-    }
-    const double* p = host_.data_ptr<double>();
-    return std::vector<double>(p, p + host_.numel());
+    host_.wait();
+    const double* p = host_.block().data_ptr<double>();
+    return std::vector<double>(p, p + sums_.numel());
   }
 
  private:
-  at::Tensor sums_, host_;
-  at::cuda::CUDAEvent arrived_;
+  at::Tensor sums_;
+  Landing host_;
 };
 std::vector<NangilaPairDesc> pair_descs(const std::vector<at::Tensor>& xi, const std::vector<at::Tensor>& xj,
                                         const std::vector<at::Tensor>& state, const std::vector<int64_t>& count_after,
