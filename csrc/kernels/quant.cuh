@@ -330,10 +330,11 @@ __device__ __forceinline__ void quantize8_bf16(uint32_t (&x)[4], uint32_t& packe
   const float s = bf16_bits_to_float(scale_bits);
   const bool live = s > 1e-30f;
   if (!live) scale_bits = 0u;
-  // 1 / s truncated to bf16, never above it. The approximate reciprocal (within 1 ulp) has the same upper 16 bits as the exact one: s has 8 significant
-  // bits, so 1 / s is at least 2^-16 of itself away from every bf16 number unless s is a power of two, and it never is one: no bf16 number
-  // lies in [6.98, 7) and 7 fl(1/7) is above 1.
-  const uint32_t inv_bits = live ? (__float_as_uint(rcp_approx(s)) >> 16) : 0u;
+  // 1 / s truncated to bf16, never above it. The approximate reciprocal is off by up to 1 ulp (two floats where 1 / s is a power of two and the floats below it
+  // lie half as far apart), so it may fall short of a bf16 number that 1 / s is: of a power of two, which s is wherever the largest magnitude is 7 2^k
+  // (7 fl(1/7) is rounded to 1). The two floats added make up for that, and for no other s do they matter: s has 8 significant
+  // bits, so 1 / s is at least 2^-16 of itself, 128 floats, away from every other bf16 number.
+  const uint32_t inv_bits = live ? ((__float_as_uint(rcp_approx(s)) + 2u) >> 16) : 0u;
   const bf162 inv2 = as_bf162(inv_bits | (inv_bits << 16));
   const uint32_t s2_bits = scale_bits | (scale_bits << 16);
   const bf162 s2 = as_bf162(s2_bits), neg_s2 = as_bf162(s2_bits ^ 0x80008000u);
