@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "fsdp_grid.cuh"
 #include "meet.cuh"
 #include "nangila_kernels.h"
 #include "quant.cuh"
@@ -192,50 +193,52 @@ __global__ void __launch_bounds__(kThreads, 5) ag_quantize_kernel(const __grid_c
   }
 }
 
-template <typename T, int BITS>
+template <typename T, int BITS, bool ALL>  // ALL: there are fewer CTAs than owners, so one takes several of these
 __global__ void __launch_bounds__(kThreads, 8) ag_expand_kernel(const __grid_constant__ NangilaAgParams p, const __grid_constant__ AgShape sh, int tiles) {
   const int vr = blockIdx.z, me = p.rank0 + vr, W = p.world, tid = threadIdx.x;
-  int o = me + 1 + int(blockIdx.y);  // the other ranks' shards
-  if (o >= W) o -= W;
   follow();
   const uint32_t failed = *reinterpret_cast<volatile uint32_t*>(&p.status[vr][kStatusCode]);  // not 0: a rank's data did not come
   const uint8_t* myreg = p.region[me];
-  T* __restrict__ out = static_cast<T*>(p.out_full[vr]) + int64_t(o) * p.shard_elems;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    const int64_t at0 = int64_t(tile) * (kTile * kPerIter) + tid * kE, left = p.shard_elems - at0;
-    const AgSlot<BITS> slot(sh, o, tile * kTile, tid);
-    const Packed<BITS>* codes = reinterpret_cast<const Packed<BITS>*>(myreg + slot.codes);
-    const uint16_t* scales = reinterpret_cast<const uint16_t*>(myreg + slot.scales);
-    Packed<BITS> w[kTile];
-    uint16_t sc[kTile];
+  int d = blockIdx.y;
+  do {
+    int o = me + 1 + d;  // the other ranks' shards
+    if (o >= W) o -= W;
+    T* __restrict__ out = static_cast<T*>(p.out_full[vr]) + int64_t(o) * p.shard_elems;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+      const int64_t at0 = int64_t(tile) * (kTile * kPerIter) + tid * kE, left = p.shard_elems - at0;
+      const AgSlot<BITS> slot(sh, o, tile * kTile, tid);
+      const Packed<BITS>* codes = reinterpret_cast<const Packed<BITS>*>(myreg + slot.codes);
+      const uint16_t* scales = reinterpret_cast<const uint16_t*>(myreg + slot.scales);
+      Packed<BITS> w[kTile];
+      uint16_t sc[kTile];
 #pragma unroll
-    for (int b = 0; b < kTile; ++b) {
-      if (b * kPerIter < left) {
-        w[b] = codes[b * kThreads];
-        sc[b] = scales[b * (kPerIter / kQuantBlock)];
+      for (int b = 0; b < kTile; ++b) {
+        if (b * kPerIter < left) {
+          w[b] = codes[b * kThreads];
+          sc[b] = scales[b * (kPerIter / kQuantBlock)];
+        }
       }
-    }
-    if (failed != 0u) return;
+      if (failed != 0u) return;
 #pragma unroll
-    for (int b = 0; b < kTile; ++b)
-      if (b * kPerIter < left) expand8<T, BITS>(w[b], sc[b], out + at0 + b * kPerIter);
-  }
+      for (int b = 0; b < kTile; ++b)
+        if (b * kPerIter < left) expand8<T, BITS>(w[b], sc[b], out + at0 + b * kPerIter);
+    }
+    d += gridDim.y;
+  } while (ALL && d < W - 1);
 }
 
 template <typename T, int BITS>
 cudaError_t launch(const NangilaAgParams& p, cudaStream_t stream) {
   const int64_t total = (p.shard_elems + kPerIter - 1) / kPerIter, tiles = (total + kTile - 1) / kTile;
-  if (total > 0x3fffffff) return cudaErrorInvalidValue;
+  if (tiles > kMaxTiles) return cudaErrorInvalidValue;
   const AgShape sh(p, BITS);
-  // fewer CTAs asked for than chunks to quantize and to expand: a cap
-  const int64_t cps = (p.shard_elems + p.chunk_elems - 1) / p.chunk_elems;
-  const int64_t cap = p.grid_x > 0 && p.grid_x < cps * (p.world + 1) ? p.grid_x : 0x7fffffff;
-  ag_quantize_kernel<T, BITS><<<dim3(unsigned(std::min(cap, tiles)), unsigned(p.nvr)), kThreads, 0, stream>>>(p, sh);
+  ag_quantize_kernel<T, BITS><<<dim3(fsdp_grid(tiles, 1, p.grid_x).x, unsigned(p.nvr)), kThreads, 0, stream>>>(p, sh);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || p.world == 1) return e;
   if ((e = launch_meet(p, p.flag_off, kTimeoutPhase3, 3u, kMeetlessCtas + 1, stream)) != cudaSuccess) return e;
-  const dim3 grid(unsigned(std::min(std::max<int64_t>(1, cap / (p.world - 1)), tiles)), unsigned(p.world - 1), unsigned(p.nvr));
-  return launch_following(ag_expand_kernel<T, BITS>, grid, kThreads, 0, stream, p, sh, int(tiles));
+  const FsdpGrid g = fsdp_grid(tiles, p.world - 1, p.grid_x);
+  auto* expand = g.walk == kWalkGroups ? ag_expand_kernel<T, BITS, true> : ag_expand_kernel<T, BITS, false>;
+  return launch_following(expand, dim3(g.x, g.y, unsigned(p.nvr)), kThreads, 0, stream, p, sh, int(tiles));
 }
 
 }  // namespace
@@ -253,7 +256,7 @@ extern "C" uint64_t nangila_ag_region_bytes(int64_t shard_elems, int32_t world, 
   return off;
 }
 
-// Chunk size for a shard: what a rank's slot is rounded up to, and the unit of the caller's cap on CTAs. About one chunk for each of the `resident`
+// Chunk size for a shard: what a rank's slot is rounded up to. About one chunk for each of the `resident`
 // CTAs that a device holds at once per rank (NANGILA_LAYOUT_CTAS), not below 4096 elements except for shards of less than four
 // such chunks. The same on every rank, whatever its device: peers write into one another's slots.
 extern "C" int32_t nangila_ag_chunk_elems(int64_t shard_elems, int32_t resident) {

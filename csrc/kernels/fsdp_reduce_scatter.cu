@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "bucket_slots.cuh"
+#include "fsdp_grid.cuh"
 #include "fsdp_reduce_scatter.cuh"
 #include "meet.cuh"
 #include "nangila_kernels.h"
@@ -53,13 +54,11 @@ struct RsShape {
 template <typename T, typename S>
 constexpr bool kPackedBf16 = std::is_same_v<T, __nv_bfloat16> && std::is_same_v<S, __nv_bfloat16>;
 
-// LOOP: the launch has fewer CTAs than tiles. (The loop's invariants cost registers; without it 64 are enough for four CTAs an SM.)
-template <typename T, typename S, bool EF, bool LOOP>
-__global__ void __launch_bounds__(kThreads, LOOP ? 2 : kPackedBf16<T, S> && !EF ? 6 : 4) rs_quantize_kernel(const __grid_constant__ NangilaPredResParams p, const __grid_constant__ RsShape sh) {
+// (A loop's invariants cost registers; without one 64 are enough for four CTAs an SM.)
+template <typename T, typename S, bool EF, Walk WALK>
+__global__ void __launch_bounds__(kThreads, WALK != kNoWalk ? 2 : kPackedBf16<T, S> && !EF ? 6 : 4) rs_quantize_kernel(const __grid_constant__ NangilaPredResParams p, const __grid_constant__ RsShape sh) {
   may_follow();
   const int vr = blockIdx.z, me = p.rank0 + vr, W = sh.W, C = sh.C, tid = threadIdx.x;
-  int o = me + 1 + int(blockIdx.y);  // remote owners first, this rank's own shard last
-  if (o >= W) o -= W;
   // A rank that has failed does nothing more. The word is looked at when the first data are there, so it costs no latency.
   const uint32_t failed = *reinterpret_cast<volatile uint32_t*>(&p.status[vr][kStatusCode]);
   const T* __restrict__ grad = static_cast<const T*>(p.grad[vr]);
@@ -67,86 +66,92 @@ __global__ void __launch_bounds__(kThreads, LOOP ? 2 : kPackedBf16<T, S> && !EF 
   const bool has_ef = EF && ef != nullptr;
   const uint32_t key = make_key(p.seed, p.step, p.bucket_id, uint32_t(me), 1u);
   const bool stochastic = p.stochastic != 0;
-  int tile = blockIdx.x;
+  int d = blockIdx.y;
   do {
-    const int j = int(unsigned(tile) / unsigned(sh.sub)), it0 = (tile - j * sh.sub) * kTile;
-    const int64_t first = int64_t(o) * sh.shard + int64_t(j) * C, limit = int64_t(o + 1) * sh.shard;
-    const bool whole = first + C <= limit;
-    uint8_t* dst = p.region[o] + sh.recv + (uint64_t(j) * W + me) * sh.slot;
-    const int64_t at0 = first + int64_t(it0) * kElemsPerIter + tid * kE;  // this lane's first element
-    const int left = min(kTile, sh.iters - it0);                          // iterations of this tile
-    const T* g0 = grad + at0;
-    S* e0 = ef + at0;  // (not used where there is no error memory)
+    int o = me + 1 + d;  // remote owners first, this rank's own shard last
+    if (o >= W) o -= W;
+    int tile = blockIdx.x;
+    do {
+      const int j = int(unsigned(tile) / unsigned(sh.sub)), it0 = (tile - j * sh.sub) * kTile;
+      const int64_t first = int64_t(o) * sh.shard + int64_t(j) * C, limit = int64_t(o + 1) * sh.shard;
+      const bool whole = first + C <= limit;
+      uint8_t* dst = p.region[o] + sh.recv + (uint64_t(j) * W + me) * sh.slot;
+      const int64_t at0 = first + int64_t(it0) * kElemsPerIter + tid * kE;  // this lane's first element
+      const int left = min(kTile, sh.iters - it0);                          // iterations of this tile
+      const T* g0 = grad + at0;
+      S* e0 = ef + at0;  // (not used where there is no error memory)
       uint32_t* codes = packed_ptr(dst, C, it0, tid);
-    uint16_t* scales = scale_ptr(dst, C, it0, tid);
-    auto put = [&](int b, uint32_t packed, uint32_t scale) {
-      codes[b * 32] = packed;
-      if ((tid & (kLanes8 - 1)) == 0) scales[b * 4] = uint16_t(scale);
-    };
-    // eight values in FP32; e: the error memory
-    auto fp32 = [&](auto guard, int b, float (&g)[kE], float (&e)[kE]) {
-      constexpr bool GUARD = decltype(guard)::value;
+      uint16_t* scales = scale_ptr(dst, C, it0, tid);
+      auto put = [&](int b, uint32_t packed, uint32_t scale) {
+        codes[b * 32] = packed;
+        if ((tid & (kLanes8 - 1)) == 0) scales[b * 4] = uint16_t(scale);
+      };
+      // eight values in FP32; e: the error memory
+      auto fp32 = [&](auto guard, int b, float (&g)[kE], float (&e)[kE]) {
+        constexpr bool GUARD = decltype(guard)::value;
 #pragma unroll
-      for (int i = 0; i < kE; ++i) e[i] = has_ef ? e[i] + sanitize(g[i]) : sanitize(g[i]);
-      uint32_t packed, scale;
-      quantize8(e, key, uint32_t((at0 + b * kElemsPerIter) >> 1), stochastic, packed, scale);
-      if (has_ef) store8<S, GUARD>(e0, b * kElemsPerIter, limit - at0, e);
-      put(b, packed, scale);
-    };
-    auto fp32_tile = [&](auto guard) {
-      constexpr bool GUARD = decltype(guard)::value;
-      constexpr int kBatch = 2;
+        for (int i = 0; i < kE; ++i) e[i] = has_ef ? e[i] + sanitize(g[i]) : sanitize(g[i]);
+        uint32_t packed, scale;
+        quantize8(e, key, uint32_t((at0 + b * kElemsPerIter) >> 1), stochastic, packed, scale);
+        if (has_ef) store8<S, GUARD>(e0, b * kElemsPerIter, limit - at0, e);
+        put(b, packed, scale);
+      };
+      auto fp32_tile = [&](auto guard) {
+        constexpr bool GUARD = decltype(guard)::value;
+        constexpr int kBatch = 2;
 #pragma unroll 1
-      for (int b0 = 0; b0 < left; b0 += kBatch) {
-        float g[kBatch][kE], e[kBatch][kE];
+        for (int b0 = 0; b0 < left; b0 += kBatch) {
+          float g[kBatch][kE], e[kBatch][kE];
 #pragma unroll
-        for (int b = 0; b < kBatch; ++b)
-          if (b0 + b < left) {
-            load8<T, GUARD>(g0, (b0 + b) * kElemsPerIter, limit - at0, g[b]);
-            if (has_ef) load8<S, GUARD>(e0, (b0 + b) * kElemsPerIter, limit - at0, e[b]);
+          for (int b = 0; b < kBatch; ++b)
+            if (b0 + b < left) {
+              load8<T, GUARD>(g0, (b0 + b) * kElemsPerIter, limit - at0, g[b]);
+              if (has_ef) load8<S, GUARD>(e0, (b0 + b) * kElemsPerIter, limit - at0, e[b]);
+            }
+          if (failed != 0u) return;
+#pragma unroll
+          for (int b = 0; b < kBatch; ++b)
+            if (b0 + b < left) fp32(guard, b0 + b, g[b], e[b]);
+        }
+      };
+      if (!whole) {
+        fp32_tile(std::true_type{});
+      } else if constexpr (kPackedBf16<T, S>) {
+        uint4 g[kTile], e[kTile];
+#pragma unroll
+        for (int b = 0; b < kTile; ++b) {
+          if (b < left) {
+            g[b] = *reinterpret_cast<const uint4*>(g0 + b * kElemsPerIter);
+            if (has_ef) e[b] = *reinterpret_cast<const uint4*>(e0 + b * kElemsPerIter);
           }
+        }
         if (failed != 0u) return;
 #pragma unroll
-        for (int b = 0; b < kBatch; ++b)
-          if (b0 + b < left) fp32(guard, b0 + b, g[b], e[b]);
-      }
-    };
-    if (!whole) {
-      fp32_tile(std::true_type{});
-    } else if constexpr (kPackedBf16<T, S>) {
-      uint4 g[kTile], e[kTile];
+        for (int b = 0; b < kTile; ++b) {
+          if (b >= left) break;
+          const uint32_t gw[4] = {g[b].x, g[b].y, g[b].z, g[b].w}, ew[4] = {e[b].x, e[b].y, e[b].z, e[b].w};
+          uint32_t x[4];
 #pragma unroll
-      for (int b = 0; b < kTile; ++b) {
-        if (b < left) {
-          g[b] = *reinterpret_cast<const uint4*>(g0 + b * kElemsPerIter);
-          if (has_ef) e[b] = *reinterpret_cast<const uint4*>(e0 + b * kElemsPerIter);
+          for (int k = 0; k < 4; ++k) x[k] = has_ef ? as_u32(__hadd2(as_bf162(gw[k]), as_bf162(ew[k]))) : gw[k];
+          if (__any_sync(0xffffffffu, maybe_nonfinite8(x))) {  // a NaN / Inf in the warp's slice (or magnitudes >= 2): sanitised in FP32
+            float gf[kE], err[kE];
+            words_to_float8(gw, gf);
+            words_to_float8(ew, err);
+            fp32(std::false_type{}, b, gf, err);
+            continue;
+          }
+          uint32_t packed, scale, qs[4];
+          quantize8_bf16(x, packed, scale, qs);
+          if (has_ef) *reinterpret_cast<uint4*>(e0 + b * kElemsPerIter) = make_uint4(x[0], x[1], x[2], x[3]);
+          put(b, packed, scale);
         }
+      } else {
+        fp32_tile(std::false_type{});
       }
-      if (failed != 0u) return;
-#pragma unroll
-      for (int b = 0; b < kTile; ++b) {
-        if (b >= left) break;
-        const uint32_t gw[4] = {g[b].x, g[b].y, g[b].z, g[b].w}, ew[4] = {e[b].x, e[b].y, e[b].z, e[b].w};
-        uint32_t x[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) x[k] = has_ef ? as_u32(__hadd2(as_bf162(gw[k]), as_bf162(ew[k]))) : gw[k];
-        if (__any_sync(0xffffffffu, maybe_nonfinite8(x))) {  // a NaN / Inf in the warp's slice (or magnitudes >= 2): sanitised in FP32
-          float gf[kE], err[kE];
-          words_to_float8(gw, gf);
-          words_to_float8(ew, err);
-          fp32(std::false_type{}, b, gf, err);
-          continue;
-        }
-        uint32_t packed, scale, qs[4];
-        quantize8_bf16(x, packed, scale, qs);
-        if (has_ef) *reinterpret_cast<uint4*>(e0 + b * kElemsPerIter) = make_uint4(x[0], x[1], x[2], x[3]);
-        put(b, packed, scale);
-      }
-    } else {
-      fp32_tile(std::false_type{});
-    }
-    tile += gridDim.x;
-  } while (LOOP && tile < sh.tiles);
+      tile += gridDim.x;
+    } while (WALK != kNoWalk && tile < sh.tiles);
+    d += gridDim.y;
+  } while (WALK == kWalkGroups && d < W);
 }
 
 template <typename T, bool PACKED>
@@ -219,29 +224,29 @@ __global__ void __launch_bounds__(kThreads, 4) rs_sum_kernel(const __grid_consta
 }
 
 template <typename T, typename S, bool EF>
-void launch_quantize(const NangilaPredResParams& p, const RsShape& sh, dim3 grid, cudaStream_t stream) {
-  if (grid.x < unsigned(sh.tiles)) rs_quantize_kernel<T, S, EF, true><<<grid, kThreads, 0, stream>>>(p, sh);
-  else rs_quantize_kernel<T, S, EF, false><<<grid, kThreads, 0, stream>>>(p, sh);
+void launch_quantize(const NangilaPredResParams& p, const RsShape& sh, cudaStream_t stream) {
+  const FsdpGrid g = fsdp_grid(sh.tiles, p.world, p.grid_x);
+  const dim3 grid(g.x, g.y, unsigned(p.nvr));
+  if (g.walk == kNoWalk) rs_quantize_kernel<T, S, EF, kNoWalk><<<grid, kThreads, 0, stream>>>(p, sh);
+  else if (g.walk == kWalkTiles) rs_quantize_kernel<T, S, EF, kWalkTiles><<<grid, kThreads, 0, stream>>>(p, sh);
+  else rs_quantize_kernel<T, S, EF, kWalkGroups><<<grid, kThreads, 0, stream>>>(p, sh);
 }
 
 template <typename T, typename S>
 cudaError_t launch(const NangilaPredResParams& p, cudaStream_t stream) {
   const int64_t sub = (p.chunk_elems / kElemsPerIter + kTile - 1) / kTile, all = p.nchunks / p.world * sub;
-  if (all > 0x3fffffff) return cudaErrorInvalidValue;
+  if (all > kMaxTiles) return cudaErrorInvalidValue;
   const RsShape sh(p);
-  // fewer CTAs than chunks asked for: a cap for all destinations together
-  const int cap = p.grid_x > 0 && p.grid_x < p.nchunks ? p.grid_x : 0;
   const int phases = (p.phase_mask & 7) == 0 ? 7 : p.phase_mask;
   if (phases & 1) {
     bool ef = false;
     for (int v = 0; v < p.nvr; ++v) ef = ef || p.ef[v] != nullptr;
-    const dim3 grid(unsigned(cap > 0 ? std::min(sh.tiles, std::max(1, cap / p.world)) : sh.tiles), unsigned(p.world), unsigned(p.nvr));
-    if (ef) launch_quantize<T, S, true>(p, sh, grid, stream);
-    else launch_quantize<T, S, false>(p, sh, grid, stream);
+    if (ef) launch_quantize<T, S, true>(p, sh, stream);
+    else launch_quantize<T, S, false>(p, sh, stream);
   }
   if (phases & 2) {
     cudaError_t e = cudaGetLastError();
-    const dim3 grid(unsigned(cap > 0 ? std::min(sh.tiles, cap) : sh.tiles), unsigned(p.nvr));
+    const dim3 grid(fsdp_grid(sh.tiles, 1, p.grid_x).x, unsigned(p.nvr));
     if (e == cudaSuccess) e = launch_meet(p, p.flag1_off, kTimeoutPhase2, 2u, int64_t(grid.x) * grid.y, stream);
     if (e != cudaSuccess) return e;
     return launch_following(rs_sum_kernel<T, kPackedBf16<T, S>>, grid, kThreads, 0, stream, p, sh);
@@ -262,6 +267,13 @@ cudaError_t launch_reduce_scatter(const NangilaPredResParams& p, cudaStream_t st
 }
 
 }  // namespace nangila
+
+extern "C" int32_t nangila_fsdp_grid(int64_t tiles, int32_t groups, int32_t cap, uint32_t* x, uint32_t* y) {
+  const nangila::FsdpGrid g = nangila::fsdp_grid(tiles, groups, cap);
+  *x = g.x;
+  *y = g.y;
+  return int32_t(g.walk);
+}
 
 // The slots of both parities and the flag words (one per rank is used; a region has room for one per chunk).
 extern "C" uint64_t nangila_rs_region_bytes(int64_t n, int32_t world, int32_t chunk_elems, uint64_t* recv1_off,

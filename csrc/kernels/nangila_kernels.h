@@ -27,10 +27,11 @@ enum NangilaDType { NANGILA_F32 = 0, NANGILA_F16 = 1, NANGILA_BF16 = 2 };
  * warm-up, Safe-Mode fallback and forced re-synchronisation, and also maintains the history.
  *
  * Multi-GPU: nvr = 1, rank0 = this rank, `region[r]` = rank r's mapping of the bucket's symmetric
- * region. Single-GPU loopback: nvr = world, rank0 = 0, grid.y = nvr, launched cooperatively.
+ * region. Single-GPU loopback: nvr = world, rank0 = 0, grid.y = nvr, launched cooperatively (modes 0 and 1).
  * grid_x is clamped to the number of CTAs of the chosen variant that the device can hold at once
  * (occupancy x SM count, divided by nvr); grid_x <= 0 asks for exactly that number. The reduce-scatter (mode 2) has kernels of its
- * own that need no residency: there grid_x below nchunks is a cap, anything else means as many CTAs as there is work for.
+ * own that need no residency and are not launched cooperatively: there a rank gets as many CTAs as there is work for, and with
+ * grid_x > 0 no more than that many in any of them. The all-gather's grid_x means the same.
  */
 typedef struct NangilaPredResParams {
   void* grad[NANGILA_MAX_VRANKS];      /* in/out: bucket, n elements of grad_dtype */
@@ -107,6 +108,9 @@ typedef struct NangilaAgParams {
 uint64_t nangila_ag_region_bytes(int64_t shard_elems, int32_t world, int32_t chunk_elems, int32_t bits,
                                  uint64_t* recv_off, uint64_t* flag_off);
 int32_t nangila_ag_chunk_elems(int64_t shard_elems, int32_t resident_ctas);
+/* The grid of such a launch: `groups` (destinations, owners) of `tiles` tiles under a cap. Returns 0 (a tile to a CTA), 1 (the CTAs walk their
+ * group's tiles) or 2 (fewer CTAs than groups: they walk the groups too). */
+int32_t nangila_fsdp_grid(int64_t tiles, int32_t groups, int32_t cap, uint32_t* x, uint32_t* y);
 int nangila_ag_launch(const NangilaAgParams* p, cudaStream_t stream);
 
 /* ---- PowerSGD on tcgen05 tensor cores (powersgd_tcgen05.cu) ------------------------------------------------ */

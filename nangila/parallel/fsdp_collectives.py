@@ -51,9 +51,8 @@ class _Base:
         self.launches = 0
         self.fallbacks = 0
         self._glue = None
-        # CTAs per launch (NANGILA_FSDP_CTAS; 0: as many as there are chunks, clamped by the launcher to what the device
-        # holds at once). The collectives overlap with the layers' compute, so a cap trades their own speed for the SMs
-        # they take from it.
+        # Most CTAs of a rank in any launch (NANGILA_FSDP_CTAS; 0: as many as there is work for). The collectives overlap with the
+        # layers' compute, so a cap trades their own speed for the SMs they take from it.
         self.ctas = int(os.environ.get("NANGILA_FSDP_CTAS", "0"))
 
     def _ensure(self, device: torch.device, group: Optional[dist.ProcessGroup]):
@@ -192,9 +191,7 @@ class NangilaReduceScatter(_Base, ReduceScatter):
         key = (n, inputs[0].dtype)
         st = self._regions.get(key)
         if st is None:
-            # Phase 2 has one task per chunk of this rank's shard: the chunk size is chosen so that those tasks fill
-            # the CTAs a whole device holds at once in whole waves (256 chunks of 64 K elements per shard left more than
-            # half of them idle in that phase)
+            # a function of the size alone (see NANGILA_LAYOUT_CTAS): slots are laid out by chunks, whole chunks go through packed BF16
             env = os.environ.get("NANGILA_CHUNK")
             resident = max(1, self._glue.LAYOUT_CTAS // self.nvr)
             chunk = int(env) if env else int(self._glue.predres_chunk_elems(n // self.world, resident))
@@ -206,11 +203,9 @@ class NangilaReduceScatter(_Base, ReduceScatter):
         ef = u.ef if u.ef is not None else [None] * self.nvr
         st["epoch"] += 1
         self.launches += 1
-        cps = st["nchunks"] // self.world
         self._glue.rs_launch(inputs, outputs, ef, self._status, st["region"].ptrs, st["r1"], st["f1"], st["nchunks"],
                              0 if self.loopback else self.rank, st["chunk"], self.stochastic, st["epoch"], self.seed,
-                             self.step + u.calls, u.index, scale, self.timeout_s,
-                             max(1, min(cps * self.world, self.ctas) if self.ctas > 0 else cps * self.world))
+                             self.step + u.calls, u.index, scale, self.timeout_s, max(0, self.ctas))
 
     def _reduce_predicted(self, u: _RsUnit, outputs: List[torch.Tensor], inputs: List[torch.Tensor], scale: float) -> None:
         from .predres_engine import PredResEngine
@@ -294,10 +289,9 @@ class NangilaAllGather(_Base, AllGather):
             self._regions[key] = st
         st["epoch"] += 1
         self.launches += 1
-        cps = (shard + st["chunk"] - 1) // st["chunk"]
         self._glue.ag_launch(inputs, outputs, self._status, st["region"].ptrs, st["r"], st["f"],
                              0 if self.loopback else self.rank, st["chunk"], self.bits, st["epoch"], self.timeout_s,
-                             max(1, min(cps * (self.world + 1), self.ctas) if self.ctas > 0 else cps * (self.world + 1)))
+                             max(0, self.ctas))
 
     def __call__(self, output_tensor: torch.Tensor, input_tensor: torch.Tensor, group: dist.ProcessGroup,
                  async_op: bool = False):
