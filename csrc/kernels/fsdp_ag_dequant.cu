@@ -7,8 +7,8 @@
 // The owner of a shard also consumes the dequantized form of its own shard, so all ranks compute
 // with bit-identical parameters. Rounding is to nearest (parameters must not pick up random noise).
 //
-// Three launches, one behind the other: ag_quantize (codes to the peers, this rank's own part of the result; it may be the
-// buffer the shard is read from), the meeting of the ranks (meet.cuh), ag_expand (the other ranks' parts). Grids of short CTAs
+// One behind the other: ag_quantize (codes to the peers, this rank's own part of the result; it may be the
+// buffer the shard is read from), the meeting of the ranks (a kernel, or the start of the next one: meet.cuh), ag_expand (the other ranks' parts). Grids of short CTAs
 // without flags or fences that the hardware hands out as SMs come free.
 // What bounds them: HBM and L2 traffic. Measured on B200, four ranks on one device, 3.1 M bf16 elements each, INT8 (25 MB in, 39 MB of codes, 100 MB
 // out): 17 us (5.2 TB/s) + 21 us (5.5 TB/s), 42.4 us for the call; as one resident kernel with block barriers and a flag per chunk 49.3 us.
@@ -57,6 +57,10 @@ template <int BITS>
 using Packed = std::conditional_t<BITS == 8, uint2, uint32_t>;  // eight codes
 
 constexpr int kTile = 4;  // iterations of 2048 elements whose loads are issued together
+// A small shard is quantized in tiles of one iteration: a CTA's four, one behind the other, are then what the call waits for. us a call, tiles of four / of
+// one: 131 072 elements, one rank of eight, bf16 8.3 / 6.9, fp32 10.3 / 8.2; four emulated ranks of as many fp32 elements (256 CTAs) 10.1 / 8.3,
+// of twice as many 11.3 / 12.9.
+constexpr int64_t kSmallCtas = 2 * 148;
 
 // A rank's shard in the exchange region: its codes one behind the other, then its scales. Worked out on the host: the number of chunks is a
 // division of 64-bit numbers, which costs a thread more than quantizing eight elements.
@@ -113,8 +117,8 @@ __device__ __forceinline__ void expand8(const Packed<BITS>& w, uint16_t scale, T
   }
 }
 
-template <typename T, int BITS>
-__global__ void __launch_bounds__(kThreads, 5) ag_quantize_kernel(const __grid_constant__ NangilaAgParams p, const __grid_constant__ AgShape sh) {
+template <typename T, int BITS, int TILE>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 4 : 5) ag_quantize_kernel(const __grid_constant__ NangilaAgParams p, const __grid_constant__ AgShape sh) {
   may_follow();
   const int vr = blockIdx.y, me = p.rank0 + vr, W = p.world, tid = threadIdx.x;
   const int total = int((p.shard_elems + kPerIter - 1) / kPerIter);
@@ -123,16 +127,16 @@ __global__ void __launch_bounds__(kThreads, 5) ag_quantize_kernel(const __grid_c
   const T* in = static_cast<const T*>(p.in_shard[vr]);
   T* own = static_cast<T*>(p.out_full[vr]) + int64_t(me) * p.shard_elems;  // may be `in`: a lane writes where it has read
   constexpr float kInvQmax = BITS == 8 ? 0.0078740157f : 0.14285715f;
-  for (int it0 = blockIdx.x * kTile; it0 < total; it0 += gridDim.x * kTile) {
+  for (int it0 = blockIdx.x * TILE; it0 < total; it0 += gridDim.x * TILE) {
     const int64_t at0 = int64_t(it0) * kPerIter + tid * kE, left = p.shard_elems - at0;  // the shard is a multiple of 8: a lane has eight values or none
-    Raw<T> raw[kTile];
+    Raw<T> raw[TILE];
 #pragma unroll
-    for (int b = 0; b < kTile; ++b) raw[b] = b * kPerIter < left ? *reinterpret_cast<const Raw<T>*>(in + at0 + b * kPerIter) : Raw<T>{};
+    for (int b = 0; b < TILE; ++b) raw[b] = b * kPerIter < left ? *reinterpret_cast<const Raw<T>*>(in + at0 + b * kPerIter) : Raw<T>{};
     if (failed != 0u) return;
-    Packed<BITS> w[kTile];
-    uint16_t sb[kTile];
+    Packed<BITS> w[TILE];
+    uint16_t sb[TILE];
 #pragma unroll
-    for (int b = 0; b < kTile; ++b) {
+    for (int b = 0; b < TILE; ++b) {
       float x[kE], amax = 0.0f;
       bool clean = false;
       if constexpr (std::is_same_v<T, __nv_bfloat16>) {
@@ -179,7 +183,7 @@ __global__ void __launch_bounds__(kThreads, 5) ag_quantize_kernel(const __grid_c
       Packed<BITS>* codes = reinterpret_cast<Packed<BITS>*>(p.region[r] + slot.codes);
       uint16_t* scales = reinterpret_cast<uint16_t*>(p.region[r] + slot.scales);
 #pragma unroll
-      for (int b = 0; b < kTile; ++b) {
+      for (int b = 0; b < TILE; ++b) {
         if (it0 + b < total) {
           codes[b * kThreads] = w[b];
           if ((tid & 7) == 0) scales[b * (kPerIter / kQuantBlock)] = sb[b];
@@ -188,16 +192,17 @@ __global__ void __launch_bounds__(kThreads, 5) ag_quantize_kernel(const __grid_c
     }
     // this rank's own part of the result: what the others make of the codes
 #pragma unroll
-    for (int b = 0; b < kTile; ++b)
+    for (int b = 0; b < TILE; ++b)
       if (b * kPerIter < left) expand8<T, BITS>(w[b], sb[b], own + at0 + b * kPerIter);
   }
 }
 
-template <typename T, int BITS, bool ALL>  // ALL: there are fewer CTAs than owners, so one takes several of these
-__global__ void __launch_bounds__(kThreads, 8) ag_expand_kernel(const __grid_constant__ NangilaAgParams p, const __grid_constant__ AgShape sh, int tiles) {
+template <typename T, int BITS, Met MET, bool ALL>  // ALL: there are fewer CTAs than owners, so one takes several of these
+__global__ void __launch_bounds__(kThreads, MET == kMetBefore ? 8 : 4) ag_expand_kernel(const __grid_constant__ NangilaAgParams p, const __grid_constant__ AgShape sh, int tiles) {
   const int vr = blockIdx.z, me = p.rank0 + vr, W = p.world, tid = threadIdx.x;
   follow();
-  const uint32_t failed = *reinterpret_cast<volatile uint32_t*>(&p.status[vr][kStatusCode]);  // not 0: a rank's data did not come
+  uint32_t seen;
+  if (!arrive<MET>(p, vr, p.flag_off, kTimeoutPhase3, 3u, seen)) return;
   const uint8_t* myreg = p.region[me];
   int d = blockIdx.y;
   do {
@@ -218,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 8) ag_expand_kernel(const __grid_con
           sc[b] = scales[b * (kPerIter / kQuantBlock)];
         }
       }
-      if (failed != 0u) return;
+      if (!all_came<MET>(p, vr, seen, kTimeoutPhase3, 3u)) return;
 #pragma unroll
       for (int b = 0; b < kTile; ++b)
         if (b * kPerIter < left) expand8<T, BITS>(w[b], sc[b], out + at0 + b * kPerIter);
@@ -232,12 +237,15 @@ cudaError_t launch(const NangilaAgParams& p, cudaStream_t stream) {
   const int64_t total = (p.shard_elems + kPerIter - 1) / kPerIter, tiles = (total + kTile - 1) / kTile;
   if (tiles > kMaxTiles) return cudaErrorInvalidValue;
   const AgShape sh(p, BITS);
-  ag_quantize_kernel<T, BITS><<<dim3(fsdp_grid(tiles, 1, p.grid_x).x, unsigned(p.nvr)), kThreads, 0, stream>>>(p, sh);
+  if (total * p.nvr <= kSmallCtas) ag_quantize_kernel<T, BITS, 1><<<dim3(fsdp_grid(total, 1, p.grid_x).x, unsigned(p.nvr)), kThreads, 0, stream>>>(p, sh);
+  else ag_quantize_kernel<T, BITS, kTile><<<dim3(fsdp_grid(tiles, 1, p.grid_x).x, unsigned(p.nvr)), kThreads, 0, stream>>>(p, sh);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || p.world == 1) return e;
-  if ((e = launch_meet(p, p.flag_off, kTimeoutPhase3, 3u, kMeetlessCtas + 1, stream)) != cudaSuccess) return e;
   const FsdpGrid g = fsdp_grid(tiles, p.world - 1, p.grid_x);
-  auto* expand = g.walk == kWalkGroups ? ag_expand_kernel<T, BITS, true> : ag_expand_kernel<T, BITS, false>;
+  const Met met = how_to_meet(p, int64_t(g.x) * g.y * p.nvr, 4 * 148);
+  if ((e = launch_meet(p, met, p.flag_off, kTimeoutPhase3, 3u, stream)) != cudaSuccess) return e;
+  auto* expand = met == kMetInLaunch ? ag_expand_kernel<T, BITS, kMetInLaunch, true> : met == kMeetHere ? ag_expand_kernel<T, BITS, kMeetHere, true>
+                 : g.walk == kWalkGroups ? ag_expand_kernel<T, BITS, kMetBefore, true> : ag_expand_kernel<T, BITS, kMetBefore, false>;
   return launch_following(expand, dim3(g.x, g.y, unsigned(p.nvr)), kThreads, 0, stream, p, sh, int(tiles));
 }
 

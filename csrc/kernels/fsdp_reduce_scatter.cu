@@ -1,9 +1,9 @@
 // Compressed gradient reduce-scatter for fully-sharded training (sm_100a). Rank o owns shard o of the bucket (W equal shards, cut
-// into chunks of chunk_elems). Three launches, one behind the other:
+// into chunks of chunk_elems). One behind the other:
 //
 //   rs_quantize   x = g + error memory, block-INT4 codes and scales of every chunk stored into the owner's slot [chunk][me] over
 //                 NVLink, new error memory
-//   meet          every rank's codes are in place (meet.cuh)
+//   meeting       every rank's codes are in place: a kernel of its own, or the start of the next one (meet.cuh)
 //   rs_sum        the sum of the W contributions of this rank's shard times out_scale
 //
 // Grids of short CTAs without flags, fences or residency that the hardware hands out as SMs come free. Slots alternate between two sets
@@ -154,12 +154,13 @@ __global__ void __launch_bounds__(kThreads, WALK != kNoWalk ? 2 : kPackedBf16<T,
   } while (WALK == kWalkGroups && d < W);
 }
 
-template <typename T, bool PACKED>
+template <typename T, bool PACKED, Met MET>
 __global__ void __launch_bounds__(kThreads, 4) rs_sum_kernel(const __grid_constant__ NangilaPredResParams p, const __grid_constant__ RsShape sh) {
   const int vr = blockIdx.y, me = p.rank0 + vr, W = sh.W, C = sh.C, tid = threadIdx.x;
   uint8_t* myreg = p.region[me];
   follow();
-  const uint32_t seen = status_seen(p);
+  uint32_t seen;
+  if (!arrive<MET>(p, vr, p.flag1_off, kTimeoutPhase2, 2u, seen)) return;
   T* __restrict__ out = static_cast<T*>(p.out_shard[vr]);
   for (int tile = blockIdx.x; tile < sh.tiles; tile += gridDim.x) {
     const int j = int(unsigned(tile) / unsigned(sh.sub)), it0 = (tile - j * sh.sub) * kTile;
@@ -193,7 +194,7 @@ __global__ void __launch_bounds__(kThreads, 4) rs_sum_kernel(const __grid_consta
           dequant8_bf16_fma2(packed[b], __floats2bfloat162_rn(s, s), acc[b]);
         }
       }
-      if (!all_came(p, vr, seen, kTimeoutPhase2, 2u)) return;
+      if (!all_came<MET>(p, vr, seen, kTimeoutPhase2, 2u)) return;
 #pragma unroll
       for (int b = 0; b < kTile; ++b)
         if (b < left) *reinterpret_cast<uint4*>(out + at0 + b * kElemsPerIter) = make_uint4(acc[b][0], acc[b][1], acc[b][2], acc[b][3]);
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(kThreads, 4) rs_sum_kernel(const __grid_consta
 #pragma unroll
           for (int b = 0; b < kBatch; ++b) dequant8_add(packed[b], bf16_bits_to_float(scale[b]), acc[b]);
         }
-        if (!all_came(p, vr, seen, kTimeoutPhase2, 2u)) return;
+        if (!all_came<MET>(p, vr, seen, kTimeoutPhase2, 2u)) return;
 #pragma unroll
         for (int b = 0; b < kBatch; ++b)
           if (b0 + b < left) {
@@ -247,9 +248,12 @@ cudaError_t launch(const NangilaPredResParams& p, cudaStream_t stream) {
   if (phases & 2) {
     cudaError_t e = cudaGetLastError();
     const dim3 grid(fsdp_grid(sh.tiles, 1, p.grid_x).x, unsigned(p.nvr));
-    if (e == cudaSuccess) e = launch_meet(p, p.flag1_off, kTimeoutPhase2, 2u, int64_t(grid.x) * grid.y, stream);
+    const Met met = how_to_meet(p, int64_t(grid.x) * grid.y, 8 * 148);
+    if (e == cudaSuccess) e = launch_meet(p, met, p.flag1_off, kTimeoutPhase2, 2u, stream);
     if (e != cudaSuccess) return e;
-    return launch_following(rs_sum_kernel<T, kPackedBf16<T, S>>, grid, kThreads, 0, stream, p, sh);
+    constexpr bool PACKED = kPackedBf16<T, S>;
+    auto* sum = met == kMetBefore ? rs_sum_kernel<T, PACKED, kMetBefore> : met == kMetInLaunch ? rs_sum_kernel<T, PACKED, kMetInLaunch> : rs_sum_kernel<T, PACKED, kMeetHere>;
+    return launch_following(sum, grid, kThreads, 0, stream, p, sh);
   }
   return cudaGetLastError();
 }
