@@ -184,30 +184,43 @@ __global__ void __launch_bounds__(T) spmv_row_blocks_bulk_kernel(const int* __re
 // that ladders and meshes keep their bits. Measured on B200, staged kernel and this one, repeated products (10^6 rows lie in L2, 4 10^6 do not):
 // ladder of 10^6 rows 24 -> 14 us, of 4 10^6 59 -> 41 us (5.5 TB/s); mesh of 10^6 nodes 35 -> 19, of 4 10^6 100 -> 56 us. With nothing in L2:
 // rows of 1, 3, 5, 6 entries near the diagonal, 10^6 rows: 23 -> 16, 39 -> 23, 52 -> 35, 55 -> 39 us; anywhere: 31 -> 17, 56 -> 28, 77 -> 39, 83 -> 45.
-// While the row pointers are on their way, a row's part of the values, columns and x is fetched into L2 from where it would lie if all rows were of the
-// same length (`mean` > 0): everything there is wanted by some row soon, so a guess that is off costs nothing. us, without / with it, three matrices in turn and
-// one again and again: ladder of 10^6 rows 11.9 / 10.4, 6.0 / 6.5; mesh of 10^6 18.0 / 15.3, 11.3 / 11.8; ladder of 4 10^6 38.1 / 33.4 either
-// way, mesh 58.3 / 48.3. Where everything lies in L2 the fetches are only in the way: ladder of 4 10^5 (22 MB) 3.5 / 3.8, mesh of 4 10^5 (35 MB) 7.3 / 7.3,
-// ladder of 7 10^5 (39 MB) 8.6 / 7.8 and 4.6 / 5.0. So: above 40 MB, where a product that finds its matrix in memory gains more than
-// one that finds it in L2 loses. (Two rows a thread instead: no gain, four: 16 % slower; one fetch per line by fewer lanes: slower than a lane for each row.)
+// While the row pointers are on their way, a thread of each CTA has L2 fetch what the CTA would need if all rows were of the same length (`mean`): whole
+// lines in one bulk prefetch, which every CTA's neighbours want soon if the guess is off. The columns alone, since these are what x waits for, or all of it.
+// us without it / as chosen, in captured products: matrices in turn, and one again and again:
+//   columns: ladder of 10^6 rows (55 MB)   12.0 / 11.3,  5.9 / 6.1     mesh of 10^6 (79 MB)     18.3 / 17.6,  11.6 / 11.6
+//   all:     ladder of 4 10^6 (223 MB)     38.4 / 34.3,  38.1 / 33.9   mesh of 4 10^6 (319 MB)  59.4 / 54.7,  59.4 / 51.2
+// So all of it where the matrix is larger than L2; the columns where a product may find it there or not (all of it there: 10.3, 7.0 and 17.0, 12.5 for the
+// first line); nothing below 40 MB, where there is hardly anything to gain. (A prefetch by every row's thread for its own entries cost a product that
+// finds its matrix in L2 more and gained less elsewhere: 11.3, 6.8 and 17.3, 11.8; 36.9, 36.1 and 60.0, 59.2.)
 //
 // The rule: no row above 16 entries, and at most 6 on average. Uneven rows cost a warp the time of its longest; at the corner of the rule
 // (rows of 1 and of 16, mean 6) what is left is 43.5 -> 41.4 us near the diagonal and 150 -> 142 for 4 10^6 rows, so longer rows and higher means
 // stay with the staged kernel; within it this kernel was the faster one for means 1 to 6, even and uneven, 10^4 to 4 10^6 rows.
 constexpr int kShortRow = 16;
 constexpr int kShortMean = 6;
-constexpr int64_t kFetchAhead = 40000000;  // bytes of matrix and vectors
+enum Ahead { kNothing, kColumns, kAll };
+constexpr int64_t kColumnsAhead = 40000000, kAllAhead = 126 << 20;  // bytes of matrix and vectors
+template <Ahead AHEAD>
 __global__ void __launch_bounds__(kThreads) spmv_short_rows_kernel(const int* __restrict__ row_ptr, const int* __restrict__ col,
                                                                    const double* __restrict__ val, const double* __restrict__ x,
                                                                    double* __restrict__ y, int n, int nnz, float mean) {
     const int r = int(blockIdx.x * unsigned(kThreads) + threadIdx.x);
     if (unsigned(r) >= unsigned(n)) return;
-    if (mean > 0.0f) {
-        const int64_t guess = max(min(int64_t(float(r) * mean), int64_t(nnz) - 1), int64_t(0));  // (the arrays have room for four entries at least)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(val + guess));
-        if ((threadIdx.x & 1) == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(col + guess));
-        if ((threadIdx.x & 15) == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(x + r));
+    if (AHEAD != kNothing && threadIdx.x == 0) {
+        const int rows = min(kThreads, n - r);
+        const int64_t from = int64_t(float(r) * mean), to = int64_t(float(r + rows) * mean);
+        auto fetch = [](const void* first, const void* last) {  // whole 16-byte units between the two
+            const uint64_t a = (reinterpret_cast<uint64_t>(first) + 15) & ~uint64_t(15), z = reinterpret_cast<uint64_t>(last) & ~uint64_t(15);
+            if (a < z) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"(uint32_t(z - a)) : "memory");
+        };
+        const int64_t f = min(from, int64_t(nnz)), t = min(to, int64_t(nnz));
+        fetch(col + f, col + t);
+        if (AHEAD == kAll) {
+            fetch(val + f, val + t);
+            fetch(x + r, x + r + rows);
+        }
     }
+    if (AHEAD != kNothing) __syncwarp();  // before the warp's loads: behind them it gains nothing
     const int s = __ldg(row_ptr + r), e = __ldg(row_ptr + r + 1);
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     for (int j = s; j < e; j += 4) {
@@ -292,7 +305,7 @@ struct NangilaSpmv {
     int* d_status = nullptr;  // set by a kernel whose bulk copy timed out
     bool plain_loads = false;  // NANGILA_SPMV_PLAIN=1: use the plain-load kernel
     bool short_rows = false;   // every row suits one thread: spmv_short_rows_kernel
-    float fetch_mean = 0.0f;   // its mean row length, 0: too small a matrix for fetching ahead
+    Ahead ahead = kNothing;    // what it fetches ahead
     int cap = kCap;            // non-zeros per staged row block: 2048 (256 threads) or 1024 (128 threads, NANGILA_SPMV_TILE=1024)
     double* d_work = nullptr;   // solver vectors (kWorkVectors), allocated on first solve
     double* d_partial = nullptr;  // partial sums, then results and counter of the solver kernel
@@ -392,7 +405,8 @@ extern "C" int nangila_spmv_load(NangilaSpmv* c, int n, int nnz, const int* row_
         int longest = 0;
         for (int r = 0; r < n; ++r) longest = std::max(longest, row_ptr[r + 1] - row_ptr[r]);
         c->short_rows = longest <= kShortRow && nnz <= int64_t(kShortMean) * n;
-        c->fetch_mean = 12 * int64_t(nnz) + 20 * int64_t(n) > kFetchAhead ? float(nnz) / float(n) : 0.0f;
+        const int64_t bytes = 12 * int64_t(nnz) + 20 * int64_t(n);
+        c->ahead = bytes > kAllAhead ? kAll : bytes > kColumnsAhead ? kColumns : kNothing;
     }
     c->h_diag_slot.assign(size_t(n), -1);
     for (int r = 0; r < n; ++r)
@@ -444,8 +458,9 @@ extern "C" int nangila_spmv_device(NangilaSpmv* c, const double* d_x, double* d_
     if (c->plain_loads) return nangila_spmv_launch(c->d_row_ptr, c->d_col, c->d_val, d_x, d_y, c->d_blocks, c->n_blocks, stream);
     if (c->n_blocks <= 0) return 0;
     if (c->short_rows) {
-        spmv_short_rows_kernel<<<unsigned((int64_t(c->n) + kThreads - 1) / kThreads), kThreads, 0, stream>>>(c->d_row_ptr, c->d_col, c->d_val, d_x,
-                                                                                                        d_y, c->n, c->nnz, c->fetch_mean);
+        auto* kernel = c->ahead == kAll ? spmv_short_rows_kernel<kAll> : c->ahead == kColumns ? spmv_short_rows_kernel<kColumns> : spmv_short_rows_kernel<kNothing>;
+        kernel<<<unsigned((int64_t(c->n) + kThreads - 1) / kThreads), kThreads, 0, stream>>>(c->d_row_ptr, c->d_col, c->d_val, d_x, d_y, c->n, c->nnz,
+                                                                                           float(c->nnz) / float(c->n));
         return int(cudaGetLastError());
     }
     if (c->cap == 1024)
