@@ -22,11 +22,14 @@
 // and small systems run on few CTAs, or on one. Measured on B200, us per iteration of whole calls, copies included, against
 // one CUDA graph of 13 kernels per iteration: mesh of 400 nodes 59 -> 3.9, 2500: 57 -> 7.0, 65 536: 70 -> 8.9, 400 000: 83 -> 22, 10^6: 180 -> 69.
 // With the values of a sum shared out among the lanes while a warp adds them up, a barrier less, and all entries of a row gathered at once:
-// 10 000 nodes 7.11 -> 6.76, 65 536: 8.90 -> 8.38, 300 000: 16.4 -> 15.7. (Partial sums that carry their number, which every CTA looks at itself instead of
+// 10 000 nodes 7.19 -> 6.81, 65 536: 8.86 -> 8.40, 300 000: 16.6 -> 15.9; ladders of 10 000: 8.07 -> 7.68, 300 000: 15.9 -> 14.8; random rows of about six
+// entries, 65 536: 12.0 -> 11.8, 300 000: 28.1 -> 28.6 to 29.2; uneven rows, 65 536 (mean 4.5): 14.2 -> 13.6. (Partial sums that carry their number, which every CTA looks at itself instead of
 // a counter, took 10 us at 65 536 nodes.)
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "signal.cuh"
 
@@ -43,7 +46,6 @@ constexpr int kEntriesPerCta = 2048;
 constexpr int kMaxCtas = 512;         // a sum reads the CTAs' slots with one thread each
 constexpr int kLongRow = 64;          // rows above this many entries are summed by a whole warp each
 constexpr int kCheckEvery = 4;        // iterations between two tests of the residual
-constexpr int kAtOnce = 5;            // entries of a row gathered together: a mesh's
 // Below these shares of what they are differences of, <r, r> and <r0, r> are summed from r itself. |r| < 0.1 |s|: an error of about
 // 1e-16 |s|^2 is then 1e-14 of |r|^2. <r0, r> may be small of itself; its line only has to catch what is nothing but rounding.
 constexpr double kCancelled = 1e-2;
@@ -243,21 +245,29 @@ __global__ void __launch_bounds__(solver_threads(RESIDENT), 1) bicgstab_kernel(c
       decltype(load(0)) own{};
       if (mine && lane == 0) own = load(r0 + i);
       double sum = 0.0;
-      if (mine) {
-        // all gathers of a short row at once, at a valid place whatever its length: the next one would wait for a trip to L2 otherwise
-        for (int j = s + lane; j < e; j += kAtOnce * lanes) {
-          double g[kAtOnce], w[kAtOnce];
+      // All gathers of a short row at once, at a valid place whatever its length: the next one would wait for a trip to L2 otherwise. As many as the warp's
+      // longest row has, since a gather that nobody needs takes its time too (five for every row: ladders 2 to 8 % slower than with one behind the other).
+      const int most = __reduce_max_sync(0xffffffffu, mine ? e - s : 0);
+      auto row = [&](auto n) {
+        constexpr int N = decltype(n)::value;
+        if (mine) {
+          for (int j = s + lane; j < e; j += N * lanes) {
+            double g[N], w[N];
 #pragma unroll
-          for (int u = 0; u < kAtOnce; ++u) {
-            const int at = min(j + u * lanes, e - 1);
-            g[u] = gather(col[at]);
-            w[u] = val[at];
+            for (int u = 0; u < N; ++u) {
+              const int at = min(j + u * lanes, e - 1);
+              g[u] = gather(col[at]);
+              w[u] = val[at];
+            }
+#pragma unroll
+            for (int u = 0; u < N; ++u)
+              if (j + u * lanes < e) sum += w[u] * g[u];
           }
-#pragma unroll
-          for (int u = 0; u < kAtOnce; ++u)
-            if (j + u * lanes < e) sum += w[u] * g[u];
         }
-      }
+      };
+      if (most <= 3 * lanes) row(std::integral_constant<int, 3>{});
+      else if (most <= 5 * lanes) row(std::integral_constant<int, 5>{});
+      else row(std::integral_constant<int, 4>{});
       for (int off = lanes >> 1; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off, lanes);
       if (mine && lane == 0) finish(r0 + i, own, sum);
     }
