@@ -127,10 +127,10 @@ def decompress_gpu(self: NangilaHook, layer_id: int, compressed: torch.Tensor, o
     known = _state(self)["layers"].get(layer_id)
     out, predicted = None, False
     with torch.cuda.device(dev):
-        if known is not None and known.n == n and known.curr.device == dev:
+        if known is not None and known.n == n and known.curr.device == dev and 0 <= layer_id <= 0xFFFFFFFF:
             out = torch.empty(n, dtype=torch.float32, device=dev)
             predicted = known.updates >= 2
-            fixed, got, queued = _glue().packet_inspect(packet, sync_mode != 0, layer_id, known.curr if predicted else None,
+            fixed, got, queued = _glue().packet_inspect(packet, sync_mode != 0, int(layer_id), known.curr if predicted else None,
                                                         known.prev if predicted else None, float(self.momentum()), out)
         else:
             fixed, got, queued = _glue().packet_inspect(packet, sync_mode != 0)
