@@ -26,6 +26,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "follow.cuh"
 #include "nangila_kernels.h"
 #include "ptx_sm100.cuh"
@@ -92,7 +94,7 @@ psgd_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  may_follow();
+  if (push.counters == nullptr) may_follow();
   follow();
 
   if (nslabs > 0) {
@@ -326,7 +328,9 @@ __global__ void __launch_bounds__(256) psgd_reconstruct_kernel(T* __restrict__ g
 // rank 8 (four factors of 512 to 4608 rows at once): 72 -> 18 us each. Before, every pass went through memory, and one thread
 // factorised with its matrices in local memory.
 // A rank on its own reads the factor where the GEMM left it. The GEMM then needs no counters, no second look at its tiles and no flag (11 -> 5.5 us), and
-// with every kernel of the chain set up while the one before it ends, the four matrices of a ResNet-50 bucket (2.4 to 1.0 M elements, rank 4) take 49 us and not 67.
+// with every kernel of the chain set up while the one before it ends, the four matrices of a ResNet-50 bucket (2.4 to 1.0 M elements, rank 4) take 48 us and not 67.
+// With several ranks (one rank of two, four, eight timed, the others' words there already; the same bucket): 92, 102, 124 us with a kernel behind the other and
+// the mean taken a column at a time; 84, 97, 122 so (rank 8: 110, 120, 149 -> 94, 107, 138).
 constexpr int kXCtas = 8;
 constexpr int kXThreads = 512;
 constexpr int kXWarps = kXThreads / 32;
@@ -389,8 +393,9 @@ __device__ __forceinline__ void factorise(const float* gram, int r, float (*L)[k
   }
 }
 
-// RMAX: compile-time bound on the rank (4, 8 or 16). SMEM: this CTA's rows fit into shared memory.
-template <int RMAX, bool SMEM>
+// RMAX: compile-time bound on the rank (4, 8 or 16). SMEM: this CTA's rows fit into shared memory. ALONE: nobody to exchange with, the
+// factor is read where the GEMM left it, four columns at a time.
+template <int RMAX, bool SMEM, bool ALONE>
 __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_constant__ NangilaPsgdExchangeParams p) {
   constexpr int kAcc = RMAX * (RMAX + 1) / 2;
   cg::cluster_group cluster = cg::this_cluster();
@@ -401,8 +406,6 @@ __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_c
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint64_t slot_bytes = (uint64_t(rows) * r * 4 + 255) & ~uint64_t(255);
   follow();
-  // nobody to exchange with: the factor is read where the GEMM left it, four columns at a time
-  const bool alone = W == 1 && p.pushed == 0 && (reinterpret_cast<uintptr_t>(p.local[vr]) & 15u) == 0;
   const uint32_t epoch = p.epoch_dev != nullptr ? *p.epoch_dev : p.epoch;
   const uint64_t base = p.recv_off + uint64_t(epoch & 1u) * W * slot_bytes;  // two slot sets, by launch parity
   uint32_t* status = p.status[vr];
@@ -421,7 +424,7 @@ __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_c
 
   // 1. store my rows of my factor (r columns, column-major) into every rank's slot [me] (unless the GEMM's
   //    epilogue has done that already)
-  if (p.pushed == 0 && !alone) {
+  if (!ALONE && p.pushed == 0) {
     for (int d = 0; d < W; ++d) {
       float* dst = reinterpret_cast<float*>(p.region[(me + d) % W] + base + uint64_t(me) * slot_bytes);
       for (int c = 0; c < r; ++c)
@@ -438,7 +441,7 @@ __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_c
   //    the cluster barriers below, doing no work)
   if (tid == 0) s_ok = 1;
   __syncthreads();
-  if (tid < W && !alone) {
+  if (!ALONE && tid < W) {
     if (!wait_flag(reinterpret_cast<const uint32_t*>(p.region[me] + p.flag_off) + tid, epoch, p.timeout_ns, status,
                    kTimeoutPhase2, uint32_t(me), uint32_t(tid), 8u, 0u))
       s_ok = 0;
@@ -451,7 +454,7 @@ __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_c
   const int pitch = SMEM ? per : rows;  // element (row r0 + i, c) at work[c * pitch + i]
   if (ok) {
     const float inv_w = 1.0f / float(W);
-    if (alone) {
+    if constexpr (ALONE) {
       for (int i = tid; i < mine; i += kXThreads) {
         const float4* row = reinterpret_cast<const float4*>(local + int64_t(r0 + i) * kCols);
 #pragma unroll
@@ -469,16 +472,28 @@ __global__ void __launch_bounds__(kXThreads) psgd_exchange_kernel(const __grid_c
           }
         }
       }
-    }
-    for (int c = alone ? r : 0; c < r; ++c)
+    } else {
+      // (all columns' loads of a few ranks on their way together)
+      const float* slots = reinterpret_cast<const float*>(p.region[me] + base) + r0;
+      const int64_t slot = int64_t(slot_bytes / 4);
       for (int i = tid; i < mine; i += kXThreads) {
-        float acc = 0.0f;
+        float acc[RMAX];
+#pragma unroll
+        for (int c = 0; c < RMAX; ++c) acc[c] = 0.0f;
+#pragma unroll 4
         for (int src = 0; src < W; ++src)
-          acc += reinterpret_cast<const float*>(p.region[me] + base + uint64_t(src) * slot_bytes)[int64_t(c) * rows + r0 + i];
-        acc *= inv_w;
-        if (!p.orth_mean) mean[int64_t(c) * rows + r0 + i] = acc;
-        work[int64_t(c) * pitch + i] = acc;
+#pragma unroll
+          for (int c = 0; c < RMAX; ++c)
+            if (c < r) acc[c] += slots[src * slot + int64_t(c) * rows + i];
+#pragma unroll
+        for (int c = 0; c < RMAX; ++c) {
+          if (c < r) {
+            if (!p.orth_mean) mean[int64_t(c) * rows + r0 + i] = acc[c] * inv_w;
+            work[int64_t(c) * pitch + i] = acc[c] * inv_w;
+          }
+        }
       }
+    }
     for (int c = r; c < kCols; ++c)
       for (int i = r0 + tid; i < r1; i += kXThreads) {
         mean[int64_t(c) * rows + i] = 0.0f;
@@ -745,13 +760,15 @@ extern "C" int nangila_psgd_exchange(const NangilaPsgdExchangeParams* p, cudaStr
   cfg.attrs = attrs;
   cfg.numAttrs = 2;
   const NangilaPsgdExchangeParams params = *p;
-  cudaError_t e;
-  if (p->rank <= 4)
-    e = smem ? cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<4, true>, params) : cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<4, false>, params);
-  else if (p->rank <= 8)
-    e = smem ? cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<8, true>, params) : cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<8, false>, params);
-  else
-    e = smem ? cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<kCols, true>, params)
-             : cudaLaunchKernelEx(&cfg, psgd_exchange_kernel<kCols, false>, params);
+  // (one rank in the launch: `local` of the group's only rank)
+  const bool alone = p->world == 1 && p->pushed == 0 && (reinterpret_cast<uintptr_t>(p->local[0]) & 15u) == 0;
+  auto launch = [&](auto rmax) {
+    constexpr int R = decltype(rmax)::value;
+    auto* kernel = smem ? (alone ? psgd_exchange_kernel<R, true, true> : psgd_exchange_kernel<R, true, false>)
+                        : (alone ? psgd_exchange_kernel<R, false, true> : psgd_exchange_kernel<R, false, false>);
+    return cudaLaunchKernelEx(&cfg, kernel, params);
+  };
+  using std::integral_constant;
+  const cudaError_t e = p->rank <= 4 ? launch(integral_constant<int, 4>{}) : p->rank <= 8 ? launch(integral_constant<int, 8>{}) : launch(integral_constant<int, kCols>{});
   return int(e);
 }
