@@ -140,7 +140,8 @@ at::Tensor packet_compress(const at::Tensor& grad, const c10::optional<at::Tenso
   };
   c10::cuda::CUDAGuard guard(grad.device());
   auto packet = at::empty({32 + nangila_packet_payload_bytes(n)}, grad.options().dtype(at::kByte));
-  // The gain's sums: in FP32 where few parts meet (64 CTAs of 2048 elements: off by 1e-7), in 64 bits beyond.
+  // The gain's sums: in FP32 where few parts meet (64 CTAs of 2048 elements: off by 1e-7, and such packets keep the bytes they have always had), in 64 bits
+  // beyond, where a thousand parts in any order moved the gain by 1e-7 to 1e-6. (nangila_packet_encode has room for FP32 only. A packet carries its gain.)
   const bool few = n <= 64 * 2048;
   auto sums = at::empty({2}, grad.options().dtype(few ? at::kFloat : at::kDouble));
   if (few) {

@@ -12,8 +12,8 @@
 // without flags or fences that the hardware hands out as SMs come free.
 // What bounds them: HBM and L2 traffic. Measured on B200, four ranks on one device, 3.1 M bf16 elements each, INT8 (25 MB in, 39 MB of codes, 100 MB
 // out): 17 us (5.2 TB/s) + 21 us (5.5 TB/s), 42.4 us for the call; as one resident kernel with block barriers and a flag per chunk 49.3 us.
-// The arithmetic is kept out of the way: with divisions by the chunk size, conversions and clamps (250 instructions per eight elements, now 90; 132 and now 35
-// to expand them) the two took 19 and 45 us.
+// The arithmetic is kept out of the way: with divisions by the chunk size, conversions and clamps the two took 19 and 45 us (now 167 and 51 instructions per
+// eight elements, the stores to three peers and this rank's own part among them).
 //
 // The reference leaves the FSDP parameter all-gather untouched (python/nangila/fsdp.py:80-236 only
 // hooks the gradient path).

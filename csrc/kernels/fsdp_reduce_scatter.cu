@@ -54,7 +54,8 @@ struct RsShape {
 template <typename T, typename S>
 constexpr bool kPackedBf16 = std::is_same_v<T, __nv_bfloat16> && std::is_same_v<S, __nv_bfloat16>;
 
-// (A loop's invariants cost registers; without one 64 are enough for four CTAs an SM.)
+// (A loop's invariants cost registers; without one 64 are enough for four CTAs an SM. Packed bf16 without error memory: six, although 16 bytes a thread
+// spill; without spills 43.0 us with five and 45.5 with four for the call above, against 42.8.)
 template <typename T, typename S, bool EF, Walk WALK>
 __global__ void __launch_bounds__(kThreads, WALK != kNoWalk ? 2 : kPackedBf16<T, S> && !EF ? 6 : 4) rs_quantize_kernel(const __grid_constant__ NangilaPredResParams p, const __grid_constant__ RsShape sh) {
   may_follow();
